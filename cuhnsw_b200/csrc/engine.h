@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "host_stage.h"
 #include "kernels.h"
 
 namespace hnsw {
@@ -199,6 +200,13 @@ class Engine {
   unsigned long long lane_clock_ = 0;
   int LaneFor(cudaStream_t stream, SearchLane** lane);
   int MarkLane(SearchLane* lane);  // records `done` on the engine's stream
+  // host-buffer search through page-locked staging; *handled = false: the size or the buffers ask for another way
+  int SearchGraphStaged(const float* q, long long nq, int topk, int ef, int* nns, float* dist, int* found,
+                        bool* handled);
+  int SearchGraphCopied(const float* q, long long nq, int topk, int ef, int* nns, float* dist, int* found);
+  static constexpr size_t kInPlaceBytes = 256u << 10;  // queries and results of a search that are staged in place
+  static constexpr int kPieces = 4;          // pieces of one search in flight
+  cudaStream_t piece_streams_[kPieces] = {};  // created when a search first needs them
   int WaitForSearches();           // every search enqueued so far, on whatever stream, is over
   int PrepareSchedule(long long nq, SearchLane* lane, SearchSchedule* s);
   double last_build_seconds_ = 0.0;
