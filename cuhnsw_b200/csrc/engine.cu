@@ -235,7 +235,38 @@ int Engine::SetData(const float* data, long long num_data, int num_dims) {
   if (num_data >= (1ll << 31) - 1) return Fail(kUnsupported, "at most 2^31 - 2 rows per index");
   int rc = AllocRows(num_data, num_dims);
   if (rc) return rc;
-  // stage through a bounded device buffer and pad rows on the device
+  if ((rc = UploadRows(data, num_dims)) != kOk) return rc;
+  has_data_ = true;
+  Log(3, "copied data (%lld x %d), row stride %d %s", n_, d_, vstride_, rows16_ ? "16-bit values" : "floats");
+  return kOk;
+}
+
+// Rows from pageable memory: several threads copy pieces into page-locked buffers, from which a piece goes to the
+// device while the next ones are copied (fp32 rows without padding by one DMA, others by the kernel that pads or rounds
+// them, reading host memory in place).  1 M x 128 fp32 rows: 49 ms through the driver's own staging.
+int Engine::UploadRows(const float* data, int num_dims) {
+  HostStage& stage = HostStage::Get();
+  const size_t row = (size_t)num_dims * sizeof(float);
+  const long long piece = std::max<long long>(1, (long long)(HostStage::kBufferBytes / row));
+  const bool plain = rows16_ == 0 && vstride_ == num_dims;
+  Pipeline pipe;
+  if (n_ > 0 && row <= HostStage::kBufferBytes && pipe.Open((n_ + piece - 1) / piece)) {
+    for (long long s = 0; s < n_; s += piece) {
+      const long long r = std::min(piece, n_ - s);
+      Pipeline::Slot& slot = pipe.Next();
+      CU(pipe.Wait(slot));
+      stage.Copy(slot.host(), data + (size_t)s * num_dims, (size_t)r * row);
+      if (plain)
+        CU(cudaMemcpyAsync(RowPtr(s), slot.host(), (size_t)r * row, cudaMemcpyHostToDevice, stream_));
+      else
+        CU(launch_pad_rows(reinterpret_cast<const float*>(slot.host()), num_dims, RowPtr(s), r, num_dims, vstride_,
+                           rows16_, stream_));
+      CU(pipe.Mark(slot, stream_));
+    }
+    CU(cudaStreamSynchronize(stream_));
+    return kOk;
+  }
+  // no page-locked memory to be had: through a bounded device buffer
   const long long rows_per_chunk = std::max<long long>(1, (64ll << 20) / num_dims);
   DevBuf<float> raw;
   CU(raw.alloc((size_t)std::min(rows_per_chunk, std::max<long long>(n_, 1)) * num_dims));
@@ -246,8 +277,39 @@ int Engine::SetData(const float* data, long long num_data, int num_dims) {
     CU(launch_pad_rows(raw.get(), num_dims, RowPtr(s), r, num_dims, vstride_, rows16_, stream_));
     CU(cudaStreamSynchronize(stream_));
   }
-  has_data_ = true;
-  Log(3, "copied data (%lld x %d), row stride %d %s", n_, d_, vstride_, rows16_ ? "16-bit values" : "floats");
+  return kOk;
+}
+
+// `count` rows of `width` ints, `stride` ints apart on the device, into a dense host array: pieces come down into
+// page-locked buffers while several threads copy the ones before into the caller's (often freshly mapped) memory.
+int Engine::DownloadRows(int* dst, const int* src, int stride, int width, long long count) {
+  const size_t row = (size_t)width * sizeof(int);
+  const long long piece = std::max<long long>(1, (long long)(HostStage::kBufferBytes / row));
+  Pipeline pipe;
+  if (!pipe.Open((count + piece - 1) / piece)) {
+    CU(cudaMemcpy2DAsync(dst, row, src, (size_t)stride * sizeof(int), row, (size_t)count, cudaMemcpyDeviceToHost,
+                         stream_));
+    CU(cudaStreamSynchronize(stream_));
+    return kOk;
+  }
+  const int depth = pipe.depth();
+  const long long pieces = (count + piece - 1) / piece;
+  for (long long i = 0; i < pieces + depth - 1; ++i) {
+    if (i < pieces) {
+      const long long s = i * piece, r = std::min(piece, count - s);
+      Pipeline::Slot& slot = pipe.At(i);
+      CU(cudaMemcpy2DAsync(slot.host(), row, src + (size_t)s * stride, (size_t)stride * sizeof(int), row, (size_t)r,
+                           cudaMemcpyDeviceToHost, stream_));
+      CU(pipe.Mark(slot, stream_));
+    }
+    const long long j = i - (depth - 1);
+    if (j >= 0) {
+      const long long s = j * piece, r = std::min(piece, count - s);
+      Pipeline::Slot& slot = pipe.At(j);
+      CU(pipe.Wait(slot));
+      HostStage::Get().Copy(dst + (size_t)s * width, slot.host(), (size_t)r * row);
+    }
+  }
   return kOk;
 }
 
@@ -844,12 +906,10 @@ int Engine::GetGraph(int* levels, int* rows0, int* rows_upper) {
   if (rc) return rc;
   CU(cudaStreamSynchronize(stream_));
   if (levels) std::memcpy(levels, levels_h_.data(), (size_t)n_ * sizeof(int));
-  if (rows0 && n_ > 0)
-    CU(cudaMemcpy2D(rows0, (size_t)opt_.max_m0 * sizeof(int), rows0_.get(), (size_t)stride0_ * sizeof(int),
-                    (size_t)opt_.max_m0 * sizeof(int), (size_t)n_, cudaMemcpyDeviceToHost));
-  if (rows_upper && total_upper_ > 0)
-    CU(cudaMemcpy2D(rows_upper, (size_t)opt_.max_m * sizeof(int), rowsU_.get(), (size_t)strideU_ * sizeof(int),
-                    (size_t)opt_.max_m * sizeof(int), (size_t)total_upper_, cudaMemcpyDeviceToHost));
+  if (rows0 && n_ > 0 && (rc = DownloadRows(rows0, rows0_.get(), stride0_, opt_.max_m0, n_)) != kOk) return rc;
+  if (rows_upper && total_upper_ > 0 &&
+      (rc = DownloadRows(rows_upper, rowsU_.get(), strideU_, opt_.max_m, total_upper_)) != kOk)
+    return rc;
   return kOk;
 }
 

@@ -69,13 +69,19 @@ class DevBuf {
   void release() {
     if (p_) cudaFree(p_);
     p_ = nullptr;
-    n_ = 0;
+    n_ = room_ = 0;
   }
+  // n elements of undefined content; what is there already is used again unless most of it would lie idle (handing 100
+  // MB back to the driver and taking it again costs 4 ms)
   cudaError_t alloc(size_t n) {
+    if (n > 0 && n <= room_ && room_ / 2 <= n) {
+      n_ = n;
+      return cudaSuccess;
+    }
     release();
     if (n == 0) return cudaSuccess;
     cudaError_t e = cudaMalloc(&p_, n * sizeof(T));
-    if (e == cudaSuccess) n_ = n;
+    if (e == cudaSuccess) n_ = room_ = n;
     else p_ = nullptr;
     return e;
   }
@@ -85,7 +91,7 @@ class DevBuf {
 
  private:
   T* p_ = nullptr;
-  size_t n_ = 0;
+  size_t n_ = 0, room_ = 0;
 };
 
 class Engine {
@@ -142,6 +148,8 @@ class Engine {
   int FailCuda(cudaError_t e, const char* what);
   int EnsureDevice();
   int AllocRows(long long num_data, int num_dims);
+  int UploadRows(const float* data, int num_dims);
+  int DownloadRows(int* dst, const int* src, int stride, int width, long long count);
   int AllocGraph();
   int ResolveVsize(int requested_cap, long long nq, int* vsize) const;  // nq < 0: construction
   GraphView View() const;

@@ -180,4 +180,60 @@ class StageBuffer {
   void* p_;
 };
 
+// A ring of staging buffers for a transfer in pieces: fill or drain one while the device works on the others.
+class Pipeline {
+ public:
+  static constexpr int kDepth = 3;
+  class Slot {
+   public:
+    unsigned char* host() const { return buffer_->get(); }
+
+   private:
+    friend class Pipeline;
+    std::unique_ptr<StageBuffer> buffer_;
+    cudaEvent_t done_ = nullptr;
+    bool pending_ = false;
+  };
+  Pipeline() = default;
+  Pipeline(const Pipeline&) = delete;
+  Pipeline& operator=(const Pipeline&) = delete;
+  // the device is through with every buffer before it goes back
+  ~Pipeline() {
+    for (Slot& s : slots_) {
+      if (s.pending_) cudaEventSynchronize(s.done_);
+      if (s.done_) cudaEventDestroy(s.done_);
+    }
+  }
+  // buffers for `pieces` pieces (at most kDepth); false: none to be had
+  bool Open(long long pieces) {
+    for (; depth_ < kDepth && depth_ < pieces; ++depth_) {
+      Slot& s = slots_[depth_];
+      s.buffer_.reset(new StageBuffer(depth_ == 0));
+      if (!s.buffer_->get() || cudaEventCreateWithFlags(&s.done_, cudaEventDisableTiming) != cudaSuccess) {
+        s.buffer_.reset();
+        cudaGetLastError();
+        break;
+      }
+    }
+    return depth_ > 0;
+  }
+  int depth() const { return depth_; }
+  Slot& At(long long i) { return slots_[i % depth_]; }
+  Slot& Next() { return At(turn_++); }
+  cudaError_t Mark(Slot& s, cudaStream_t stream) {
+    s.pending_ = true;
+    return cudaEventRecord(s.done_, stream);
+  }
+  cudaError_t Wait(Slot& s) {
+    if (!s.pending_) return cudaSuccess;
+    s.pending_ = false;
+    return cudaEventSynchronize(s.done_);
+  }
+
+ private:
+  Slot slots_[kDepth];
+  int depth_ = 0;
+  long long turn_ = 0;
+};
+
 }  // namespace hnsw

@@ -273,9 +273,10 @@ class CuHNSWBind:
   def get_graph(self):
     info = self.describe()
     n = info["num_data"]
-    levels = np.zeros(n, np.int32)
-    rows0 = np.full((n, info["max_m0"]), -1, np.int32)
-    rows_u = np.full((max(info["upper_rows"], 1), info["max_m"]), -1, np.int32)
+    levels = np.empty(n, np.int32)  # the engine writes every element it is given
+    rows0 = np.empty((n, info["max_m0"]), np.int32)
+    rows_u = (np.empty if info["upper_rows"] else lambda shape, dtype: np.full(shape, -1, dtype))(
+      (max(info["upper_rows"], 1), info["max_m"]), np.int32)
     self._check(self._lib.cuhnsw_get_graph(self._h, levels.ctypes.data, rows0.ctypes.data, rows_u.ctypes.data))
     return levels, rows0, rows_u
 
