@@ -1,12 +1,19 @@
 #include "engine.h"
 
+#include <fcntl.h>
+#include <sys/stat.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <atomic>
+#include <cerrno>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
+#include <functional>
 #include <sstream>
 
 #include "json_min.h"
@@ -43,6 +50,44 @@ struct FileHeader {
 };
 #pragma pack(pop)
 static_assert(sizeof(FileHeader) == 96, "hnswlib header is 96 bytes");
+
+// Whole transfers to and from a file descriptor; false: error or end of file.
+bool WriteAll(int fd, const void* data, size_t bytes) {
+  const char* p = static_cast<const char*>(data);
+  while (bytes > 0) {
+    const ssize_t w = ::write(fd, p, bytes);
+    if (w < 0 && errno == EINTR) continue;
+    if (w <= 0) return false;
+    p += w;
+    bytes -= (size_t)w;
+  }
+  return true;
+}
+bool ReadAt(int fd, void* data, size_t bytes, long long at) {
+  char* p = static_cast<char*>(data);
+  while (bytes > 0) {
+    const ssize_t r = ::pread(fd, p, bytes, (off_t)at);
+    if (r < 0 && errno == EINTR) continue;
+    if (r <= 0) return false;
+    p += r;
+    at += r;
+    bytes -= (size_t)r;
+  }
+  return true;
+}
+// The same by several threads (a read of cached pages is a copy), in parts of whole records of `rec` bytes; then(first,
+// count) is called for each part's records while they are still in that thread's cache.
+bool ReadRecords(int fd, void* data, size_t rec, long long count, long long at,
+                 const std::function<void(long long, long long)>& then) {
+  const long long part = std::max<long long>(1, (long long)((1u << 20) / rec));
+  std::atomic<bool> ok{true};
+  HostStage::Get().ParallelFor((int)((count + part - 1) / part), [&](int i) {
+    const long long lo = i * part, r = std::min(part, count - lo);
+    if (!ReadAt(fd, static_cast<char*>(data) + (size_t)lo * rec, (size_t)r * rec, at + lo * (long long)rec)) ok = false;
+    else then(lo, r);
+  });
+  return ok;
+}
 }  // namespace
 
 Engine::Engine() { HostStage::Get().AddUser(); }
@@ -922,18 +967,20 @@ int Engine::SaveIndex(const char* path) {
   int rc = EnsureDevice();
   if (rc) return rc;
   CU(cudaStreamSynchronize(stream_));
-  std::FILE* f = std::fopen(path, "wb");
-  if (!f) return Fail(kIoError, std::string("cannot open ") + path + " for writing");
+  // An existing file is overwritten in place and cut to its new length at the end: its cached pages are used again
+  // instead of being freed and allocated anew.
+  const int fd = ::open(path, O_WRONLY | O_CREAT | O_CLOEXEC, 0666);
+  if (fd < 0) return Fail(kIoError, std::string("cannot open ") + path + " for writing");
   // closes the file on every way out; a file that was not written to the end is removed
   struct Guard {
-    std::FILE* f;
+    int fd;
     const char* path;
     bool done = false;
     ~Guard() {
-      if (f) std::fclose(f);
+      if (fd >= 0) ::close(fd);
       if (!done) std::remove(path);
     }
-  } guard{f, path};
+  } guard{fd, path};
   const int m = opt_.max_m, m0 = opt_.max_m0;
   const size_t rec = 4 + 4 * (size_t)m0 + 4 * (size_t)d_ + 8;
   FileHeader h;
@@ -950,30 +997,43 @@ int Engine::SaveIndex(const char* path) {
   h.m = (uint64_t)m;
   h.mult = opt_.level_mult;
   h.ef_construction = (uint64_t)opt_.ef_construction;
-  bool ok = std::fwrite(&h, sizeof(h), 1, f) == 1;
-  // Level-0 records are put together on the device, 32 MB at a time, exactly as they lie in the file: one
+  bool ok = WriteAll(fd, &h, sizeof(h));
+  // Level-0 records are put together on the device, piece by piece, exactly as they lie in the file: one
   // kernel packs the adjacency rows into degree word + neighbour slots and writes the labels, another moves
-  // the vectors out of their padded (fp32 or 16-bit) rows; the host only writes the chunk out.  Labels of a
-  // loaded index are 64-bit values the device does not hold: the host patches those in.
+  // the vectors out of their padded (fp32 or 16-bit) rows; a piece comes down into a page-locked buffer while the
+  // host writes out the ones before.  Labels of a loaded index are 64-bit values the device does not hold: the host
+  // patches those in.
   const long long rec_words = (long long)(rec / 4);
-  const long long chunk = std::max<long long>(1, (32ll << 20) / (long long)rec);
+  const long long chunk = std::max<long long>(1, (long long)(HostStage::kBufferBytes / rec));
+  const long long pieces = (n_ + chunk - 1) / chunk;
   const size_t chunk_rows = (size_t)std::min(chunk, std::max<long long>(n_, 1));
-  DevBuf<unsigned> packed;
-  CU(packed.alloc(chunk_rows * (size_t)rec_words));
-  std::vector<unsigned char> out(chunk_rows * rec);
-  for (long long s = 0; s < n_ && ok; s += chunk) {
-    const long long r = std::min(chunk, n_ - s);
-    CU(launch_pack_links(rows0_.get() + (size_t)s * stride0_, stride0_, r, s, m0, packed.get(), rec_words, stream_));
-    CU(launch_unpad_rows(RowPtr(s), reinterpret_cast<float*>(packed.get()) + 1 + m0, rec_words, r, d_, vstride_,
-                         rows16_, stream_));
-    CU(cudaMemcpyAsync(out.data(), packed.get(), (size_t)r * rec, cudaMemcpyDeviceToHost, stream_));
-    CU(cudaStreamSynchronize(stream_));
+  Pipeline pipe;
+  std::vector<unsigned char> pageable;  // one record above the size of a staging buffer, or no page-locked memory
+  if (rec > HostStage::kBufferBytes || !pipe.Open(std::max<long long>(pieces, 1))) pageable.resize(chunk_rows * rec);
+  const int depth = pageable.empty() ? pipe.depth() : 1;
+  for (int i = 0; i < depth; ++i) CU(records_[i].reserve(chunk_rows * (size_t)rec_words));
+  auto host = [&](long long i) { return pageable.empty() ? pipe.At(i).host() : pageable.data(); };
+  for (long long i = 0; i < pieces + depth - 1 && ok; ++i) {
+    if (i < pieces) {
+      const long long s = i * chunk, r = std::min(chunk, n_ - s);
+      unsigned* to = records_[i % depth].get();
+      CU(launch_pack_links(rows0_.get() + (size_t)s * stride0_, stride0_, r, s, m0, to, rec_words, stream_));
+      CU(launch_unpad_rows(RowPtr(s), reinterpret_cast<float*>(to) + 1 + m0, rec_words, r, d_, vstride_, rows16_,
+                           stream_));
+      CU(cudaMemcpyAsync(host(i), to, (size_t)r * rec, cudaMemcpyDeviceToHost, stream_));
+      if (pageable.empty()) CU(pipe.Mark(pipe.At(i), stream_));
+      else CU(cudaStreamSynchronize(stream_));
+    }
+    const long long j = i - (depth - 1);
+    if (j < 0) continue;
+    if (pageable.empty()) CU(pipe.Wait(pipe.At(j)));
+    const long long s = j * chunk, r = std::min(chunk, n_ - s);
     if (labelled_)
-      for (long long i = 0; i < r; ++i) {
-        const uint64_t label = (uint64_t)labels_h_[(size_t)(s + i)];
-        std::memcpy(out.data() + (size_t)(i + 1) * rec - 8, &label, 8);
+      for (long long k = 0; k < r; ++k) {
+        const uint64_t label = (uint64_t)labels_h_[(size_t)(s + k)];
+        std::memcpy(host(j) + (size_t)(k + 1) * rec - 8, &label, 8);
       }
-    ok = std::fwrite(out.data(), rec, (size_t)r, f) == (size_t)r;
+    ok = WriteAll(fd, host(j), (size_t)r * rec);
   }
   // upper-layer link lists: a length word per node, then its rows; gathered into the same buffer and written
   // whenever it fills
@@ -981,12 +1041,12 @@ int Engine::SaveIndex(const char* path) {
   if (total_upper_ > 0)
     CU(cudaMemcpy(upper.data(), rowsU_.get(), (size_t)total_upper_ * strideU_ * sizeof(int), cudaMemcpyDeviceToHost));
   const size_t per_link = 4 + 4 * (size_t)m;
+  std::vector<unsigned char> out(std::max<size_t>(1u << 20, 4 + per_link * (size_t)(max_level_ + 1)));
   size_t fill = 0;
   auto flush = [&]() {
-    if (fill && ok) ok = std::fwrite(out.data(), 1, fill, f) == fill;
+    if (fill && ok) ok = WriteAll(fd, out.data(), fill);
     fill = 0;
   };
-  out.resize(std::max<size_t>(out.size(), 4 + per_link * (size_t)(max_level_ + 1)));
   for (long long i = 0; i < n_ && ok; ++i) {
     const int lv = levels_h_[(size_t)i];
     const uint32_t nbytes = (uint32_t)(per_link * (size_t)lv);
@@ -1009,8 +1069,13 @@ int Engine::SaveIndex(const char* path) {
     fill += 4 + nbytes;
   }
   flush();
-  guard.f = nullptr;
-  ok = (std::fclose(f) == 0) && ok;
+  struct stat st;
+  if (ok && ::fstat(fd, &st) == 0 && S_ISREG(st.st_mode)) {
+    const off_t end = ::lseek(fd, 0, SEEK_CUR);
+    ok = end >= 0 && (st.st_size == end || ::ftruncate(fd, end) == 0);
+  }
+  guard.fd = -1;
+  ok = (::close(fd) == 0) && ok;
   if (!ok) return Fail(kIoError, std::string("short write to ") + path);
   guard.done = true;
   Log(3, "saved index to %s", path);
@@ -1020,17 +1085,17 @@ int Engine::SaveIndex(const char* path) {
 int Engine::LoadIndex(const char* path) {
   if (!inited_) return Fail(kBadState, "init() must be called first");
   if (!path) return Fail(kInvalidArgument, "null path");
-  std::FILE* f = std::fopen(path, "rb");
-  if (!f) return Fail(kIoError, std::string("cannot open ") + path);
+  const int fd = ::open(path, O_RDONLY | O_CLOEXEC);
+  if (fd < 0) return Fail(kIoError, std::string("cannot open ") + path);
   struct Closer {
-    std::FILE* f;
-    ~Closer() { std::fclose(f); }
-  } closer{f};
-  std::fseek(f, 0, SEEK_END);
-  const long long fsize = std::ftell(f);
-  std::fseek(f, 0, SEEK_SET);
+    int fd;
+    ~Closer() { ::close(fd); }
+  } closer{fd};
+  struct stat st;
+  if (::fstat(fd, &st) != 0) return Fail(kIoError, std::string("cannot read ") + path);
+  const long long fsize = (long long)st.st_size;
   FileHeader h;
-  if (fsize < (long long)sizeof(h) || std::fread(&h, sizeof(h), 1, f) != 1)
+  if (fsize < (long long)sizeof(h) || !ReadAt(fd, &h, sizeof(h), 0))
     return Fail(kIoError, "index file is shorter than its header");
   if (h.max_m0 < 1 || h.max_m0 > (uint64_t)kMaxLinksHost || h.max_m < 1 || h.max_m > h.max_m0)
     return Fail(kUnsupported, "index file: need 1 <= maxM <= maxM0 <= 64");
@@ -1066,29 +1131,41 @@ int Engine::LoadIndex(const char* path) {
   std::vector<long long> labels((size_t)n);
   const long long rec_words = (long long)(rec / 4);
   {
-    const long long chunk = std::max<long long>(1, (32ll << 20) / (long long)rec);
+    // several threads read a piece into a page-locked buffer while the device takes the ones before apart
+    const long long chunk = std::max<long long>(1, (long long)(HostStage::kBufferBytes / rec));
+    const long long pieces = (n + chunk - 1) / chunk;
     const size_t rows_in_chunk = (size_t)std::min(chunk, std::max<long long>(n, 1));
-    std::vector<unsigned char> buf(rows_in_chunk * rec);
-    DevBuf<unsigned> raw;
     DevBuf<unsigned long long> bad;
-    CU(raw.alloc(rows_in_chunk * (size_t)rec_words));
+    Pipeline pipe;
+    std::vector<unsigned char> pageable;  // one record above the size of a staging buffer, or no page-locked memory
+    if (rec > HostStage::kBufferBytes || !pipe.Open(std::max<long long>(pieces, 1))) pageable.resize(rows_in_chunk * rec);
+    const int depth = pageable.empty() ? pipe.depth() : 1;
+    for (int i = 0; i < depth; ++i) CU(records_[i].reserve(rows_in_chunk * (size_t)rec_words));
     CU(bad.alloc(1));
     CU(cudaMemsetAsync(bad.get(), 0xff, sizeof(unsigned long long), stream_));
-    for (long long s = 0; s < n; s += chunk) {
-      const long long r = std::min(chunk, n - s);
-      if (std::fread(buf.data(), rec, (size_t)r, f) != (size_t)r) return Fail(kIoError, "index file: short read");
-      CU(cudaMemcpyAsync(raw.get(), buf.data(), (size_t)r * rec, cudaMemcpyHostToDevice, stream_));
-      CU(launch_unpack_links(raw.get(), rec_words, r, s, m0, n, rows0_.get() + (size_t)s * stride0_, stride0_,
+    for (long long i = 0; i < pieces; ++i) {
+      const long long s = i * chunk, r = std::min(chunk, n - s);
+      if (pageable.empty()) CU(pipe.Wait(pipe.At(i)));
+      unsigned char* buf = pageable.empty() ? pipe.At(i).host() : pageable.data();
+      unsigned* to = records_[i % depth].get();
+      const bool read = ReadRecords(fd, buf, rec, r, (long long)sizeof(h) + s * (long long)rec,
+                                    [&](long long first, long long count) {
+                                      for (long long k = first; k < first + count; ++k) {
+                                        uint64_t label;
+                                        std::memcpy(&label, buf + (size_t)(k + 1) * rec - 8, 8);
+                                        labels[(size_t)(s + k)] = (long long)label;
+                                      }
+                                    });
+      if (!read) return Fail(kIoError, "index file: short read");
+      CU(cudaMemcpyAsync(to, buf, (size_t)r * rec, cudaMemcpyHostToDevice, stream_));
+      CU(launch_unpack_links(to, rec_words, r, s, m0, n, rows0_.get() + (size_t)s * stride0_, stride0_,
                              labels_d_.get() + s, bad.get(), stream_));
-      CU(launch_pad_rows(reinterpret_cast<const float*>(raw.get() + 1 + m0), rec_words, RowPtr(s), r, d, vstride_,
-                         rows16_, stream_));
-      for (long long i = 0; i < r; ++i) {
-        uint64_t label;
-        std::memcpy(&label, buf.data() + (size_t)(i + 1) * rec - 8, 8);
-        labels[(size_t)(s + i)] = (long long)label;
-      }
-      CU(cudaStreamSynchronize(stream_));  // buf and raw are reused by the next chunk
+      CU(launch_pad_rows(reinterpret_cast<const float*>(to + 1 + m0), rec_words, RowPtr(s), r, d, vstride_, rows16_,
+                         stream_));
+      if (pageable.empty()) CU(pipe.Mark(pipe.At(i), stream_));
+      if (!pageable.empty()) CU(cudaStreamSynchronize(stream_));
     }
+    CU(cudaStreamSynchronize(stream_));
     unsigned long long first_bad = 0;
     CU(cudaMemcpy(&first_bad, bad.get(), sizeof(first_bad), cudaMemcpyDeviceToHost));
     if (first_bad != ~0ull) {
@@ -1105,19 +1182,26 @@ int Engine::LoadIndex(const char* path) {
   const size_t per_link = 4 + 4 * (size_t)m;
   levels_h_.assign((size_t)n, 0);
   std::vector<int> rowsU;
-  std::vector<unsigned char> lbuf;
+  const long long lists_at = (long long)sizeof(h) + n * (long long)rec;
+  std::vector<unsigned char> lists((size_t)(fsize - lists_at));
+  if (!ReadRecords(fd, lists.data(), 1, (long long)lists.size(), lists_at, [](long long, long long) {}))
+    return Fail(kIoError, "index file: short read");
+  size_t pos = 0;
   for (long long i = 0; i < n; ++i) {
     uint32_t nbytes;
-    if (std::fread(&nbytes, 4, 1, f) != 1) return Fail(kIoError, "index file: truncated link lists");
+    if (lists.size() - pos < 4) return Fail(kIoError, "index file: truncated link lists");
+    std::memcpy(&nbytes, lists.data() + pos, 4);
+    pos += 4;
     if (nbytes % per_link || nbytes / per_link > 64) return Fail(kParseError, "index file: bad link list size");
     const int lv = (int)(nbytes / per_link);
     if (lv > h.maxlevel) return Fail(kParseError, "index file: a node lies above the file's top level");
     levels_h_[(size_t)i] = lv;
     if (!nbytes) continue;
-    lbuf.resize(nbytes);
-    if (std::fread(lbuf.data(), 1, nbytes, f) != nbytes) return Fail(kIoError, "index file: truncated link lists");
+    if (lists.size() - pos < nbytes) return Fail(kIoError, "index file: truncated link lists");
+    const unsigned char* list = lists.data() + pos;
+    pos += nbytes;
     for (int l = 0; l < lv; ++l) {
-      const unsigned char* o = lbuf.data() + per_link * (size_t)l;
+      const unsigned char* o = list + per_link * (size_t)l;
       uint32_t deg;
       std::memcpy(&deg, o, 4);
       deg &= 0xffffu;

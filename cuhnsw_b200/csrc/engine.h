@@ -181,6 +181,7 @@ class Engine {
 
   DevBuf<float> vec_;
   DevBuf<int> rows0_, rowsU_, levels_d_, upper_base_d_, labels_d_;
+  DevBuf<unsigned> records_[Pipeline::kDepth];  // pieces of an index file on their way (8 MB each, once a file was used)
   DevBuf<unsigned long long> counters_;  // [0] search ticket, [1..2] build tickets, [4..7] stats
   bool stats_on_ = false;
   // Scratch of one search in flight: its ticket counter and the grow-only arrays of the
