@@ -1,0 +1,84 @@
+"""Transfers between ordinary host arrays and the device go through page-locked buffers of 8 MB, in pieces: sizes
+around the edges of a piece and of the in-place path (256 KB), against the device-buffer search and the numpy reader of
+index files."""
+import numpy as np
+import pytest
+
+from conftest import assert_same_bits, engine_options
+from cuhnsw_b200 import CuHNSW
+from oracle import index_file
+
+pytestmark = pytest.mark.gpu
+
+PIECE = 8 << 20
+
+
+def _index(n, d, **opt):
+  rng = np.random.default_rng(n + d)
+  base = rng.integers(-8, 9, (n, d)).astype(np.float32)
+  opt = dict(dict(dist_type="l2", max_m=4, max_m0=8, ef_construction=8, seed=5, batch_max=4096), **opt)
+  eng = CuHNSW(engine_options(opt))
+  eng.set_data(base)
+  eng.build()
+  return eng, base, rng
+
+
+@pytest.mark.parametrize("d,topk", [(7, 1), (20, 100)])
+def test_host_searches_around_the_edges_of_the_staging_sizes(d, topk):
+  import torch
+  eng, _, rng = _index(3000, d)
+  per_query = 4 * (d + 2 * topk + 1)
+  in_place, piece = (256 << 10) // per_query, (PIECE - 1024) // per_query
+  q = rng.standard_normal((5 * piece + 13, d)).astype(np.float32)
+  dq = torch.from_numpy(q).cuda()
+  ids = torch.empty((len(q), topk), dtype=torch.int32, device="cuda")
+  dist = torch.empty((len(q), topk), dtype=torch.float32, device="cuda")
+  found = torch.empty((len(q),), dtype=torch.int32, device="cuda")
+  eng.obj.search_knn_device(dq.data_ptr(), len(q), topk, 100, ids.data_ptr(), dist.data_ptr(), found.data_ptr())
+  eng.obj.synchronize()
+  want = ids.cpu().numpy(), dist.cpu().numpy(), found.cpu().numpy()
+  for nq in (1, in_place, in_place + 1, piece, piece + 1, 2 * piece + 1, len(q)):
+    got = eng.search_knn(q[:nq], topk, 100)
+    assert (got[0] == want[0][:nq]).all() and (got[2] == want[2][:nq]).all(), nq
+    assert_same_bits(got[1], want[1][:nq])
+
+
+@pytest.mark.parametrize("n,d,row_dtype,max_m0", [(40_000, 104, "f32", 8), (33_001, 77, "f32", 64),
+                                                  (50_001, 50, "f16", 33), (300, 9, "bf16", 8)])
+def test_rows_graph_and_files_of_several_pieces(n, d, row_dtype, max_m0, tmp_path):
+  """Rows with and without padding, 16-bit rows, adjacency tables and files of more than three pieces; a file saved
+  over a longer one is cut to its length; small integers are exact in every row type."""
+  eng, base, _ = _index(n, d, row_dtype=row_dtype, max_m0=max_m0)
+  path = str(tmp_path / "x.index")
+  with open(path, "wb") as out:
+    out.write(b"\xff" * (n * (4 * d + 4 * max_m0 + 12) + (1 << 20)))
+  eng.save_index(path)
+  levels, rows0, rows_u = eng.obj.get_graph()
+  g = index_file.load(path, "l2")
+  assert (g.vec == base).all() and (g.levels == levels).all() and (g.rows0 == rows0).all()
+  assert (g.rowsU == rows_u[:g.rowsU.shape[0]]).all() and (g.labels == np.arange(n)).all()
+  labels = np.arange(n, dtype=np.int64) * (1 << 33) + 7
+  index_file.save(path, g, g.header["mult"], g.header["ef_construction"], labels=labels)
+  other = CuHNSW(engine_options(dict(dist_type="l2", row_dtype=row_dtype)))
+  other.load_index(path)
+  again = str(tmp_path / "y.index")
+  other.save_index(again)
+  assert open(path, "rb").read() == open(again, "rb").read()
+  assert (other.obj.get_graph()[1] == rows0).all()
+
+
+@pytest.mark.parametrize("rows,d", [(1, 3), (40_000, 50), (42_000, 50), (70_001, 33)])
+def test_set_data_copies_and_normalises_like_one_thread(rows, d):
+  """Below and above the size from which several threads share the work; a second corpus over the first."""
+  rng = np.random.default_rng(rows)
+  eng = CuHNSW(engine_options(dict(dist_type="dot", nrz=True)))
+  for _ in range(2):
+    x = rng.standard_normal((rows, d))
+    eng.set_data(x)
+    want = np.array(x, dtype=np.float32)
+    want /= np.linalg.norm(want, axis=1, keepdims=True)
+    assert_same_bits(eng.data, want)
+  kept = eng.data
+  before = kept.copy()
+  eng.set_data(-x)
+  assert_same_bits(kept, before)  # an array the caller holds is not written over
