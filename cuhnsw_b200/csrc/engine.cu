@@ -152,8 +152,8 @@ int Engine::EnsureDevice() {
   device_ = dev;
   sm_count_ = prop.multiProcessorCount;
   smem_optin_ = prop.sharedMemPerBlockOptin;
-  CU(counters_.alloc(8));
-  CU(cudaMemset(counters_.get(), 0, 8 * sizeof(unsigned long long)));
+  CU(counters_.alloc(8 + kSearchLanes));
+  CU(cudaMemset(counters_.get(), 0, counters_.size() * sizeof(unsigned long long)));
   Log(3, "device %d: %s, sm_%d%d, %d SMs, %zu B shared memory per block", dev, prop.name, prop.major, prop.minor,
       sm_count_, smem_optin_);
   return kOk;
@@ -615,7 +615,7 @@ int Engine::SearchGraphDevice(const float* d_q, long long nq, int topk, int ef, 
   p.out_found = d_found;
   SearchLane* lane = nullptr;
   if ((rc = LaneFor(stream_, &lane)) != kOk) return rc;
-  p.ticket = lane->ticket.get();
+  p.ticket = counters_.get() + 8 + (lane - lanes_);
   p.stats = stats_on_ ? counters_.get() + 4 : nullptr;
   SearchSchedule sched;
   // the launcher schedules only batches of more than one wave of its kernel (4 CTAs to 32 warps per SM);
@@ -640,7 +640,6 @@ int Engine::LaneFor(cudaStream_t stream, SearchLane** out) {
       if (pick->pending) CU(cudaEventSynchronize(pick->done));  // its last search is over before another stream uses it
       pick->pending = false;
     }
-    if (!pick->ticket.get()) CU(pick->ticket.alloc(1));
     if (!pick->done) CU(cudaEventCreateWithFlags(&pick->done, cudaEventDisableTiming));
     pick->stream = stream;
     pick->used = true;
@@ -666,10 +665,13 @@ int Engine::WaitForSearches() {
 }
 
 int Engine::PrepareSchedule(long long nq, SearchLane* lane, SearchSchedule* s) {
+  // batches of up to kBlockSortMax queries are ordered without the last two arrays and the sort's storage
+  const bool large = nq > kBlockSortMax;
   if (nq > lane->capacity) {
+    lane->capacity = 0;  // (what there is goes back first)
     const long long cap = std::max<long long>(nq, 1024);
-    CU(lane->sched.reserve((size_t)cap * 6));
-    CU(lane->sched_tmp.reserve(search_schedule_tmp_bytes(cap)));
+    CU(lane->sched.reserve((size_t)cap * (large ? 6 : 4)));
+    if (large) CU(lane->sched_tmp.reserve(search_schedule_tmp_bytes(cap)));
     lane->capacity = cap;
   }
   unsigned* base = lane->sched.get();
@@ -678,9 +680,9 @@ int Engine::PrepareSchedule(long long nq, SearchLane* lane, SearchSchedule* s) {
   s->entry_node = reinterpret_cast<int*>(base);
   s->entry_dist = reinterpret_cast<float*>(base + c);
   s->keys = base + 2 * c;
-  s->keys_sorted = base + 3 * c;
-  s->index = reinterpret_cast<int*>(base + 4 * c);
-  s->order = reinterpret_cast<int*>(base + 5 * c);
+  s->order = reinterpret_cast<int*>(base + 3 * c);
+  s->keys_sorted = large ? base + 4 * c : nullptr;
+  s->index = large ? reinterpret_cast<int*>(base + 5 * c) : nullptr;
   s->sort_tmp = lane->sched_tmp.get();
   s->sort_tmp_bytes = lane->sched_tmp.size();
   return kOk;
@@ -747,6 +749,15 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
   if (nslots == 0) return kOk;
   *handled = true;
   const cudaStream_t own = stream_;
+  // every stream's scratch before the first launch: an allocation waits for what runs
+  for (int i = 0; i < nslots && pieces > 1 && !rc; ++i) {
+    SearchLane* lane = nullptr;
+    SearchSchedule sched;
+    if ((rc = LaneFor(slots[i].stream, &lane)) == kOk && (rc = ReserveIo(lane, IoOf(most, topk))) == kOk &&
+        opt_.search_schedule)
+      rc = PrepareSchedule(most, lane, &sched);
+  }
+  if (rc) return rc;
   // waits for a piece and hands its results to the caller
   auto collect = [&](Piece& s) -> cudaError_t {
     const cudaError_t e = cudaStreamSynchronize(s.stream);
@@ -788,7 +799,10 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
     rc = small ? SearchGraphDevice(s.q, s.count, topk, ef, s.ids, s.dist, s.found)
                : SearchGraphCopied(s.q, s.count, topk, ef, s.ids, s.dist, s.found);
     stream_ = own;
-    if (rc) s.count = 0;
+    if (rc) {
+      cudaStreamSynchronize(s.stream);  // a copy from the buffer may be under way
+      s.count = 0;
+    }
   }
   // what is still in flight, oldest first
   for (long long i = pieces; i < pieces + nslots; ++i) {
@@ -830,21 +844,36 @@ int Engine::SearchGraphAsync(const float* q, long long nq, int topk, int ef, int
   return SearchGraphCopied(q, nq, topk, ef, nns, dist, found);
 }
 
+// queries | ids | distances | counts of a host-buffer search on the device, on 256-byte boundaries
+Engine::LaneIo Engine::IoOf(long long nq, int topk) const {
+  const auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  LaneIo io;
+  io.ids = up((size_t)nq * d_ * 4);
+  io.dist = io.ids + up((size_t)nq * topk * 4);
+  io.found = io.dist + up((size_t)nq * topk * 4);
+  io.bytes = io.found + up((size_t)nq * 4);
+  return io;
+}
+int Engine::ReserveIo(SearchLane* lane, const LaneIo& io) {
+  CU(lane->io.reserve(io.bytes));
+  return kOk;
+}
+
 // host buffers in and out through the stream's device copies of them
 int Engine::SearchGraphCopied(const float* q, long long nq, int topk, int ef, int* nns, float* dist, int* found) {
   SearchLane* lane = nullptr;
   int rc = LaneFor(stream_, &lane);
   if (rc) return rc;
-  CU(lane->q.reserve((size_t)nq * d_));
-  CU(lane->ids.reserve((size_t)nq * topk));
-  CU(lane->dist.reserve((size_t)nq * topk));
-  CU(lane->found.reserve((size_t)nq));
-  CU(cudaMemcpyAsync(lane->q.get(), q, (size_t)nq * d_ * sizeof(float), cudaMemcpyHostToDevice, stream_));
-  rc = SearchGraphDevice(lane->q.get(), nq, topk, ef, lane->ids.get(), lane->dist.get(), lane->found.get());
+  const LaneIo io = IoOf(nq, topk);
+  if ((rc = ReserveIo(lane, io)) != kOk) return rc;
+  unsigned char* base = lane->io.get();
+  CU(cudaMemcpyAsync(base, q, (size_t)nq * d_ * sizeof(float), cudaMemcpyHostToDevice, stream_));
+  rc = SearchGraphDevice(reinterpret_cast<const float*>(base), nq, topk, ef, reinterpret_cast<int*>(base + io.ids),
+                         reinterpret_cast<float*>(base + io.dist), reinterpret_cast<int*>(base + io.found));
   if (rc) return rc;
-  CU(cudaMemcpyAsync(nns, lane->ids.get(), (size_t)nq * topk * sizeof(int), cudaMemcpyDeviceToHost, stream_));
-  CU(cudaMemcpyAsync(dist, lane->dist.get(), (size_t)nq * topk * sizeof(float), cudaMemcpyDeviceToHost, stream_));
-  CU(cudaMemcpyAsync(found, lane->found.get(), (size_t)nq * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  CU(cudaMemcpyAsync(nns, base + io.ids, (size_t)nq * topk * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  CU(cudaMemcpyAsync(dist, base + io.dist, (size_t)nq * topk * sizeof(float), cudaMemcpyDeviceToHost, stream_));
+  CU(cudaMemcpyAsync(found, base + io.found, (size_t)nq * sizeof(int), cudaMemcpyDeviceToHost, stream_));
   return MarkLane(lane);  // the staging buffers are in use until the copies are through
 }
 

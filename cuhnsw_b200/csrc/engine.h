@@ -182,10 +182,10 @@ class Engine {
   DevBuf<float> vec_;
   DevBuf<int> rows0_, rowsU_, levels_d_, upper_base_d_, labels_d_;
   DevBuf<unsigned> records_[Pipeline::kDepth];  // pieces of an index file on their way (8 MB each, once a file was used)
-  DevBuf<unsigned long long> counters_;  // [0] search ticket, [1..2] build tickets, [4..7] stats
+  DevBuf<unsigned long long> counters_;  // [0] search ticket, [1..2] build tickets, [4..7] stats, [8..] tickets of the search lanes
   bool stats_on_ = false;
   // Scratch of one search in flight: its ticket counter and the grow-only arrays of the
-  // longest-first schedule (six words per query + sort storage).  A search uses the set that belongs to the
+  // longest-first schedule (four words per query; six and the sort's storage for large batches).  A search uses the set that belongs to the
   // stream it is enqueued on, so searches enqueued on different streams can run at the same time: the tail of
   // one batch (a launch lasts as long as its longest walk) overlaps with the next batch.  A stream beyond
   // kSearchLanes takes over the least recently used set after waiting for the search that used it last (through
@@ -196,14 +196,17 @@ class Engine {
     unsigned long long stamp = 0;
     cudaEvent_t done = nullptr;  // recorded behind the last thing a search put on the stream
     bool pending = false;
-    DevBuf<unsigned long long> ticket;
     DevBuf<unsigned> sched;
     DevBuf<unsigned char> sched_tmp;
     long long capacity = 0;
     // grow-only device copies of the host-buffer searches' queries and results
-    DevBuf<float> q, dist;
-    DevBuf<int> ids, found;
+    DevBuf<unsigned char> io;
   };
+  struct LaneIo {
+    size_t ids, dist, found, bytes;  // offsets
+  };
+  LaneIo IoOf(long long nq, int topk) const;
+  int ReserveIo(SearchLane* lane, const LaneIo& io);
   static constexpr int kSearchLanes = 8;
   SearchLane lanes_[kSearchLanes];
   unsigned long long lane_clock_ = 0;

@@ -16,9 +16,6 @@
 namespace hnsw {
 
 constexpr int kWarpsPerCta = 2;
-// batches of up to this many queries are ordered by one CTA (sort_schedule_kernel) instead of the four kernels
-// of a device-wide radix sort (10 000 queries on a B200: 19 us in one launch against 27 us in four)
-constexpr long long kBlockSortMax = 10240;
 
 template <class Dist, bool kReverse>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, Dist::kSearchMinCtas)
@@ -109,8 +106,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) entry_kernel(SearchParams p
     // sort key: farthest entry first.  Small batches are sorted by one CTA (sort_schedule_kernel), which wants
     // the query number in the low half of the word.
     const unsigned key = ~f2ord(dcur);
-    s.keys[qi] = p.nq <= kBlockSortMax ? ((key & 0xffff0000u) | (unsigned)qi) : key;
-    s.index[qi] = (int)qi;
+    if (p.nq <= kBlockSortMax) {
+      s.keys[qi] = (key & 0xffff0000u) | (unsigned)qi;
+    } else {
+      s.keys[qi] = key;
+      s.index[qi] = (int)qi;
+    }
     if (p.stats) {
       atomicAdd(p.stats + 0, (unsigned long long)wc.evals);
       atomicAdd(p.stats + 2, (unsigned long long)wc.sweeps);
