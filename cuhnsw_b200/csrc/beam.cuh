@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "distance.cuh"
 #include "kernels.h"
+#include "smem.cuh"
 
 namespace hnsw {
 
@@ -45,30 +46,24 @@ __host__ __device__ inline int visited_entry_bytes(long long n, int entries) {
   return tag_bits <= 15 ? 2 : 4;
 }
 
-// Per-warp shared-memory state.
-struct WarpList {
-  unsigned long long* keys;  // ascending (distance, id); capacity `cap`
-  int* spos;                 // 32 ints of scratch
-  unsigned* vt;              // visited table: buckets of two tags (2 x 16 bit in one word, or 2 x 32 bit)
-  unsigned hmask;            // 2^B - 1, B = id_bits(n)
-  int tag_bits;              // low bits of the hash kept as the tag; the rest is the bucket number
+// Lossy set of node ids in shared memory with no false positives.  id -> h = id * odd mod 2^B is a bijection on B-bit
+// numbers, so (bucket, tag) = (high bits, low bits) of h identifies the id exactly and only the tag has to be stored.
+// Each bucket keeps its two most recent tags; a displaced id can only cause a repeated distance evaluation, never a
+// different result, because duplicates are rejected when merging into the list and a key that left the list can
+// never re-enter.
+struct VisitedTable {
+  unsigned vt;     // shared-memory address: buckets of two tags (2 x 16 bit in one word, or 2 x 32 bit)
+  unsigned hmask;  // 2^B - 1, B = id_bits(n)
+  int tag_bits;    // low bits of the hash kept as the tag; the rest is the bucket number
   unsigned tag_mask;
-  bool wide;                 // 32-bit tags
+  bool wide;       // 32-bit tags
   int vbytes;
-  int cap;
-  int size;
-  int cursor;  // every key before `cursor` is expanded
-  unsigned long long worst;  // largest key of a full list, KEY_MAX while there is room
 
-  __host__ __device__ static size_t smem_bytes(int cap, int entries, long long n) {
-    return (size_t)((cap + 31) / 32 * 32) * 8 + 32 * 4 + (size_t)entries * visited_entry_bytes(n, entries);
+  __host__ __device__ static size_t smem_bytes(int entries, long long n) {
+    return (size_t)entries * visited_entry_bytes(n, entries);
   }
-  __device__ __forceinline__ void bind(void* smem, int cap_, int entries, long long n) {
-    keys = reinterpret_cast<unsigned long long*>(smem);
-    int capr = (cap_ + 31) / 32 * 32;
-    spos = reinterpret_cast<int*>(keys + capr);
-    vt = reinterpret_cast<unsigned*>(spos + 32);
-    cap = cap_;
+  __device__ __forceinline__ void bind_table(unsigned smem, int entries, long long n) {
+    vt = smem;
     const int b = id_bits(n);
     int kb = 0;
     while ((2 << kb) < entries) ++kb;
@@ -77,6 +72,60 @@ struct WarpList {
     tag_mask = (1u << tag_bits) - 1u;
     wide = tag_bits > 15;
     vbytes = entries * (wide ? 4 : 2);
+  }
+  // empties the table; warp w of `warps` does its share
+  __device__ __forceinline__ void clear(int w, int warps) {
+    for (int i = w * 32 + lane_id(); i < vbytes / 16; i += warps * 32) sts128(vt + 16 * i, ~0u, ~0u, ~0u, ~0u);
+  }
+  // Is the id in the table?  Any value may be asked for; no branch but the one on the table's kind, so that a warp
+  // with a few live lanes runs straight through.
+  __device__ __forceinline__ bool knows(int id) const {
+    const unsigned h = ((unsigned)id * 2654435761u) & hmask;
+    const unsigned tag = h & tag_mask;
+    if (!wide) {
+      const unsigned x = lds32(vt + 4 * (h >> tag_bits)) ^ (tag * 0x10001u);
+      return (x & 0xffffu) == 0u || x < 0x10000u;
+    }
+    const uint2 w = lds64(vt + 8 * (h >> tag_bits));
+    return w.x == tag || w.y == tag;
+  }
+  // the same, and an id that is not there enters if `on`
+  __device__ __forceinline__ bool test_and_set(int id, bool on = true) {
+    const unsigned h = ((unsigned)id * 2654435761u) & hmask;
+    const unsigned tag = h & tag_mask;
+    if (!wide) {
+      const unsigned at = vt + 4 * (h >> tag_bits);
+      const unsigned w = lds32(at), x = w ^ (tag * 0x10001u);
+      const bool known = (x & 0xffffu) == 0u || x < 0x10000u;
+      if (on && !known) sts32(at, (w << 16) | tag);
+      return known;
+    }
+    const unsigned at = vt + 8 * (h >> tag_bits);
+    const uint2 w = lds64(at);
+    const bool known = w.x == tag || w.y == tag;
+    if (on && !known) sts64(at, tag, w.x);
+    return known;
+  }
+};
+
+// Per-warp shared-memory state.
+struct WarpList : VisitedTable {
+  unsigned long long* keys;  // ascending (distance, id); capacity `cap`
+  int* spos;                 // 32 ints of scratch
+  int cap;
+  int size;
+  int cursor;  // every key before `cursor` is expanded
+  unsigned long long worst;  // largest key of a full list, KEY_MAX while there is room
+
+  __host__ __device__ static size_t smem_bytes(int cap, int entries, long long n) {
+    return (size_t)((cap + 31) / 32 * 32) * 8 + 32 * 4 + VisitedTable::smem_bytes(entries, n);
+  }
+  __device__ __forceinline__ void bind(void* smem, int cap_, int entries, long long n) {
+    keys = reinterpret_cast<unsigned long long*>(smem);
+    int capr = (cap_ + 31) / 32 * 32;
+    spos = reinterpret_cast<int*>(keys + capr);
+    bind_table(kept(smem_addr(spos + 32)), entries, n);
+    cap = cap_;
     size = 0;
     cursor = 0;
     worst = KEY_MAX;
@@ -85,34 +134,11 @@ struct WarpList {
   // O(nodes touched); the reference resets through a touched-slot list
   // (cuda_search_kernels.cuh:145-147).
   __device__ __forceinline__ void reset() {
-    uint4* p = reinterpret_cast<uint4*>(vt);
-    const uint4 e = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (int i = lane_id(); i < vbytes / 16; i += 32) p[i] = e;
+    clear(0, 1);
     size = 0;
     cursor = 0;
     worst = KEY_MAX;
     __syncwarp();
-  }
-  // Lossy set with no false positives.  id -> h = id * odd mod 2^B is a bijection on B-bit
-  // numbers, so (bucket, tag) = (high bits, low bits) of h identifies the id exactly and only
-  // the tag has to be stored.  Each bucket keeps its two most recent tags; a displaced id can
-  // only cause a repeated distance evaluation, never a different result, because duplicates are
-  // rejected when merging into the list and a key that left the list can never re-enter.
-  __device__ __forceinline__ bool test_and_set(int id) {
-    const unsigned h = ((unsigned)id * 2654435761u) & hmask;
-    const unsigned bucket = h >> tag_bits;
-    const unsigned tag = h & tag_mask;
-    if (!wide) {
-      const unsigned w = vt[bucket];
-      if ((w & 0xffffu) == tag || (w >> 16) == tag) return true;
-      vt[bucket] = (w << 16) | tag;
-      return false;
-    }
-    uint2* p = reinterpret_cast<uint2*>(vt) + bucket;
-    const uint2 w = *p;
-    if (w.x == tag || w.y == tag) return true;
-    *p = make_uint2(tag, w.x);
-    return false;
   }
   __device__ __forceinline__ void mark(int id) {
     if (lane_id() == 0) test_and_set(id);

@@ -24,6 +24,7 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "smem.cuh"
 
 namespace hnsw {
 
@@ -111,6 +112,15 @@ __device__ __forceinline__ void fma4(float4& acc, const float4& a, const float4&
   }
 }
 
+// fma4 into accumulators that hold zero: the same values but for the sign of a zero, which no distance keeps
+template <bool kDot>
+__device__ __forceinline__ float4 first4(const float4& a, const float4& b) {
+  // (__fmul_rn: the compiler must not fuse these products with the additions of fold4)
+  if (kDot) return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+  const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z, dw = a.w - b.w;
+  return make_float4(__fmul_rn(dx, dx), __fmul_rn(dy, dy), __fmul_rn(dz, dz), __fmul_rn(dw, dw));
+}
+
 __device__ __forceinline__ float fold4(const float4& a) { return (a.x + a.y) + (a.z + a.w); }
 
 // ---------------------------------------------------------------------------
@@ -135,12 +145,17 @@ struct DistSmall {
   // rows of 128 floats are 15 % slower there (1 M x 128: 0.477 against 0.415 s)
   static constexpr int kBuildMinCtas = C <= 3 ? 16 : 12;
   static constexpr int kWarpsPerSmTarget = 32;
+  static constexpr bool kSharedQuery = false;  // every warp keeps its own copy of the query
   __host__ __device__ static constexpr size_t smem_bytes(int) { return 0; }
 
   VecTable t;
   float4 q[C];
+  int lane_no;
 
-  __device__ __forceinline__ void init(const VecTable& tab, void*) { t = tab; }
+  __device__ __forceinline__ void init(const VecTable& tab, void*) {
+    t = tab;
+    lane_no = lane_number();
+  }
 
   // query from an unpadded row of d floats in global memory
   __device__ __forceinline__ void load_query(const float* qp) {
@@ -196,6 +211,40 @@ struct DistSmall {
     }
     return result;
   }
+
+  // Rows r = 8 w .. 8 w + 7, 8 (w + warps) ..., below n, of a pool of (id, address) pairs in shared memory: the words
+  // (distance image, id) of row r go to its address.  A team takes two rows at a time, whose lane sums are folded together: the first exchange of
+  // the butterfly leaves one row in each half of the team (the pairs that are added are the same, so are the
+  // sums), and eight rows cost 5 shuffles instead of the 16 of two passes of eval().
+  __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps) {
+    if (t.dist_type == DIST_DOT) eval_pool_t<true>(pool, n, w, warps);
+    else eval_pool_t<false>(pool, n, w, warps);
+  }
+  template <bool kDot>
+  __device__ __forceinline__ void eval_pool_t(unsigned pool, int n, int w, int warps) {
+    const int team = lane_no >> 3, tl = lane_no & 7;
+    const bool second = tl & 4;
+    for (int r0 = 8 * w; r0 < n; r0 += 8 * warps) {
+      const int ra = r0 + team, rb = ra + 4;
+      // rows past n are folded onto the last one: a harmless repeated load whose result nobody writes
+      const uint2 ea = lds64(pool + 8 * min(ra, n - 1)), eb = lds64(pool + 8 * min(rb, n - 1));
+      float4 va[C], vb[C];
+      Row::template load<C, 8, true>(t.vec + (size_t)ea.x * t.row_bytes, tl, 0, t.nchunk, va);
+      Row::template load<C, 8, true>(t.vec + (size_t)eb.x * t.row_bytes, tl, 0, t.nchunk, vb);
+      float4 aa = first4<kDot>(q[0], va[0]), ab = first4<kDot>(q[0], vb[0]);
+#pragma unroll
+      for (int c = 1; c < C; ++c) {
+        fma4(aa, q[c], va[c], kDot ? DIST_DOT : DIST_L2);
+        fma4(ab, q[c], vb[c], kDot ? DIST_DOT : DIST_L2);
+      }
+      const float sa = fold4(aa), sb = fold4(ab);
+      float s = (second ? sb : sa) + __shfl_xor_sync(FULL, second ? sa : sb, 4);
+      s += __shfl_xor_sync(FULL, s, 2);
+      s += __shfl_xor_sync(FULL, s, 1);
+      if (kDot) s = -s;
+      if ((tl & 3) == 0 && (second ? rb : ra) < n) sts64(second ? eb.y : ea.y, f2ord(s), second ? eb.x : ea.x);
+    }
+  }
 };
 
 // ---------------------------------------------------------------------------
@@ -212,6 +261,7 @@ struct DistLargeT {
   static constexpr int kSearchMinCtas = kMinCtasT;
   static constexpr int kBuildMinCtas = 8;
   static constexpr int kWarpsPerSmTarget = 16;
+  static constexpr bool kSharedQuery = true;   // one copy in shared memory
   __host__ __device__ static constexpr size_t smem_bytes(int d) { return (size_t)((d + 127) / 128) * 128 * sizeof(float); }
 
   VecTable t;
@@ -280,6 +330,17 @@ struct DistLargeT {
       }
     }
     return result;
+  }
+  // Rows r = w, w + warps, ... below n of a pool of (id, address) pairs in shared memory: the words (distance image,
+  // id) of row r go to its address.
+  __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps) {
+    const int lane = lane_id();
+    for (int r0 = w; r0 < n; r0 += 32 * warps) {
+      const int cnt = min(32, (n - r0 + warps - 1) / warps);
+      const uint2 e = lds64(pool + 8 * min(r0 + lane * warps, n - 1));
+      const float s = eval((int)e.x, cnt);
+      if (lane < cnt) sts64(e.y, f2ord(s), e.x);
+    }
   }
 };
 

@@ -152,6 +152,7 @@ int Engine::EnsureDevice() {
   device_ = dev;
   sm_count_ = prop.multiProcessorCount;
   smem_optin_ = prop.sharedMemPerBlockOptin;
+  smem_per_sm_ = prop.sharedMemPerMultiprocessor;
   CU(counters_.alloc(8 + kSearchLanes));
   CU(cudaMemset(counters_.get(), 0, counters_.size() * sizeof(unsigned long long)));
   Log(3, "device %d: %s, sm_%d%d, %d SMs, %zu B shared memory per block", dev, prop.name, prop.major, prop.minor,
@@ -452,13 +453,13 @@ int Engine::ResolveVsize(int cap, long long nq, int* vsize) const {
     // Largest table that still lets the kernel keep its target number of warps resident per SM
     // (the walk is latency bound: resident warps matter more than a few repeated evaluations),
     // but never below ~4 entries per list slot, where repeats explode.
-    // Wide rows and few queries: the kernels chosen there keep 4 CTAs per SM resident whatever the table
+    // Wide rows and few queries: the kernel chosen there keeps 4 CTAs per SM resident whatever the table
     // size, and a repeated evaluation re-reads kilobytes.  Measured on 1M x 960, 1000 queries, ef 500:
-    // 3576 evaluations per query and 5.67 ms with 2048 entries, 2099 and 4.98 ms with 16384.
+    // 3576 evaluations per query with 2048 entries, 2099 with 16384.
     const int kind = nq < 0 ? kSearchWarp
-                            : search_kernel_kind(d_, nq, opt_.search_team, opt_.reverse_cand ? 1 : 0, sm_count_);
-    const int warps = d_ <= 128 ? 32 : kind == kSearchTeam ? 4 : kind == kSearchWarpDeep ? 8 : 16;
-    const int top = kind == kSearchTeam ? 16384 : kind == kSearchWarpDeep ? 8192 : 4096;
+                            : search_kernel_kind(d_, cap, nq, opt_.search_team, opt_.reverse_cand ? 1 : 0, sm_count_);
+    const int warps = d_ <= 128 ? 32 : kind == kSearchWarpDeep ? 8 : 16;
+    const int top = kind == kSearchWarpDeep ? 8192 : 4096;
     const long long budget = (long long)smem_optin_ / warps - 640;
     const int floor_entries = std::min(4096, std::max(512, next_pow2(4ll * cap)));
     v = top;
@@ -606,6 +607,9 @@ int Engine::SearchGraphDevice(const float* d_q, long long nq, int topk, int ef, 
   p.topk = topk;
   p.ef = ef;
   p.vsize = vsize;
+  p.table_request = opt_.visited_table_size;
+  p.smem_optin = smem_optin_;
+  p.smem_per_sm = smem_per_sm_;
   p.reverse_cand = opt_.reverse_cand ? 1 : 0;
   p.team = opt_.search_team;
   p.smem_per_warp = 0;
@@ -618,9 +622,9 @@ int Engine::SearchGraphDevice(const float* d_q, long long nq, int topk, int ef, 
   p.ticket = counters_.get() + 8 + (lane - lanes_);
   p.stats = stats_on_ ? counters_.get() + 4 : nullptr;
   SearchSchedule sched;
-  // the launcher schedules only batches of more than one wave of its kernel (4 CTAs to 32 warps per SM);
+  // the launcher schedules only batches of more than one wave of its kernel (2 CTAs to 32 warps per SM);
   // below the smallest wave there is nothing to prepare
-  const bool schedule = nq > (long long)sm_count_ * 4 && opt_.search_schedule;
+  const bool schedule = nq > (long long)sm_count_ * 2 && opt_.search_schedule;
   if (schedule && (rc = PrepareSchedule(nq, lane, &sched)) != kOk) return rc;
   CU(launch_search(p, sm_count_, stream_, schedule ? &sched : nullptr));
   return MarkLane(lane);
@@ -910,6 +914,9 @@ int Engine::SearchGraphStatic(const float* q, long long nq, int topk, int ef, in
   p.topk = topk;
   p.ef = ef;
   p.vsize = vsize;
+  p.table_request = opt_.visited_table_size;
+  p.smem_optin = smem_optin_;
+  p.smem_per_sm = smem_per_sm_;
   p.reverse_cand = opt_.reverse_cand ? 1 : 0;
   p.team = opt_.search_team;
   p.smem_per_warp = 0;

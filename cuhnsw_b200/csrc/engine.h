@@ -41,7 +41,7 @@ struct Options {
   int visited_list_size = 8192;
   bool nrz = false;
   bool reverse_cand = false;
-  int search_team = -1;  // d > 128: 1 = CTA per query, 0 = warp per query, -1 = chosen by batch size
+  int search_team = -1;  // 1 = CTA per query, 0 = warp per query, -1 = chosen by batch size
   std::string row_dtype = "f32";  // "f16" / "bf16": rows stored in 16 bits, distances in fp32 over the stored values
   bool search_schedule = true;  // batches of more than one wave: serve the queries with the farthest entry first
   bool zero_copy = true;        // host-buffer searches on page-locked buffers: the kernels read and write them in place
@@ -160,7 +160,7 @@ class Engine {
   std::string err_;
   int device_ = -1;
   int sm_count_ = 0;
-  size_t smem_optin_ = 0;
+  size_t smem_optin_ = 0, smem_per_sm_ = 0;
   cudaStream_t stream_ = nullptr;  // legacy default stream unless SetStream is called
 
   long long n_ = 0;

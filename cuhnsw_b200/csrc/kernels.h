@@ -30,9 +30,12 @@ struct SearchParams {
   long long nq;
   int topk;
   int ef;
-  int vsize;             // visited table entries per warp (power of two)
+  int vsize;             // visited table entries per warp (power of two); one CTA per query: chosen by its launcher
+  int table_request = 0; // the option visited_table_size: entries per query the caller wants, 0 = by size
+  size_t smem_optin = 0; // shared memory a CTA / an SM can have
+  size_t smem_per_sm = 0;
   int reverse_cand;      // expand the farthest unexpanded key first
-  int team = -1;         // rows wider than 128 floats: 1 = one CTA per query, 0 = one warp per query, -1 = by batch size
+  int team = -1;         // 1 = one CTA per query, 0 = one warp per query, -1 = by batch size
   int smem_per_warp;     // filled by the launcher
   const int* labels;     // optional id -> label map (index loaded from a file)
   int* out_ids;          // nq x topk
@@ -74,12 +77,16 @@ size_t search_schedule_tmp_bytes(long long nq);
 cudaError_t launch_search(const SearchParams& p, int sm_count, cudaStream_t stream,
                           const SearchSchedule* sched = nullptr);
 size_t search_smem_per_cta(int d, int ef, int vsize, long long n);
-// which search kernel a batch gets: rows <= 128 floats; wide rows with many / some / few queries
+// which search kernel a batch gets: one warp per query (narrow rows; wide rows; wide rows, few queries) or one CTA
 enum SearchKernelKind { kSearchWarpSmall = 0, kSearchWarp = 1, kSearchWarpDeep = 2, kSearchTeam = 3 };
-int search_kernel_kind(int d, long long nq, int team, int reverse_cand, int sm_count);
-// d > 128 only: one CTA of four warps per query, the extra warps share the distance evaluations
-cudaError_t launch_search_team(const SearchParams& p, int sm_count, cudaStream_t stream,
-                               const SearchSchedule* sched = nullptr);
+int search_kernel_kind(int d, int ef, long long nq, int team, int reverse_cand, int sm_count);
+// one CTA per query (search_walk.cuh), by row type
+cudaError_t launch_search_walk_f32(const SearchParams& p, int sm_count, cudaStream_t stream,
+                                   const SearchSchedule* sched);
+cudaError_t launch_search_walk_f16(const SearchParams& p, int sm_count, cudaStream_t stream,
+                                   const SearchSchedule* sched);
+cudaError_t launch_search_walk_bf16(const SearchParams& p, int sm_count, cudaStream_t stream,
+                                    const SearchSchedule* sched);
 // first stage of a scheduled search: descent of every query + sort; fills p.order / entry_node / entry_dist
 cudaError_t schedule_search(SearchParams& p, const SearchSchedule& sched, int sm_count, cudaStream_t stream);
 // search whose device staging and work ticket live in a fixed file-scope device array (no allocation)

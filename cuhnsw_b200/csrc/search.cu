@@ -243,14 +243,21 @@ size_t search_smem_per_cta(int d, int ef, int vsize, long long n) {
   return per_warp * kWarpsPerCta;
 }
 
-// Rows wider than 128 floats, fewer queries than warp slots: resident warps do not matter, the time of one
-// step does.  Up to 7 queries per SM one CTA of four warps per query shares the distance evaluations of every
-// step; up to 10 per SM one warp per query keeps 32 float4 loads in flight instead of 16.
-// Measured on 1M x 960 (ef 100 / 500): 100 queries 0.85 / 3.0 ms against 1.47 / 4.3 ms with one warp per
-// query, 1000 queries 1.48 / 5.9 against 1.74 / 6.0 ms, 1480 queries 1.79 / 7.2 against 2.17 / 6.8 ms.
-int search_kernel_kind(int d, long long nq, int team, int reverse_cand, int sm_count) {
+// One CTA per query while that is the faster way: up to so many queries per SM.  Narrow rows: the longer the walks, the
+// longer a launch waits for its last ones (ef 50: 14 queries per SM; in between in proportion; ef 200 and more: 42).  Wide
+// rows: 10, very wide ones 14.  Measured, one warp / one CTA per query, ms: 300 000 x 96 f16, 4000 queries, ef 50: 0.33 /
+// 0.36, ef 128: 0.76 / 0.64, ef 400: 2.13 / 1.60, 6000: 0.39 / 0.49, 0.79 / 0.84, 2.19 / 1.94; 200 000 x 300 f16, ef 100,
+// 1000 queries: 0.75 / 0.53, 2000: 0.73 / 0.74; 150 000 x 960, ef 500, 2000: 3.56 / 3.16, 3000: 4.12 / 4.43.  More figures
+// are in search_walk.cuh.  Expanding the farthest key first knows no next nodes to prepare: always one warp.
+static long long team_limit(int d, int ef, int sm_count) {
+  const int per_sm = d > 512 ? 14 : d > 128 ? 10 : ef * 27 / 128 < 14 ? 14 : ef * 27 / 128 > 42 ? 42 : ef * 27 / 128;
+  return (long long)sm_count * per_sm;
+}
+// Otherwise one warp per query; for few queries over wide rows with 32 float4 loads in flight instead of 16 (1 M x 960,
+// 1000 queries: 6.0 against 8.5 ms at ef 500).
+int search_kernel_kind(int d, int ef, long long nq, int team, int reverse_cand, int sm_count) {
+  if (!reverse_cand && (team == 1 || (team < 0 && nq <= team_limit(d, ef, sm_count)))) return kSearchTeam;
   if (d <= 128) return kSearchWarpSmall;
-  if (!reverse_cand && (team == 1 || (team < 0 && nq <= (long long)sm_count * 7))) return kSearchTeam;
   if (nq <= (long long)sm_count * 10) return kSearchWarpDeep;
   return kSearchWarp;
 }
@@ -264,16 +271,17 @@ static cudaError_t launch_search_rows(const SearchParams& p, int sm_count, cudaS
   if (d <= 64) return launch_search_t<typename E::D64>(p, sm_count, stream, sched);
   if (d <= 96) return launch_search_t<typename E::D96>(p, sm_count, stream, sched);
   if (d <= 128) return launch_search_t<typename E::D128>(p, sm_count, stream, sched);
-  switch (search_kernel_kind(d, p.nq, p.team, p.reverse_cand, sm_count)) {
-    case kSearchTeam: return launch_search_team(p, sm_count, stream, sched);
-    case kSearchWarpDeep: return launch_search_t<typename E::WideDeep>(p, sm_count, stream, sched);
-    default: break;
-  }
+  if (search_kernel_kind(d, p.ef, p.nq, p.team, p.reverse_cand, sm_count) == kSearchWarpDeep)
+    return launch_search_t<typename E::WideDeep>(p, sm_count, stream, sched);
   return launch_search_t<typename E::Wide>(p, sm_count, stream, sched);
 }
 
 cudaError_t launch_search(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   if (p.nq <= 0) return cudaSuccess;
+  if (search_kernel_kind(p.g.d, p.ef, p.nq, p.team, p.reverse_cand, sm_count) == kSearchTeam)
+    return p.g.rows16 == kRowsF16    ? launch_search_walk_f16(p, sm_count, stream, sched)
+           : p.g.rows16 == kRowsBF16 ? launch_search_walk_bf16(p, sm_count, stream, sched)
+                                     : launch_search_walk_f32(p, sm_count, stream, sched);
 #define CALL(R) launch_search_rows<R>(p, sm_count, stream, sched)
   return HNSW_WITH_ROWS(p.g.rows16, CALL);
 #undef CALL

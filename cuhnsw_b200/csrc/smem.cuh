@@ -1,0 +1,53 @@
+// Shared memory by 32-bit address.  A generic pointer into shared memory that is kept in a struct makes the compiler
+// build the shared window's base again at every access (a special-register read, a move and an add, 10 % of the
+// instructions of a walk); an address taken once is a register plus an immediate offset.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace hnsw {
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// an address the compiler keeps in a register instead of deriving it again at each use
+__device__ __forceinline__ unsigned kept(unsigned at) {
+  unsigned v;
+  asm volatile("mov.u32 %0, %1;" : "=r"(v) : "r"(at));
+  return v;
+}
+
+__device__ __forceinline__ unsigned lds32(unsigned at) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(unsigned at) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts32(unsigned at, unsigned v) {
+  asm volatile("st.shared.u32 [%0], %1;" : : "r"(at), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts64(unsigned at, unsigned x, unsigned y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" : : "r"(at), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sts128(unsigned at, unsigned x, unsigned y, unsigned z, unsigned w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" : : "r"(at), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ unsigned atomic_add_shared(unsigned at, unsigned v) {
+  unsigned old;
+  asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(at), "r"(v) : "memory");
+  return old;
+}
+
+__device__ __forceinline__ void atomic_or_shared(unsigned at, unsigned v) {
+  asm volatile("red.shared.or.b32 [%0], %1;" : : "r"(at), "r"(v) : "memory");
+}
+
+// The lane number, read once: the compiler does not fetch it again where registers are short.
+__device__ __forceinline__ int lane_number() {
+  unsigned v;
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(v));
+  return (int)v;
+}
+
+}  // namespace hnsw
