@@ -21,6 +21,7 @@
 
 #include "kernels.h"
 #include "beam.cuh"
+#include "walk.cuh"
 
 namespace hnsw {
 
@@ -251,6 +252,141 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_s
   }
 }
 
+// The same selection (select_neighbors with no newcomer) by the W warps of a CTA over the ascending keys of a KeyList:
+// each warp tests one of the next W candidates against the accepted neighbours and against the candidates before its
+// own; which of those were accepted is known once all have reported, so the outcome is that of one candidate after the
+// other.  ids, dist, flags: shared-memory addresses (kMaxLinks words each, W words).  Every warp returns the degree.
+template <class Dist, int W>
+__device__ __forceinline__ int select_team(Dist& de, unsigned keys, int nc, int m, int nn_num, int save_remains,
+                                           unsigned ids, unsigned dist, unsigned flags, int w, WalkCounters& wc) {
+  constexpr unsigned kTurnedDown = 0x80000000u;
+  const int lane = lane_number();
+  const int max_head = min(m, nc);
+  int tail = max_head - 1;
+  int head = min(nn_num, max_head);
+  for (int j = threadIdx.x; j < head; j += 32 * W) {
+    const uint2 k = lds64(keys + 8 * j);
+    sts32(ids + 4 * j, k.y >> 1);
+    sts32(dist + 4 * j, __float_as_uint(ord2f(k.x)));
+  }
+  __syncthreads();
+  for (int j0 = head; j0 < nc && head < m; j0 += W) {
+    unsigned flag = 0;
+    if (j0 + w < nc) {
+      const uint2 k = lds64(keys + 8 * (j0 + w));
+      const float cd = ord2f(__shfl_sync(FULL, k.x, 0));
+      de.load_query_row((int)(__shfl_sync(FULL, k.y, 0) >> 1));
+      for (int base = 0; base < head && flag == 0; base += 8) {
+        const int n = min(8, head - base);
+        const int id = lane < n ? (int)lds32(ids + 4 * (base + lane)) : 0;
+        const float dd = de.eval_eight(id, n);
+        wc.evals += n;
+        if (__any_sync(FULL, lane < n && cd > dd)) flag = kTurnedDown;
+      }
+      if (w > 0 && flag == 0) {
+        const int id = lane < w ? (int)(lds64(keys + 8 * (j0 + lane)).y >> 1) : 0;
+        const float dd = de.eval_eight(id, w);
+        wc.evals += w;
+        flag = __ballot_sync(FULL, lane < w && cd > dd);
+      }
+    }
+    if (lane == 0) sts32(flags + 4 * w, flag);
+    __syncthreads();
+    unsigned taken = kTurnedDown;
+    for (int u = 0; u < W && j0 + u < nc && head < m; ++u) {
+      const bool skip = (__shfl_sync(FULL, lds32(flags + 4 * u), 0) & taken) != 0;
+      int at = -1;
+      if (!skip) {
+        at = head++;
+        taken |= 1u << u;
+      } else if (tail >= head) {
+        at = tail--;
+      }
+      if (threadIdx.x == 0 && at >= 0) {
+        const uint2 k = lds64(keys + 8 * (j0 + u));
+        sts32(ids + 4 * at, k.y >> 1);
+        sts32(dist + 4 * at, __float_as_uint(ord2f(k.x)));
+      }
+    }
+    __syncthreads();
+  }
+  return save_remains ? max_head : head;
+}
+
+// Phase A for batches that leave the machine idle (the first of every level, and small corpora): one CTA per node, whose
+// walk prepares several nodes at a time (walk.cuh) and whose warps share the selection.
+constexpr int kTeamWarps = 4, kTeamNodes = 8;
+constexpr int kTeamTable = 4096;          // entries of its visited table
+// largest batch, in nodes per SM (whole builds with 0 / 10 / 20 / 40: 100 000 x 50 24.6 / 23.6 / 24.1 / 25.0 ms,
+// 1 M x 128 364 / 363 / 365 / 370, 30 000 x 960 340 / 332 / 338 / 366, 300 000 x 96 f16 35.0 / 34.4 / 34.8 / 35.9)
+constexpr int kTeamPerSm = 10;
+constexpr size_t kTeamSmem = 56u << 10;   // more shared memory than this leaves fewer than four CTAs per SM
+template <class Dist>
+using BuildWalk = Walk<Dist, kTeamWarps, kTeamNodes>;
+// walk, the selection's arrays, and for wide rows a query for each warp's candidate
+template <class Dist>
+inline size_t build_team_smem(const BuildLevel& L, int vsize) {
+  return (Dist::smem_bytes(L.g.d) * (1 + kTeamWarps) +
+          BuildWalk<Dist>::smem_bytes(L.ef_construction, L.stride, vsize, L.g.n) + kMaxLinks * 8 + 16 + 15) / 16 * 16;
+}
+template <class Dist>
+__global__ void __launch_bounds__(32 * kTeamWarps, Dist::kTeamMinCtas) build_search_team_kernel(BatchParams p, int vsize) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = lane_number();
+  const BuildLevel& L = p.L;
+  const VecTable tab = make_table(L.g);
+  unsigned char* at = smem;
+  BuildWalk<Dist> walk;
+  walk.de.init(tab, at);
+  at += Dist::smem_bytes(L.g.d);
+  const int w = walk.warp();
+  Dist own;  // this warp's candidate during selection, where the walk's query is shared
+  if (Dist::kSharedQuery) own.init(tab, at + (size_t)w * Dist::smem_bytes(L.g.d));
+  at += Dist::smem_bytes(L.g.d) * kTeamWarps;
+  const unsigned ids = kept(smem_addr(at)), dist = ids + 4 * kMaxLinks, flags = dist + 4 * kMaxLinks;
+  at += kMaxLinks * 8 + 16;
+  walk.bind(at, L.ef_construction, L.stride, vsize, L.g.n);
+  walk.rows = L.rows;
+  walk.upper_base = L.g.upper_base;
+  walk.level = L.level;
+  const auto select = [&](int nc) {
+    return select_team<Dist, kTeamWarps>(Dist::kSharedQuery ? own : walk.de, walk.list.keys, nc, L.max_m, p.nn_num,
+                                         L.save_remains, ids, dist, flags, w, walk.wc);
+  };
+  if (w > 0) {
+    while (walk.help(nullptr) != kWalkOver) select(walk.posted(WalkBoard<kTeamNodes>::kPool));
+    if (p.S.stats && lane == 0) atomicAdd(p.S.stats + 0, (unsigned long long)walk.wc.evals);
+    return;
+  }
+  for (;;) {
+    long long t = 0;
+    if (lane == 0) t = (long long)atomicAdd(p.S.ticket, 1ull);
+    t = __shfl_sync(FULL, t, 0);
+    if (t >= p.count) break;
+    const int s = L.nodes ? __ldg(L.nodes + p.first + t) : (int)(p.first + t);
+    walk.start(kWalkNode, nullptr, s);
+    // seeds: the node's current row (cuda_build_kernels.cuh:203-212)
+    walk.seed_row(walk.row_of(s));
+    walk.run();
+    if (lane == 0) sts32(walk.board + WalkBoard<kTeamNodes>::kPool, walk.list.size);
+    walk.post(kWalkSelect);
+    const int deg = select(walk.list.size);
+    int* so = p.S.st_ids + (size_t)t * L.stride;
+    float* sd = p.S.st_dist + (size_t)t * L.stride;
+    for (int j = lane; j < L.stride; j += 32) {
+      so[j] = (j < deg) ? (int)lds32(ids + 4 * j) : -1;
+      sd[j] = (j < deg) ? __uint_as_float(lds32(dist + 4 * j)) : 0.0f;
+    }
+    __syncwarp();
+  }
+  walk.finish();
+  if (p.S.stats && lane == 0) {
+    atomicAdd(p.S.stats + 0, (unsigned long long)walk.wc.evals);
+    atomicAdd(p.S.stats + 1, (unsigned long long)walk.wc.expansions);
+    atomicAdd(p.S.stats + 3, (unsigned long long)walk.wc.inserts);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // phase B: apply staged rows, emit proposals (one thread per row slot)
 // ---------------------------------------------------------------------------
@@ -430,7 +566,16 @@ static cudaError_t build_batch_t(const BuildLevel& L, const BuildScratch& S, lon
   p.nn_num = (int)(L.max_m * (double)L.heuristic_coef);
   cudaError_t e = cudaMemsetAsync(S.ticket, 0, 2 * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return e;
-  {
+  const int team_vsize = L.vsize_fixed ? L.vsize : L.vsize > kTeamTable ? L.vsize : kTeamTable;
+  const size_t team_smem = build_team_smem<Dist>(L, team_vsize);
+  if (!L.reverse_cand && count <= (long long)sm_count * kTeamPerSm && team_smem <= kTeamSmem) {
+    auto kern = build_search_team_kernel<Dist>;
+    int grid = 1;
+    e = grid_for(kern, team_smem, 32 * kTeamWarps, sm_count, count, &grid);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, 32 * kTeamWarps, team_smem, stream>>>(p, team_vsize);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  } else {
     size_t per_warp = build_smem_per_warp<Dist>(L.g.d, p.cap, L.vsize, L.g.n);
     p.per_warp = (int)per_warp;
     size_t smem = per_warp * kBuildWarps;

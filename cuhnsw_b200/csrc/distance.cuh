@@ -145,6 +145,7 @@ struct DistSmall {
   // rows of 128 floats are 15 % slower there (1 M x 128: 0.477 against 0.415 s)
   static constexpr int kBuildMinCtas = C <= 3 ? 16 : 12;
   static constexpr int kWarpsPerSmTarget = 32;
+  static constexpr int kTeamMinCtas = 5;  // construction with one CTA of four warps per node
   static constexpr bool kSharedQuery = false;  // every warp keeps its own copy of the query
   __host__ __device__ static constexpr size_t smem_bytes(int) { return 0; }
 
@@ -177,6 +178,10 @@ struct DistSmall {
   // Lane r (r < n <= 32, n >= 1) holds a row id; returns the distance to it in lane r.
   __device__ __forceinline__ float eval(int id, int n) {
     return t.dist_type == DIST_DOT ? eval_t<true, kBatch>(id, n) : eval_t<false, kBatch>(id, n);
+  }
+  // the same with the rows of two passes on their way together
+  __device__ __forceinline__ float eval_eight(int id, int n) {
+    return t.dist_type == DIST_DOT ? eval_t<true, 2>(id, n) : eval_t<false, 2>(id, n);
   }
   template <bool kDot, int kB>
   __device__ __forceinline__ float eval_t(int id, int n) {
@@ -261,6 +266,7 @@ struct DistLargeT {
   static constexpr int kSearchMinCtas = kMinCtasT;
   static constexpr int kBuildMinCtas = 8;
   static constexpr int kWarpsPerSmTarget = 16;
+  static constexpr int kTeamMinCtas = 4;
   static constexpr bool kSharedQuery = true;   // one copy in shared memory
   __host__ __device__ static constexpr size_t smem_bytes(int d) { return (size_t)((d + 127) / 128) * 128 * sizeof(float); }
 
@@ -331,6 +337,7 @@ struct DistLargeT {
     }
     return result;
   }
+  __device__ __forceinline__ float eval_eight(int id, int n) { return eval(id, n); }
   // Rows r = w, w + warps, ... below n of a pool of (id, address) pairs in shared memory: the words (distance image,
   // id) of row r go to its address.
   __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps) {

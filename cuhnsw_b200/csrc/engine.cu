@@ -562,6 +562,7 @@ int Engine::BuildGraph() {
     L.save_remains = opt_.save_remains ? 1 : 0;
     L.reverse_cand = opt_.reverse_cand ? 1 : 0;
     L.vsize = vsize;
+    L.vsize_fixed = opt_.visited_table_size > 0 ? 1 : 0;
     CU(launch_init_level(L, counters_.get() + 3, sm_count_, stream_));
     long long p = 0;
     while (p < nl) {

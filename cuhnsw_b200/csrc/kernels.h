@@ -113,6 +113,7 @@ struct BuildLevel {
   int save_remains;
   int reverse_cand;
   int vsize;
+  int vsize_fixed;       // vsize is the caller's own figure (option visited_table_size)
 };
 
 struct BuildScratch {

@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_walk_kernel(SearchParams
     qi = __shfl_sync(FULL, qi, 0);
     if (__any_sync(FULL, qi >= p.nq)) break;
     if (p.order) qi = __ldg(p.order + qi);
-    walk.start(p.queries, qi);
+    walk.start(kWalkQuery, p.queries, qi);
     int cur;
     float dcur;
     if (p.entry_node) {

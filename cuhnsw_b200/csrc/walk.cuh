@@ -187,7 +187,7 @@ struct WalkBoard {
   static constexpr int kReq = kCount + 4 * P;     // P + 1 selected keys
   static constexpr int kBytes = (kReq + 8 * (P + 1) + 15) / 16 * 16;
 };
-enum { kWalkOver = 0, kWalkQuery = 1, kWalkRound = 2, kWalkRows = 3 };
+enum { kWalkOver = 0, kWalkQuery = 1, kWalkRound = 2, kWalkRows = 3, kWalkNode = 4, kWalkSelect = 5 };
 
 template <class Dist, int W, int P>
 struct Walk {
@@ -284,16 +284,17 @@ struct Walk {
       if (i < count && lane == 0) sts32(board + Board::kCount + 4 * (w + W * i), (unsigned)have[i]);
   }
 
-  // Warps 1 .. W - 1 of a CTA per query: every operation starts and ends at a block barrier, as warp 0's do.
-  __device__ __forceinline__ void help(const float* queries) {
+  // Warps 1 .. W - 1: every operation starts and ends at a block barrier, as warp 0's do.  Returns, behind its first
+  // barrier, the first operation that is not the walk's own.
+  __device__ __forceinline__ int help(const float* queries) {
     const int w = warp();
     for (;;) {
       __syncthreads();
       const int op = posted(Board::kOp);
-      if (op == kWalkOver) return;
-      if (op == kWalkQuery) {
-        const long long qi = (unsigned)posted(Board::kQuery);
-        if (!Dist::kSharedQuery) de.load_query(queries + (size_t)qi * de.t.d);
+      if (op == kWalkOver || op == kWalkSelect) return op;
+      if (op == kWalkQuery || op == kWalkNode) {
+        if (!Dist::kSharedQuery) load(op, queries);
+        if (op == kWalkNode) self = posted(Board::kQuery);
         vis.clear(w, W);
       } else {
         if (op == kWalkRound) {
@@ -304,6 +305,12 @@ struct Walk {
       }
       __syncthreads();
     }
+  }
+  // the query whose number is on the board, or the stored row
+  __device__ __forceinline__ void load(int op, const float* queries) {
+    const long long qi = (unsigned)posted(Board::kQuery);
+    if (op == kWalkQuery) de.load_query(queries + (size_t)qi * de.t.d);
+    else de.load_query_row((int)qi);
   }
 
   // ---- warp 0 ----
@@ -319,10 +326,12 @@ struct Walk {
     __syncthreads();
     wc.evals += n;
   }
-  __device__ __forceinline__ void start(const float* queries, long long qi) {
-    if (lane == 0) sts32(board + Board::kQuery, (unsigned)qi);
-    post(kWalkQuery);
-    de.load_query(queries + (size_t)qi * de.t.d);
+  // query `i` of `queries` (op kWalkQuery), or stored row i, which the walk then leaves out (kWalkNode)
+  __device__ __forceinline__ void start(int op, const float* queries, long long i) {
+    if (lane == 0) sts32(board + Board::kQuery, (unsigned)i);
+    post(op);
+    load(op, queries);
+    if (op == kWalkNode) self = (int)i;
     vis.clear(0, W);
     __syncthreads();
   }
@@ -372,6 +381,30 @@ struct Walk {
   __device__ __forceinline__ void seed(int id, float dist) {
     list.seed(f2ord(dist), (unsigned)id);
     if (lane == 0) vis.test_and_set(id);
+    __syncwarp();
+  }
+
+  // list = the neighbours in an adjacency row of the searched layer
+  __device__ __forceinline__ void seed_row(const int* row) {
+    list.clear();
+    int n = 0;
+    for (int base = 0; base < stride; base += 32) {
+      const int nid = base + lane < stride ? __ldg(row + base + lane) : -1;
+      const bool on = nid >= 0 && nid != self;
+      const unsigned m = __ballot_sync(FULL, on);
+      const int at = n + __popc(m & list.lower);
+      if (on) sts64(pool + 8 * at, (unsigned)nid, found + 8 * at);
+      vis.test_and_set(nid, on);
+      n += __popc(m);
+    }
+    if (n == 0) return;
+    evaluate_rows(n);
+    for (int i = lane; i < n; i += 32) {
+      const uint2 k = lds64(found + 8 * i);
+      sts64(pool + 8 * i, k.x, 2 * k.y);
+    }
+    __syncwarp();
+    for (int base = 0; base < n; base += 32) list.merge(pool + 8 * base, min(32, n - base));
     __syncwarp();
   }
 
