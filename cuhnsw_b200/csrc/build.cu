@@ -49,20 +49,17 @@ struct SelBuf {
 // overwritten.
 template <class Dist>
 __device__ __forceinline__ int select_neighbors(Dist& de, const unsigned long long* cands, int nc, int m,
-                                                int nn_num, int save_remains, int new_comer, SelBuf& sel,
-                                                WalkCounters& wc) {
+                                                int nn_num, int save_remains, SelBuf& sel, WalkCounters& wc) {
   const int lane = lane_id();
   int head = 0;
   int tail = min(m, nc) - 1;
   const int max_head = tail + 1;
-  bool nc_in = false;
   for (int j = 0; j < nc; ++j) {
     if (head >= m) break;
     const unsigned long long k = cands[j];
     const int cid = key_id(k);
     const float cd = key_dist(k);
-    const bool freepass = head < nn_num || (new_comer >= 0 && !nc_in && cid != new_comer);
-    if (freepass) {
+    if (head < nn_num) {
       if (lane == 0) {
         sel.ids[head] = cid;
         sel.dist[head] = cd;
@@ -73,28 +70,20 @@ __device__ __forceinline__ int select_neighbors(Dist& de, const unsigned long lo
     }
     bool skip = false;
     de.load_query_row(cid);
-    if (new_comer >= 0 && nc_in) {
-      float dd = de.eval(new_comer, 1);
-      dd = __shfl_sync(FULL, dd, 0);
-      wc.evals += 1;
-      skip = cd > dd;
-    } else {
-      // the accepted neighbours are tested four at a time (one distance pass), closest first: most
-      // candidates are turned down by one of the first ones, and the rows of the others are then never
-      // read (1.18 M x 50: build 0.208 -> 0.192 s; 8 per vote 0.201 s)
-      constexpr int kVote = 4;
-      for (int base = 0; base < head; base += kVote) {
-        int n = min(kVote, head - base);
-        int id = (lane < n) ? sel.ids[base + lane] : 0;
-        float dd = de.eval(id, n);
-        wc.evals += n;
-        if (__any_sync(FULL, lane < n && cd > dd)) {
-          skip = true;
-          break;
-        }
+    // the accepted neighbours are tested four at a time (one distance pass), closest first: most
+    // candidates are turned down by one of the first ones, and the rows of the others are then never
+    // read (1.18 M x 50: build 0.208 -> 0.192 s; 8 per vote 0.201 s)
+    constexpr int kVote = 4;
+    for (int base = 0; base < head; base += kVote) {
+      int n = min(kVote, head - base);
+      int id = (lane < n) ? sel.ids[base + lane] : 0;
+      float dd = de.eval(id, n);
+      wc.evals += n;
+      if (__any_sync(FULL, lane < n && cd > dd)) {
+        skip = true;
+        break;
       }
     }
-    if (cid == new_comer && !skip) nc_in = true;
     if (skip && tail >= head) {
       if (lane == 0) {
         sel.ids[tail] = cid;
@@ -112,6 +101,57 @@ __device__ __forceinline__ int select_neighbors(Dist& de, const unsigned long lo
   }
   __syncwarp();
   return save_remains ? max_head : head;
+}
+
+// The same with the shortcut for one newcomer in a row that has been through selection (new_comer of SearchHeuristic): the
+// others are known to bear with each other, so those closer than the newcomer stay, the newcomer is tested against
+// them, and if it stays those farther than it are tested against it alone.  Distances are symmetric to the bit, so all
+// tests use the newcomer's row as the query: two reads deep instead of one read after the other for each candidate
+// behind it.  at: the newcomer's place in cands.
+template <class Dist>
+__device__ __forceinline__ int select_with_newcomer(Dist& de, const unsigned long long* cands, int nc, int at, int m,
+                                                    int nn_num, SelBuf& sel, WalkCounters& wc) {
+  const int lane = lane_id();
+  // rejected: the newcomer's own place, or none
+  bool in = false, out = false;
+  if (at >= nn_num && at < min(m, nc)) {
+    const unsigned long long k = cands[at];
+    const float cd = key_dist(k);
+    de.load_query_row(key_id(k));
+    for (int base = 0; base < at && !out; base += 8) {
+      const int n = min(8, at - base);
+      const int id = lane < n ? key_id(cands[base + lane]) : 0;
+      const float dd = de.eval_eight(id, n);
+      wc.evals += n;
+      out = __any_sync(FULL, lane < n && cd > dd);
+    }
+    in = !out;
+  }
+  int head = 0;
+  for (int base = 0; base < nc && head < m; base += 32) {
+    const int j = base + lane;
+    bool keep = j < nc && !(out && j == at);
+    const unsigned long long k = keep ? cands[j] : 0ull;
+    if (in && base + 32 > at + 1) {
+      const int from = max(at + 1 - base, 0), n = min(32, nc - base) - from;  // lanes from .. from + n - 1 lie behind it
+      if (n > 0) {
+        const int id = __shfl_sync(FULL, key_id(k), (lane + from) & 31);
+        const float dd = de.eval_eight(lane < n ? id : 0, n);
+        wc.evals += n;
+        const float mine = __shfl_sync(FULL, dd, (lane - from) & 31);
+        if (keep && lane >= from) keep = !(key_dist(k) > mine);
+      }
+    }
+    const unsigned mask = __ballot_sync(FULL, keep);
+    const int place = head + __popc(mask & ((1u << lane) - 1u));
+    if (keep && place < m) {
+      sel.ids[place] = key_id(k);
+      sel.dist[place] = key_dist(k);
+    }
+    head = min(m, head + __popc(mask));
+  }
+  __syncwarp();
+  return head;
 }
 
 template <class Dist>
@@ -208,6 +248,7 @@ struct BatchParams {
   int per_warp;
   int cap;
   long long total;  // count * stride proposals
+  int chunk;        // proposals a warp of the reverse kernel takes at a time (a power of two up to 32)
   int nn_num;
 };
 
@@ -236,7 +277,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_s
     expand_row(de, wl, L.rows + row_index(L.g.upper_base, L.level, s) * L.stride, L.stride, s, wc);
     if (L.reverse_cand) beam_layer_reverse(de, wl, L.rows, L.stride, L.g.upper_base, L.level, s, wc);
     else beam_layer(de, wl, L.rows, L.stride, L.g.upper_base, L.level, s, wc);
-    int deg = select_neighbors(de, wl.keys, wl.size, L.max_m, p.nn_num, L.save_remains, -1, sel, wc);
+    int deg = select_neighbors(de, wl.keys, wl.size, L.max_m, p.nn_num, L.save_remains, sel, wc);
     int* so = p.S.st_ids + (size_t)t * L.stride;
     float* sd = p.S.st_dist + (size_t)t * L.stride;
     for (int j = lane; j < L.stride; j += 32) {
@@ -423,15 +464,16 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_r
   const unsigned* keys = p.S.pkeys_sorted;
   const unsigned long long* vals = p.S.pvals_sorted;
   const unsigned none = (unsigned)L.g.n;
-  const long long nchunk = (p.total + 31) / 32;
+  const long long nchunk = (p.total + p.chunk - 1) / p.chunk;
   for (;;) {
     long long c = 0;
     if (lane == 0) c = (long long)atomicAdd(p.S.ticket + 1, 1ull);
     c = __shfl_sync(FULL, c, 0);
     if (c >= nchunk) break;
-    const long long i = c * 32 + lane;
-    const unsigned ki = (i < p.total) ? keys[i] : none;
-    const unsigned kprev = (i > 0 && i < p.total) ? keys[i - 1] : none;
+    const long long i = c * p.chunk + lane;
+    const bool mine = lane < p.chunk && i < p.total;
+    const unsigned ki = mine ? keys[i] : none;
+    const unsigned kprev = (i > 0 && mine) ? keys[i - 1] : none;
     const bool is_head = (ki != none) && (i == 0 || kprev != ki);
     unsigned heads = __ballot_sync(FULL, is_head);
     while (heads) {
@@ -456,7 +498,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_r
       __syncwarp();
       bool went = L.went[dst] != 0;
       bool changed = false;
-      for (long long pi = c * 32 + b; pi < p.total && keys[pi] == (unsigned)dst; ++pi) {
+      for (long long pi = c * p.chunk + b; pi < p.total && keys[pi] == (unsigned)dst; ++pi) {
         const unsigned long long v = vals[pi];
         const int s = (int)(v >> 32);
         const float sd = __uint_as_float((unsigned)v);
@@ -479,16 +521,21 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_r
           ncand += __popc(om);
         }
         __syncwarp();
+        int at = 0;  // the newcomer's place
         for (int e = lane; e < ncand; e += 32) {
           const unsigned long long ke = sel.tmp[e];
           int rank = 0;
           for (int f = 0; f < ncand; ++f) rank += (sel.tmp[f] < ke) ? 1 : 0;
           wl.keys[rank] = ke;
+          if (e == 0) at = rank;
         }
+        at = __shfl_sync(FULL, at, 0);
         __syncwarp();
         if (ncand > L.ef_construction) ncand = L.ef_construction;
-        const int new_comer = (!L.save_remains && went) ? s : -1;
-        deg = select_neighbors(de, wl.keys, ncand, L.max_m, p.nn_num, L.save_remains, new_comer, sel, wc);
+        if (!L.save_remains && went)
+          deg = select_with_newcomer(de, wl.keys, ncand, at, L.max_m, p.nn_num, sel, wc);
+        else
+          deg = select_neighbors(de, wl.keys, ncand, L.max_m, p.nn_num, L.save_remains, sel, wc);
         went = true;
         changed = true;
       }
@@ -604,7 +651,11 @@ static cudaError_t build_batch_t(const BuildLevel& L, const BuildScratch& S, lon
     p.per_warp = (int)per_warp;
     size_t smem = per_warp * kBuildWarps;
     int grid = 1;
-    long long chunks = (p.total + 31) / 32;
+    // a warp folds the targets that begin in its chunk one after the other: while there are fewer proposals than the
+    // chip has warps, one each (at most 16 CTAs of two warps per SM)
+    p.chunk = 32;
+    while (p.chunk > 1 && p.total < (long long)p.chunk * sm_count * 32) p.chunk >>= 1;
+    const long long chunks = (p.total + p.chunk - 1) / p.chunk;
     e = grid_for(build_reverse_kernel<Dist>, smem, kBuildWarps * 32, sm_count,
                  (chunks + kBuildWarps - 1) / kBuildWarps, &grid);
     if (e != cudaSuccess) return e;
