@@ -108,10 +108,12 @@ struct VisitedTable {
   }
 };
 
-// Per-warp shared-memory state.
+// Per-warp shared-memory state.  Loop bounds and branch conditions come from ballots, shuffles and reductions rather than
+// from loads, so that the compiler knows them to be the same in every lane: a warp-wide operation under a condition it
+// cannot be sure of costs a divergence check and a register move each (27 of 374 instructions per expansion).
 struct WarpList : VisitedTable {
-  unsigned long long* keys;  // ascending (distance, id); capacity `cap`
-  int* spos;                 // 32 ints of scratch
+  unsigned keys;  // shared-memory address of `cap` 64-bit keys, ascending (distance, id)
+  unsigned spos;  // 32 words of scratch
   int cap;
   int size;
   int cursor;  // every key before `cursor` is expanded
@@ -121,14 +123,31 @@ struct WarpList : VisitedTable {
     return (size_t)((cap + 31) / 32 * 32) * 8 + 32 * 4 + VisitedTable::smem_bytes(entries, n);
   }
   __device__ __forceinline__ void bind(void* smem, int cap_, int entries, long long n) {
-    keys = reinterpret_cast<unsigned long long*>(smem);
-    int capr = (cap_ + 31) / 32 * 32;
-    spos = reinterpret_cast<int*>(keys + capr);
-    bind_table(kept(smem_addr(spos + 32)), entries, n);
+    keys = kept(smem_addr(smem));
+    const int capr = (cap_ + 31) / 32 * 32;
+    spos = keys + 8 * capr;
+    bind_table(spos + 32 * 4, entries, n);
     cap = cap_;
     size = 0;
     cursor = 0;
     worst = KEY_MAX;
+  }
+  // key i with its flag
+  __device__ __forceinline__ unsigned long long key(int i) const {
+    const uint2 w = lds64(keys + 8 * i);
+    return ((unsigned long long)w.y << 32) | w.x;
+  }
+  __device__ __forceinline__ void set_key(int i, unsigned long long k) const {
+    sts64(keys + 8 * i, (unsigned)k, (unsigned)(k >> 32));
+  }
+  // low words (id and flag) of two neighbouring keys, the same in every lane
+  __device__ __forceinline__ uint2 low_words(int i) const {
+    const unsigned w = lds32(keys + 8 * (i + (lane_id() & 1)));
+    return make_uint2(__shfl_sync(FULL, w, 0), __shfl_sync(FULL, w, 1));
+  }
+  __device__ __forceinline__ void flag_key(int i, unsigned low) const {
+    if (lane_id() == 0) sts32(keys + 8 * i, low | (unsigned)KEY_FLAG);
+    __syncwarp();
   }
   // The table size is proportional to the list capacity, so clearing it is
   // O(nodes touched); the reference resets through a touched-slot list
@@ -150,9 +169,9 @@ struct WarpList : VisitedTable {
   // order with "insert if not full or smaller than the largest, evicting the
   // largest" (cuda_utils_kernels.cuh:220-225).  Returns the smallest position a
   // newcomer took, or `cap` when nothing was inserted.
-  __device__ __forceinline__ int merge(unsigned long long key, bool active, WalkCounters& wc) {
+  __device__ __forceinline__ int merge(unsigned long long nk, bool active, WalkCounters& wc) {
     const int lane = lane_id();
-    bool keep = active && key < worst;
+    bool keep = active && nk < worst;
     const unsigned km0 = __ballot_sync(FULL, keep);
     if (km0 == 0) return cap;
     // pos = number of list keys smaller than the new key
@@ -161,16 +180,14 @@ struct WarpList : VisitedTable {
     const int nch = (size + 31) >> 5;
     if (__popc(km0) <= 4 && nch <= 32) {
       // up to four newcomers: two-level search by the whole warp, one newcomer at a time
+      const unsigned long long pv = (lane < nch) ? (key(min(lane * 32 + 31, size - 1)) & KEY_MASK) : KEY_MAX;
       for (unsigned mm = km0; mm; mm &= mm - 1) {
         const int b = __ffs(mm) - 1;
-        const unsigned long long kb = shfl64(key, b);
-        int c = 0;
-        if (nch > 1) {
-          const unsigned long long pv = (lane < nch) ? (keys[min(lane * 32 + 31, size - 1)] & KEY_MASK) : KEY_MAX;
-          c = __popc(__ballot_sync(FULL, pv < kb));  // chunks entirely below kb (lanes >= nch hold KEY_MAX)
-        }
+        const unsigned long long kb = shfl64(nk, b);
+        // chunks entirely below kb (lanes >= nch hold KEY_MAX)
+        const int c = nch > 1 ? __popc(__ballot_sync(FULL, pv < kb)) : 0;
         const int i = c * 32 + lane;
-        const unsigned long long kv = (i < size) ? (keys[i] & KEY_MASK) : KEY_MAX;
+        const unsigned long long kv = (i < size) ? (key(i) & KEY_MASK) : KEY_MAX;
         const unsigned lt = __ballot_sync(FULL, kv < kb);
         const unsigned eq = __ballot_sync(FULL, kv == kb);
         if (lane == b) {
@@ -184,15 +201,14 @@ struct WarpList : VisitedTable {
       const int cs = (nch + 31) >> 5;
       for (unsigned mm = km0; mm; mm &= mm - 1) {
         const int b = __ffs(mm) - 1;
-        const unsigned long long kb = shfl64(key, b);
-        const unsigned long long pv =
-            (lane * cs < nch) ? (keys[min((lane + 1) * cs * 32 - 1, size - 1)] & KEY_MASK) : KEY_MAX;
+        const unsigned long long kb = shfl64(nk, b);
+        const unsigned long long pv = (lane * cs < nch) ? (key(min((lane + 1) * cs * 32 - 1, size - 1)) & KEY_MASK) : KEY_MAX;
         const int c = __popc(__ballot_sync(FULL, pv < kb));  // spans entirely below kb
         int below = 0;
         bool same = false;
         for (int j = 0; j < cs; ++j) {
           const int i = (c * cs + j) * 32 + lane;
-          const unsigned long long kv = (i < size) ? (keys[i] & KEY_MASK) : KEY_MAX;
+          const unsigned long long kv = (i < size) ? (key(i) & KEY_MASK) : KEY_MAX;
           const unsigned lt = __ballot_sync(FULL, kv < kb);
           same = same || __ballot_sync(FULL, kv == kb) != 0;
           below += __popc(lt);
@@ -208,12 +224,12 @@ struct WarpList : VisitedTable {
       while (__any_sync(FULL, lo < hi)) {
         if (lo < hi) {
           int mid = (lo + hi) >> 1;
-          if ((keys[mid] & KEY_MASK) < key) lo = mid + 1;
+          if ((key(mid) & KEY_MASK) < nk) lo = mid + 1;
           else hi = mid;
         }
       }
       pos = lo;
-      dup = keep && pos < size && (keys[pos] & KEY_MASK) == key;
+      dup = keep && pos < size && (key(pos) & KEY_MASK) == nk;
     }
     if (dup) keep = false;  // already listed
     const unsigned km = __ballot_sync(FULL, keep);
@@ -228,58 +244,60 @@ struct WarpList : VisitedTable {
       for (int hi = size; hi > minpos; hi -= 64) {
         const int i = hi - 32 + lane, i2 = i - 32;
         const bool have = i >= minpos, have2 = i2 >= minpos;
-        const unsigned long long v = have ? keys[i] : 0ull;
-        const unsigned long long v2 = have2 ? keys[i2] : 0ull;
+        const unsigned at = keys + 8 * i;
+        const uint2 v = lds64(have ? at : keys);
+        const uint2 v2 = lds64(have2 ? at - 256 : keys);
         __syncwarp();
-        if (have && i + 1 < cap) keys[i + 1] = v;
-        if (have2) keys[i2 + 1] = v2;  // i2 + 1 <= size - 32 < cap
+        if (have && i + 1 < cap) sts64(at + 8, v.x, v.y);
+        if (have2) sts64(at - 248, v2.x, v2.y);  // i2 + 1 <= size - 32 < cap
       }
-      if (keep) keys[pos] = key;  // pos < cap: either the list is not full or key < worst
+      if (keep) set_key(pos, nk);  // pos < cap: either the list is not full or nk < worst
     } else {
       int rk = 0;
       for (unsigned mm = km; mm; mm &= mm - 1) {
         const int b = __ffs(mm) - 1;
-        const unsigned long long kb = shfl64(key, b);
-        rk += (kb < key) ? 1 : 0;
+        const unsigned long long kb = shfl64(nk, b);
+        rk += (kb < nk) ? 1 : 0;
       }
-      if (keep) spos[rk] = pos;  // newcomer positions, ascending
+      if (keep) sts32(spos + 4 * rk, (unsigned)pos);  // newcomer positions, ascending
+      minpos = (int)__reduce_min_sync(FULL, keep ? (unsigned)pos : 0x7fffffffu);
       __syncwarp();
-      minpos = spos[0];
-      const int mypos = (lane < m) ? spos[lane] : 0x7fffffff;
+      const int mypos = (lane < m) ? (int)lds32(spos + 4 * lane) : 0x7fffffff;
       for (int hi = size; hi > minpos; hi -= 64) {
         // key i moves up by the number of newcomers placed at or before it; that number is the same for a
         // whole window of 32 unless a newcomer lands inside it.  Two windows per turn, both read before
         // either is written.
         const int i = hi - 32 + lane, i2 = i - 32;
         const bool have = i >= minpos, have2 = i2 >= minpos;
-        const unsigned long long v = have ? keys[i] : 0ull;
-        const unsigned long long v2 = have2 ? keys[i2] : 0ull;
+        const unsigned at = keys + 8 * i;
+        const uint2 v = lds64(have ? at : keys);
+        const uint2 v2 = lds64(have2 ? at - 256 : keys);
         const int below2 = __popc(__ballot_sync(FULL, mypos <= hi - 64));
         const int below = __popc(__ballot_sync(FULL, mypos <= hi - 32));
         const int upto = __popc(__ballot_sync(FULL, mypos <= hi - 1));
         int cnt = below, cnt2 = below2;
-        for (int j = below; j < upto; ++j) cnt += (spos[j] <= i) ? 1 : 0;
-        for (int j = below2; j < below; ++j) cnt2 += (spos[j] <= i2) ? 1 : 0;
+        for (int j = below; j < upto; ++j) cnt += ((int)lds32(spos + 4 * j) <= i) ? 1 : 0;
+        for (int j = below2; j < below; ++j) cnt2 += ((int)lds32(spos + 4 * j) <= i2) ? 1 : 0;
         __syncwarp();
-        if (have && i + cnt < cap) keys[i + cnt] = v;
-        if (have2 && i2 + cnt2 < cap) keys[i2 + cnt2] = v2;
+        if (have && i + cnt < cap) sts64(at + 8 * cnt, v.x, v.y);
+        if (have2 && i2 + cnt2 < cap) sts64(at - 256 + 8 * cnt2, v2.x, v2.y);
       }
-      if (keep && pos + rk < cap) keys[pos + rk] = key;
+      if (keep && pos + rk < cap) set_key(pos + rk, nk);
     }
     size = min(cap, size + m);
     cursor = min(cursor, minpos);
     wc.inserts += m;
     __syncwarp();
-    worst = (size >= cap) ? (keys[cap - 1] & KEY_MASK) : KEY_MAX;
+    worst = (size >= cap) ? (key(cap - 1) & KEY_MASK) : KEY_MAX;
     return minpos;
   }
 
-  // list = {key}
-  __device__ __forceinline__ void seed(unsigned long long key) {
-    if (lane_id() == 0) keys[0] = key;
+  // list = {k}
+  __device__ __forceinline__ void seed(unsigned long long k) {
+    if (lane_id() == 0) set_key(0, k);
     size = 1;
     cursor = 0;
-    worst = cap <= 1 ? (key & KEY_MASK) : KEY_MAX;
+    worst = cap <= 1 ? (k & KEY_MASK) : KEY_MAX;
     __syncwarp();
   }
 
@@ -289,7 +307,7 @@ struct WarpList : VisitedTable {
     int c = cursor;
     while (c < size) {
       int i = c + lane;
-      bool open = (i < size) && !(keys[i] & KEY_FLAG);
+      bool open = (i < size) && !(lds32(keys + 8 * i) & (unsigned)KEY_FLAG);
       unsigned m = __ballot_sync(FULL, open);
       if (m) {
         c += __ffs(m) - 1;
@@ -307,13 +325,13 @@ template <class Dist>
 __device__ __forceinline__ int expand_chunk(Dist& de, WarpList& wl, int nid, int self, WalkCounters& wc) {
   const int lane = lane_id();
   bool fresh = (nid >= 0) && (nid != self);
-  if (fresh) fresh = !wl.test_and_set(nid);
+  fresh = !wl.test_and_set(nid, fresh) && fresh;
   const unsigned fm = __ballot_sync(FULL, fresh);
   if (fm == 0) return wl.cap;
   const int n = __popc(fm);
-  if (fresh) wl.spos[__popc(fm & ((1u << lane) - 1))] = nid;
+  if (fresh) sts32(wl.spos + 4 * __popc(fm & ((1u << lane) - 1)), (unsigned)nid);
   __syncwarp();
-  const int cid = wl.spos[lane];
+  const int cid = (int)lds32(wl.spos + 4 * lane);
   // the shuffles inside eval() order this read before any later write of spos
   const float dist = de.eval(cid, n);
   wc.evals += n;
@@ -351,13 +369,13 @@ __device__ __forceinline__ void beam_layer(Dist& de, WarpList& wl, const int* __
   int pf_node = -1, pf_val = -1;
   wl.advance();
   if (wl.cursor >= wl.size) return;
-  unsigned long long k = wl.keys[wl.cursor];
+  // low words of the closest unexpanded key and of the key after it
+  uint2 k = wl.low_words(wl.cursor);
   for (;;) {
-    // k = keys[cursor] is the closest unexpanded key
-    const unsigned long long k2 = (wl.cursor + 1 < wl.size) ? wl.keys[wl.cursor + 1] : KEY_FLAG;
-    if (lane == 0) wl.keys[wl.cursor] = k | KEY_FLAG;
-    __syncwarp();
-    const int cur = key_id(k);
+    const int at = wl.cursor;  // position of the key being expanded; insertions at or before it move the cursor
+    const unsigned k2 = at + 1 < wl.size ? k.y : (unsigned)KEY_FLAG;
+    wl.flag_key(at, k.x);
+    const int cur = (int)(k.x & 0x7fffffffu);
     const int* row = rows + row_index(upper_base, level, cur) * stride;
     int nid;
     if (cur == pf_node) {
@@ -366,13 +384,13 @@ __device__ __forceinline__ void beam_layer(Dist& de, WarpList& wl, const int* __
       nid = (lane < stride) ? __ldg(row + lane) : -1;
     }
     pf_node = -1;
-    if (!(k2 & KEY_FLAG)) {
-      pf_node = key_id(k2);
+    const bool open2 = !(k2 & (unsigned)KEY_FLAG);
+    if (open2) {
+      pf_node = (int)k2;
       const int* nrow = rows + row_index(upper_base, level, pf_node) * stride;
       pf_val = (lane < stride) ? __ldg(nrow + lane) : -1;
     }
     wc.expansions += 1;
-    const int at = wl.cursor;  // position of the key being expanded; insertions at or before it move the cursor
     int first_new = expand_chunk(de, wl, nid, self, wc);
     for (int base = 32; base < stride; base += 32) {
       const int l = base + lane;
@@ -380,16 +398,15 @@ __device__ __forceinline__ void beam_layer(Dist& de, WarpList& wl, const int* __
     }
     // next key: a newcomer placed at or before at + 1, else the old successor if it is still unexpanded,
     // else scan on
-    if (first_new > at + 1 && !(k2 & KEY_FLAG)) {
+    if (first_new > at + 1 && open2) {
       // no newcomer in front of the old successor: it sits at at + 1 unchanged
       wl.cursor = at + 1;
-      k = k2;
-      continue;
+    } else {
+      __syncwarp();
+      wl.advance();
+      if (wl.cursor >= wl.size) break;
     }
-    __syncwarp();
-    wl.advance();
-    if (wl.cursor >= wl.size) break;
-    k = wl.keys[wl.cursor];
+    k = wl.low_words(wl.cursor);
   }
 }
 
@@ -405,7 +422,7 @@ __device__ __forceinline__ void beam_layer_reverse(Dist& de, WarpList& wl, const
     int at = -1;
     for (int base = hi & ~31; hi >= 0 && base >= 0; base -= 32) {
       const int i = base + lane;
-      const bool open = (i <= hi) && !(wl.keys[i] & KEY_FLAG);
+      const bool open = (i <= hi) && !(lds32(wl.keys + 8 * i) & (unsigned)KEY_FLAG);
       const unsigned m = __ballot_sync(FULL, open);
       if (m) {
         at = base + 31 - __clz(m);
@@ -413,11 +430,10 @@ __device__ __forceinline__ void beam_layer_reverse(Dist& de, WarpList& wl, const
       }
     }
     if (at < 0) break;
-    const unsigned long long k = wl.keys[at];
+    const unsigned k = wl.low_words(at).x;
     __syncwarp();
-    if (lane == 0) wl.keys[at] = k | KEY_FLAG;
-    __syncwarp();
-    const int* row = rows + row_index(upper_base, level, key_id(k)) * stride;
+    wl.flag_key(at, k);
+    const int* row = rows + row_index(upper_base, level, (int)k) * stride;
     wc.expansions += 1;
     int first_new = wl.cap;
     for (int base = 0; base < stride; base += 32) {
@@ -433,7 +449,7 @@ __device__ __forceinline__ void beam_layer_reverse(Dist& de, WarpList& wl, const
 // neighbour of the current node, move to the closest one if it is strictly
 // closer (first in row order among equals), repeat until no move.
 template <class Dist>
-__device__ __forceinline__ void greedy_descent(Dist& de, int* scratch, const int* __restrict__ rowsU, int strideU,
+__device__ __forceinline__ void greedy_descent(Dist& de, unsigned scratch, const int* __restrict__ rowsU, int strideU,
                                                const int* __restrict__ upper_base, int top, int bottom_excl,
                                                int& cur, float& dcur, WalkCounters& wc) {
   const int lane = lane_id();
@@ -452,9 +468,9 @@ __device__ __forceinline__ void greedy_descent(Dist& de, int* scratch, const int
         unsigned fm = __ballot_sync(FULL, ok);
         if (fm == 0) continue;
         int n = __popc(fm);
-        if (ok) scratch[__popc(fm & ((1u << lane) - 1))] = nid;
+        if (ok) sts32(scratch + 4 * __popc(fm & ((1u << lane) - 1)), (unsigned)nid);
         __syncwarp();
-        int cid = scratch[lane];
+        int cid = (int)lds32(scratch + 4 * lane);
         __syncwarp();
         float dist = de.eval(cid, n);
         wc.evals += n;

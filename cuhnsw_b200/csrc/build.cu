@@ -44,11 +44,11 @@ struct SelBuf {
 };
 
 // Neighbour selection of the reference (SearchHeuristic, cuda_build_kernels.cuh:68-162).
-// cands: ascending keys (distance to the row owner, id), flags ignored.  Writes
+// cands: a list of ascending keys (distance to the row owner, id), flags ignored.  Writes
 // sel.ids/sel.dist and returns the new degree.  The distance engine's query is
 // overwritten.
 template <class Dist>
-__device__ __forceinline__ int select_neighbors(Dist& de, const unsigned long long* cands, int nc, int m,
+__device__ __forceinline__ int select_neighbors(Dist& de, const WarpList& cands, int nc, int m,
                                                 int nn_num, int save_remains, SelBuf& sel, WalkCounters& wc) {
   const int lane = lane_id();
   int head = 0;
@@ -56,7 +56,7 @@ __device__ __forceinline__ int select_neighbors(Dist& de, const unsigned long lo
   const int max_head = tail + 1;
   for (int j = 0; j < nc; ++j) {
     if (head >= m) break;
-    const unsigned long long k = cands[j];
+    const unsigned long long k = cands.key(j);
     const int cid = key_id(k);
     const float cd = key_dist(k);
     if (head < nn_num) {
@@ -109,18 +109,18 @@ __device__ __forceinline__ int select_neighbors(Dist& de, const unsigned long lo
 // tests use the newcomer's row as the query: two reads deep instead of one read after the other for each candidate
 // behind it.  at: the newcomer's place in cands.
 template <class Dist>
-__device__ __forceinline__ int select_with_newcomer(Dist& de, const unsigned long long* cands, int nc, int at, int m,
+__device__ __forceinline__ int select_with_newcomer(Dist& de, const WarpList& cands, int nc, int at, int m,
                                                     int nn_num, SelBuf& sel, WalkCounters& wc) {
   const int lane = lane_id();
   // rejected: the newcomer's own place, or none
   bool in = false, out = false;
   if (at >= nn_num && at < min(m, nc)) {
-    const unsigned long long k = cands[at];
+    const unsigned long long k = cands.key(at);
     const float cd = key_dist(k);
     de.load_query_row(key_id(k));
     for (int base = 0; base < at && !out; base += 8) {
       const int n = min(8, at - base);
-      const int id = lane < n ? key_id(cands[base + lane]) : 0;
+      const int id = lane < n ? key_id(cands.key(base + lane)) : 0;
       const float dd = de.eval_eight(id, n);
       wc.evals += n;
       out = __any_sync(FULL, lane < n && cd > dd);
@@ -131,7 +131,7 @@ __device__ __forceinline__ int select_with_newcomer(Dist& de, const unsigned lon
   for (int base = 0; base < nc && head < m; base += 32) {
     const int j = base + lane;
     bool keep = j < nc && !(out && j == at);
-    const unsigned long long k = keep ? cands[j] : 0ull;
+    const unsigned long long k = keep ? cands.key(j) : 0ull;
     if (in && base + 32 > at + 1) {
       const int from = max(at + 1 - base, 0), n = min(32, nc - base) - from;  // lanes from .. from + n - 1 lie behind it
       if (n > 0) {
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_s
     expand_row(de, wl, L.rows + row_index(L.g.upper_base, L.level, s) * L.stride, L.stride, s, wc);
     if (L.reverse_cand) beam_layer_reverse(de, wl, L.rows, L.stride, L.g.upper_base, L.level, s, wc);
     else beam_layer(de, wl, L.rows, L.stride, L.g.upper_base, L.level, s, wc);
-    int deg = select_neighbors(de, wl.keys, wl.size, L.max_m, p.nn_num, L.save_remains, sel, wc);
+    int deg = select_neighbors(de, wl, wl.size, L.max_m, p.nn_num, L.save_remains, sel, wc);
     int* so = p.S.st_ids + (size_t)t * L.stride;
     float* sd = p.S.st_dist + (size_t)t * L.stride;
     for (int j = lane; j < L.stride; j += 32) {
@@ -526,16 +526,16 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_r
           const unsigned long long ke = sel.tmp[e];
           int rank = 0;
           for (int f = 0; f < ncand; ++f) rank += (sel.tmp[f] < ke) ? 1 : 0;
-          wl.keys[rank] = ke;
+          wl.set_key(rank, ke);
           if (e == 0) at = rank;
         }
         at = __shfl_sync(FULL, at, 0);
         __syncwarp();
         if (ncand > L.ef_construction) ncand = L.ef_construction;
         if (!L.save_remains && went)
-          deg = select_with_newcomer(de, wl.keys, ncand, at, L.max_m, p.nn_num, sel, wc);
+          deg = select_with_newcomer(de, wl, ncand, at, L.max_m, p.nn_num, sel, wc);
         else
-          deg = select_neighbors(de, wl.keys, ncand, L.max_m, p.nn_num, L.save_remains, sel, wc);
+          deg = select_neighbors(de, wl, ncand, L.max_m, p.nn_num, L.save_remains, sel, wc);
         went = true;
         changed = true;
       }

@@ -61,7 +61,7 @@ knn_search_kernel(SearchParams p) {
       int id = -1;
       float dist = __int_as_float(0x7f800000);
       if (j < found) {
-        unsigned long long k = wl.keys[j];
+        unsigned long long k = wl.key(j);
         id = key_id(k);
         dist = key_dist(k);
         if (p.labels) id = __ldg(p.labels + id);
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) entry_kernel(SearchParams p
   float dcur = de.eval(cur, 1);
   dcur = __shfl_sync(FULL, dcur, 0);
   wc.evals += 1;
-  greedy_descent(de, scratch[warp], p.g.rowsU, p.g.strideU, p.g.upper_base, p.g.max_level, 0, cur, dcur, wc);
+  greedy_descent(de, smem_addr(scratch[warp]), p.g.rowsU, p.g.strideU, p.g.upper_base, p.g.max_level, 0, cur, dcur, wc);
   if (lane == 0) {
     s.entry_node[qi] = cur;
     s.entry_dist[qi] = dcur;

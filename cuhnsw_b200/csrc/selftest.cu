@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(32) selftest_list_kernel(int cap, const float*
     for (int e = 0; e < expand[b]; ++e) {
       wl.advance();
       if (wl.cursor >= wl.size) break;
-      if (lane == 0) wl.keys[wl.cursor] |= KEY_FLAG;
+      if (lane == 0) wl.set_key(wl.cursor, wl.key(wl.cursor) | KEY_FLAG);
       __syncwarp();
     }
     const int lo = batch_begin[b], n = batch_begin[b + 1] - lo;
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(32) selftest_list_kernel(int cap, const float*
     __syncwarp();
   }
   wl.advance();
-  for (int i = lane; i < wl.size; i += 32) out_keys[i] = wl.keys[i];
+  for (int i = lane; i < wl.size; i += 32) out_keys[i] = wl.key(i);
   if (lane == 0) {
     *out_size = wl.size;
     *out_cursor = wl.cursor;
