@@ -474,20 +474,14 @@ __device__ __forceinline__ void greedy_descent(Dist& de, unsigned scratch, const
         __syncwarp();
         float dist = de.eval(cid, n);
         wc.evals += n;
-        float dm = (lane < n) ? dist : __int_as_float(0x7f800000);
-        int lm = lane;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          float od = __shfl_xor_sync(FULL, dm, off);
-          int ol = __shfl_xor_sync(FULL, lm, off);
-          if (od < dm || (od == dm && ol < lm)) {
-            dm = od;
-            lm = ol;
-          }
-        }
-        if (dm < best_d) {
-          best_d = dm;
-          best_id = __shfl_sync(FULL, cid, lm);
+        // closest, the first in row order among equals; a NaN is never closest
+        const unsigned image = lane < n && dist == dist ? f2ord(dist) : ~0u;
+        const unsigned least = __reduce_min_sync(FULL, image);
+        const int at = __ffs(__ballot_sync(FULL, image == least)) - 1;
+        const int id = __shfl_sync(FULL, cid, at);
+        if (least != ~0u && ord2f(least) < best_d) {
+          best_d = ord2f(least);
+          best_id = id;
         }
       }
       if (best_id != cur) {

@@ -7,6 +7,8 @@
 // (cpp/include/cuda_search_kernels.cuh:11-165, cpp/src/cuhnsw_build.cu:210-290),
 // which re-flatten and re-upload the graph on every call, launch once per
 // layer and keep the heap in global memory.
+#include <algorithm>
+
 #include <cub/block/block_radix_sort.cuh>
 #include <cub/device/device_radix_sort.cuh>
 
@@ -17,7 +19,10 @@ namespace hnsw {
 
 constexpr int kWarpsPerCta = 2;
 
-template <class Dist, bool kReverse>
+// kEntries: the batch has been scheduled, every query's descent has ended at entry_node / entry_dist.  An instance of its
+// own because with the descent in the same kernel the compiler takes the whole walk for divergent: 315 instead of 367
+// instructions per expansion (20 000 queries, 600 000 x 50, ef 200: 1.76 against 1.94 ms).
+template <class Dist, bool kReverse, bool kEntries>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, Dist::kSearchMinCtas)
 knn_search_kernel(SearchParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -35,14 +40,14 @@ knn_search_kernel(SearchParams p) {
     if (lane == 0) qi = (long long)atomicAdd(p.ticket, 1ull);
     qi = __shfl_sync(FULL, qi, 0);
     if (qi >= p.nq) break;
-    if (p.order) qi = __ldg(p.order + qi);
+    if (p.order) qi = __shfl_sync(FULL, __ldg(p.order + qi), 0);
     de.load_query(p.queries + (size_t)qi * p.g.d);
     wl.reset();
     int cur;
     float dcur;
-    if (p.entry_node) {
-      cur = __ldg(p.entry_node + qi);
-      dcur = __ldg(p.entry_dist + qi);
+    if (kEntries) {
+      cur = __shfl_sync(FULL, __ldg(p.entry_node + qi), 0);
+      dcur = __shfl_sync(FULL, __ldg(p.entry_dist + qi), 0);
     } else {
       cur = p.g.enter_point;
       dcur = de.eval(cur, 1);
@@ -207,6 +212,14 @@ static cudaError_t launch_search_t(const SearchParams& p0, int sm_count, cudaStr
                          : launch_search_tr<Dist, false>(p0, sm_count, stream, sched);
 }
 
+// CTAs of a search kernel that an SM holds
+template <class K>
+static cudaError_t residents(K kern, size_t smem, int* per_sm) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, kWarpsPerCta * 32, smem);
+  return e != cudaSuccess ? e : *per_sm < 1 ? cudaErrorInvalidConfiguration : cudaSuccess;
+}
+
 template <class Dist, bool kReverse>
 static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaStream_t stream,
                                     const SearchSchedule* sched) {
@@ -215,25 +228,24 @@ static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaSt
   per_warp = (per_warp + 15) / 16 * 16;
   p.smem_per_warp = (int)per_warp;
   size_t smem = per_warp * kWarpsPerCta;
-  auto kern = knn_search_kernel<Dist, kReverse>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarpsPerCta * 32, smem);
+  cudaError_t e = residents(knn_search_kernel<Dist, kReverse, false>, smem, &per_sm);
   if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  long long want = (p.nq + kWarpsPerCta - 1) / kWarpsPerCta;
-  long long grid = (long long)per_sm * sm_count;
-  if (grid > want) grid = want;
-  if (grid < 1) grid = 1;
+  const long long want = (p.nq + kWarpsPerCta - 1) / kWarpsPerCta;
+  long long grid = std::max(1ll, std::min((long long)per_sm * sm_count, want));
+  e = cudaMemsetAsync(p.ticket, 0, sizeof(unsigned long long), stream);
+  if (e != cudaSuccess) return e;
   // more queries than resident warps: start the long walks first
   if (sched && p.nq > grid * kWarpsPerCta && p.nq <= sched->capacity && p.nq <= 0x7fffffffll) {
     e = schedule_search(p, *sched, sm_count, stream);
     if (e != cudaSuccess) return e;
+    e = residents(knn_search_kernel<Dist, kReverse, true>, smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    grid = std::max(1ll, std::min((long long)per_sm * sm_count, want));
+    knn_search_kernel<Dist, kReverse, true><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
+  } else {
+    knn_search_kernel<Dist, kReverse, false><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
   }
-  e = cudaMemsetAsync(p.ticket, 0, sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
-  kern<<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
   return cudaGetLastError();
 }
 

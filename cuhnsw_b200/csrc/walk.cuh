@@ -361,7 +361,8 @@ struct Walk {
         int best_id = cur;
         float best_d = dcur;
         for (int base = 0; base < n; base += 32) {
-          const uint2 k = base + lane < n ? lds64(found + 8 * (base + lane)) : make_uint2(~0u, ~0u);
+          uint2 k = base + lane < n ? lds64(found + 8 * (base + lane)) : make_uint2(~0u, ~0u);
+          if (k.x < f2ord(-__int_as_float(0x7f800000))) k.x = ~0u;  // a negative NaN is not closest
           const unsigned least = __reduce_min_sync(FULL, k.x);
           const int at = __ffs(__ballot_sync(FULL, k.x == least)) - 1;  // first in row order
           const int id = __shfl_sync(FULL, (int)k.y, at);
