@@ -256,13 +256,13 @@ size_t search_smem_per_cta(int d, int ef, int vsize, long long n) {
 }
 
 // One CTA per query while that is the faster way: up to so many queries per SM.  Narrow rows: the longer the walks, the
-// longer a launch waits for its last ones (ef 50: 14 queries per SM; in between in proportion; ef 200 and more: 42).  Wide
+// longer a launch waits for its last ones (ef 50: 14 queries per SM; in between in proportion; ef 170 and more: 36).  Wide
 // rows: 10, very wide ones 14.  Measured, one warp / one CTA per query, ms: 300 000 x 96 f16, 4000 queries, ef 50: 0.33 /
 // 0.36, ef 128: 0.76 / 0.64, ef 400: 2.13 / 1.60, 6000: 0.39 / 0.49, 0.79 / 0.84, 2.19 / 1.94; 200 000 x 300 f16, ef 100,
 // 1000 queries: 0.75 / 0.53, 2000: 0.73 / 0.74; 150 000 x 960, ef 500, 2000: 3.56 / 3.16, 3000: 4.12 / 4.43.  More figures
 // are in search_walk.cuh.  Expanding the farthest key first knows no next nodes to prepare: always one warp.
 static long long team_limit(int d, int ef, int sm_count) {
-  const int per_sm = d > 512 ? 14 : d > 128 ? 10 : ef * 27 / 128 < 14 ? 14 : ef * 27 / 128 > 42 ? 42 : ef * 27 / 128;
+  const int per_sm = d > 512 ? 14 : d > 128 ? 10 : ef * 27 / 128 < 14 ? 14 : ef * 27 / 128 > 36 ? 36 : ef * 27 / 128;
   return (long long)sm_count * per_sm;
 }
 // Otherwise one warp per query; for few queries over wide rows with 32 float4 loads in flight instead of 16 (1 M x 960,

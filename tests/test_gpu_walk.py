@@ -39,7 +39,7 @@ def test_walk_equals_the_oracle(d, max_m0, dist_type, values):
     assert stats["expansions"] == int(want[3][:, 1].sum()) and stats["sweeps"] == int(want[3][:, 2].sum())
 
 
-@pytest.mark.parametrize("d,ef,nq", [(20, 40, 2072), (50, 200, 3996), (50, 200, 6216), (140, 40, 1480),
+@pytest.mark.parametrize("d,ef,nq", [(20, 40, 2072), (50, 200, 3996), (50, 200, 5328), (140, 40, 1480),
                                      (600, 120, 592), (600, 120, 2072)])
 def test_batches_on_both_sides_of_a_change_of_kernel(d, ef, nq):
   """A batch of the largest size of one kernel and one query more (148 SMs), against one warp per query."""
