@@ -494,45 +494,57 @@ int Engine::BuildGraph() {
   int vsize = 0;
   if (ResolveVsize(std::max(opt_.ef_construction, kMaxLinksHost + 8), -1, &vsize) != kOk)
     return Fail(kUnsupported, "ef_construction does not fit in shared memory");
-  DevBuf<float> dist0, distU, st_dist;
-  DevBuf<unsigned char> went;
-  DevBuf<int> st_ids, nodes_d;
-  DevBuf<unsigned> pkeys, pkeys_sorted;
-  DevBuf<unsigned long long> pvals, pvals_sorted;
-  DevBuf<unsigned char> sort_tmp;
-  CU(dist0.alloc((size_t)n_ * stride0_));
-  CU(distU.alloc((size_t)std::max<long long>(total_upper_, 1) * strideU_));
-  CU(went.alloc((size_t)n_));
-  CU(st_ids.alloc((size_t)bmax * smax));
-  CU(st_dist.alloc((size_t)bmax * smax));
-  CU(pkeys.alloc((size_t)bmax * smax));
-  CU(pkeys_sorted.alloc((size_t)bmax * smax));
-  CU(pvals.alloc((size_t)bmax * smax));
-  CU(pvals_sorted.alloc((size_t)bmax * smax));
-  size_t tmp_bytes = build_sort_tmp_bytes(bmax * smax);
-  CU(sort_tmp.alloc(tmp_bytes + 256));
+  std::vector<std::vector<int>> level_nodes((size_t)max_level_ + 1);
+  for (long long i = 0; i < n_; ++i)
+    for (int l = 1; l <= levels_h_[i]; ++l) level_nodes[l].push_back((int)i);
+  const size_t max_upper_nodes = max_level_ >= 1 ? level_nodes[1].size() : 0;
+
+  // Everything the construction needs besides the graph, in one allocation (a dozen of them, and handing them back, took
+  // 3 to 30 ms).  Up to kBuildScratchKept bytes stay with the handle for its next build.
+  const size_t items = (size_t)bmax * smax;
+  const size_t tmp_bytes = build_sort_tmp_bytes((long long)items);
+  size_t total = 0;
+  const auto part = [&total](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  const size_t at_dist0 = part((size_t)n_ * stride0_ * 4);
+  const size_t at_distU = part((size_t)std::max<long long>(total_upper_, 1) * strideU_ * 4);
+  const size_t at_went = part((size_t)n_);
+  const size_t at_ids = part(items * 4), at_dist = part(items * 4);
+  const size_t at_keys = part(items * 4), at_keys2 = part(items * 4);
+  const size_t at_vals = part(items * 8), at_vals2 = part(items * 8);
+  const size_t at_tmp = part(tmp_bytes + 256);
+  const size_t at_nodes = part(std::max<size_t>(max_upper_nodes, 1) * 4);
+  CU(build_scratch_.alloc(total));
+  unsigned char* const base = build_scratch_.get();
+  // goes back on every way out unless it is small
+  struct GiveBack {
+    DevBuf<unsigned char>* buf;
+    ~GiveBack() {
+      if (buf->size() > kBuildScratchKept) buf->release();
+    }
+  } give_back{&build_scratch_};
   // rows start empty on every level
   CU(launch_fill_i32(rows0_.get(), n_ * stride0_, -1, stream_));
   CU(launch_fill_i32(rowsU_.get(), std::max<long long>(total_upper_, 1) * strideU_, -1, stream_));
 
-  std::vector<std::vector<int>> level_nodes((size_t)max_level_ + 1);
-  for (long long i = 0; i < n_; ++i)
-    for (int l = 1; l <= levels_h_[i]; ++l) level_nodes[l].push_back((int)i);
-  size_t max_upper_nodes = max_level_ >= 1 ? level_nodes[1].size() : 0;
-  CU(nodes_d.alloc(std::max<size_t>(max_upper_nodes, 1)));
-
   BuildScratch S;
-  S.st_ids = st_ids.get();
-  S.st_dist = st_dist.get();
-  S.pkeys = pkeys.get();
-  S.pkeys_sorted = pkeys_sorted.get();
-  S.pvals = pvals.get();
-  S.pvals_sorted = pvals_sorted.get();
-  S.sort_tmp = sort_tmp.get();
+  S.st_ids = reinterpret_cast<int*>(base + at_ids);
+  S.st_dist = reinterpret_cast<float*>(base + at_dist);
+  S.pkeys = reinterpret_cast<unsigned*>(base + at_keys);
+  S.pkeys_sorted = reinterpret_cast<unsigned*>(base + at_keys2);
+  S.pvals = reinterpret_cast<unsigned long long*>(base + at_vals);
+  S.pvals_sorted = reinterpret_cast<unsigned long long*>(base + at_vals2);
+  S.sort_tmp = base + at_tmp;
   S.sort_tmp_bytes = tmp_bytes;
   S.ticket = counters_.get() + 1;
   S.stats = stats_on_ ? counters_.get() + 4 : nullptr;
 
+  float* const dist0 = reinterpret_cast<float*>(base + at_dist0);
+  float* const distU = reinterpret_cast<float*>(base + at_distU);
+  int* const nodes_d = reinterpret_cast<int*>(base + at_nodes);
   long long batches = 0;
   for (int l = max_level_; l >= 0; --l) {
     const long long nl = l == 0 ? n_ : (long long)level_nodes[l].size();
@@ -540,7 +552,7 @@ int Engine::BuildGraph() {
     if (l > 0) {
       // the previous level's launches still read nodes_d
       CU(cudaStreamSynchronize(stream_));
-      CU(cudaMemcpyAsync(nodes_d.get(), level_nodes[l].data(), (size_t)nl * sizeof(int), cudaMemcpyHostToDevice,
+      CU(cudaMemcpyAsync(nodes_d, level_nodes[l].data(), (size_t)nl * sizeof(int), cudaMemcpyHostToDevice,
                          stream_));
     } else {
       CU(cudaStreamSynchronize(stream_));
@@ -549,14 +561,14 @@ int Engine::BuildGraph() {
     L.g = View();
     L.level = l;
     L.rows = l == 0 ? rows0_.get() : rowsU_.get();
-    L.dists = l == 0 ? dist0.get() : distU.get();
-    L.distU = distU.get();
+    L.dists = l == 0 ? dist0 : distU;
+    L.distU = distU;
     L.stride = l == 0 ? stride0_ : strideU_;
     L.max_m = l == 0 ? opt_.max_m0 : opt_.max_m;
     L.levels = levels_d_.get();
-    L.nodes = l == 0 ? nullptr : nodes_d.get();
+    L.nodes = l == 0 ? nullptr : nodes_d;
     L.n_level = nl;
-    L.went = went.get();
+    L.went = base + at_went;
     L.ef_construction = opt_.ef_construction;
     L.heuristic_coef = (float)opt_.heuristic_coef;
     L.save_remains = opt_.save_remains ? 1 : 0;
