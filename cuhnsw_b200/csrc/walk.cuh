@@ -86,9 +86,14 @@ struct KeyList {
       for (; step > 128; step >>= 1)
         if (less(lds64(min(at + 8 * step - 8, end)), key)) at += 8 * step;
     }
+    // four ways at a time: three reads under way together, four dependent steps instead of eight
 #pragma unroll
-    for (int step = 128; step > 0; step >>= 1)
-      if (less(lds64(min(at + 8 * step - 8, end)), key)) at += 8 * step;
+    for (int step = 64; step > 0; step >>= 2) {
+      int n = 0;
+#pragma unroll
+      for (int u = 1; u <= 3; ++u) n += less(lds64(min(at + 8 * u * step - 8, end)), key) ? 1 : 0;
+      at += 8 * n * step;
+    }
     {
       const uint2 v = lds64(at);
       keep = keep && !(v.x == key.x && (v.y | 1u) == key.y + 1u);  // listed already?
@@ -125,17 +130,26 @@ struct KeyList {
     const unsigned bit = 1u << lane;
     const int lowest = first >> 5;
     int w = (grown - 1) >> 5;
-    unsigned here = keys + 8 * (32 * w + lane);
-    bool exists = 32 * w + lane < grown;
-    for (; w >= lowest; --w) {
-      const unsigned word = lds32(marks + 4 * w);
-      below -= __popc(word);
-      const bool moves = exists && !(word & bit);
-      const uint2 v = lds64(moves ? here - 8 * (below + __popc(word & lower)) : keys);
+    // four windows at a time, top down: all are read before the first is written, and what they read lies below
+    // everything the windows before them wrote
+    for (; w >= lowest; w -= 4) {
+      unsigned word[4];
+      uint2 v[4];
+      bool moves[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) word[u] = lds32(marks + 4 * max(w - u, 0));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = 32 * (w - u) + lane;
+        below -= __popc(word[u]);
+        moves[u] = w - u >= lowest && i < grown && !(word[u] & bit);
+        v[u] = lds64(moves[u] ? keys + 8 * (i - below - __popc(word[u] & lower)) : keys);
+      }
       __syncwarp();
-      if (moves) sts64(here, v.x, v.y);
-      here -= 256;
-      exists = true;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (moves[u]) sts64(keys + 8 * (32 * (w - u) + lane), v[u].x, v[u].y);
+      __syncwarp();
     }
     __syncwarp();
     if (in) sts64(keys + 8 * place, key.x, key.y);
