@@ -41,7 +41,7 @@ struct SearchParams {
   int* out_ids;          // nq x topk
   float* out_dist;       // nq x topk
   int* out_found;        // nq
-  unsigned long long* ticket;  // work counter (zeroed by the launcher)
+  unsigned long long* ticket;  // work counter (zeroed by the launcher; null: block b serves query b)
   unsigned long long* stats;   // optional: evals, expansions, sweeps, inserts
   // filled by the launcher when it schedules the batch (see SearchSchedule): ticket t serves query order[t],
   // whose greedy descent through the upper layers has already ended at entry_node / entry_dist

@@ -27,10 +27,12 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_walk_kernel(SearchParams
     return;
   }
   for (;;) {
-    long long qi = 0;
-    if (lane == 0) qi = (long long)atomicAdd(p.ticket, 1ull);
-    qi = __shfl_sync(FULL, qi, 0);
-    if (__any_sync(FULL, qi >= p.nq)) break;
+    long long qi = blockIdx.x;
+    if (p.ticket) {
+      if (lane == 0) qi = (long long)atomicAdd(p.ticket, 1ull);
+      qi = __shfl_sync(FULL, qi, 0);
+      if (__any_sync(FULL, qi >= p.nq)) break;
+    }
     if (p.order) qi = __ldg(p.order + qi);
     walk.start(kWalkQuery, p.queries, qi);
     int cur;
@@ -59,6 +61,7 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_walk_kernel(SearchParams
     }
     if (lane == 0) p.out_found[qi] = found;
     __syncwarp();
+    if (!p.ticket) break;
   }
   walk.finish();
   if (p.stats && lane == 0) {
@@ -115,8 +118,8 @@ cudaError_t launch_walk_t(const SearchParams& p0, int table_top, int sm_count, c
     e = schedule_search(p, *sched, sm_count, stream);
     if (e != cudaSuccess) return e;
   }
-  e = cudaMemsetAsync(p.ticket, 0, sizeof(unsigned long long), stream);
-  if (e != cudaSuccess) return e;
+  if (p.nq <= grid) p.ticket = nullptr;  // a CTA for every query: nothing to hand out, and no counter to clear
+  else if ((e = cudaMemsetAsync(p.ticket, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
   kern<<<(unsigned)grid, 32 * W, smem, stream>>>(p);
   return cudaGetLastError();
 }
