@@ -97,11 +97,22 @@ class CuHNSW:
       # the copy of the previous corpus is written over if nobody else holds it
       if rows is None or rows.shape != data.shape or sys.getrefcount(rows) > 2 or np.may_share_memory(rows, data):
         rows = np.empty(data.shape, np.float32)
-      _fill_rows(rows, data, self.opt.nrz)
-    else:
-      rows = np.array(data, dtype=np.float32, copy=True)
-      if self.opt.nrz:
-        rows /= np.linalg.norm(rows, axis=1, keepdims=True)
+      self.data = rows
+      self.logger.info("data shape: %d x %d", *rows.shape)
+      if (not self.opt.nrz and data.dtype == np.float32 and data.flags.c_contiguous and
+          rows.nbytes >= _SHARED_ROWS_BYTES):
+        # the device gets the caller's rows as they are, while the copy is made
+        with concurrent.futures.ThreadPoolExecutor(1) as beside:
+          copied = beside.submit(_fill_rows, rows, data, False)
+          self.obj.set_data(data)
+          copied.result()
+      else:
+        _fill_rows(rows, data, self.opt.nrz)
+        self.obj.set_data(rows)
+      return
+    rows = np.array(data, dtype=np.float32, copy=True)
+    if self.opt.nrz:
+      rows /= np.linalg.norm(rows, axis=1, keepdims=True)
     self.data = rows
     self.logger.info("data shape: %d x %d", *rows.shape)
     self.obj.set_data(rows)
