@@ -500,7 +500,8 @@ int Engine::BuildGraph() {
   const size_t max_upper_nodes = max_level_ >= 1 ? level_nodes[1].size() : 0;
 
   // Everything the construction needs besides the graph, in one allocation (a dozen of them, and handing them back, took
-  // 3 to 30 ms).  Up to kBuildScratchKept bytes stay with the handle for its next build.
+  // 3 to 30 ms).  From a handle's second build on, up to kBuildScratchKept bytes stay for the next one; after the first
+  // they go back, and the handle's search buffers take their place without the driver mapping new memory.
   const size_t items = (size_t)bmax * smax;
   const size_t tmp_bytes = build_sort_tmp_bytes((long long)items);
   size_t total = 0;
@@ -519,13 +520,14 @@ int Engine::BuildGraph() {
   const size_t at_nodes = part(std::max<size_t>(max_upper_nodes, 1) * 4);
   CU(build_scratch_.alloc(total));
   unsigned char* const base = build_scratch_.get();
-  // goes back on every way out unless it is small
+  // on every way out
   struct GiveBack {
     DevBuf<unsigned char>* buf;
+    bool first;
     ~GiveBack() {
-      if (buf->size() > kBuildScratchKept) buf->release();
+      if (first || buf->size() > kBuildScratchKept) buf->release();
     }
-  } give_back{&build_scratch_};
+  } give_back{&build_scratch_, builds_++ == 0};
   // rows start empty on every level
   CU(launch_fill_i32(rows0_.get(), n_ * stride0_, -1, stream_));
   CU(launch_fill_i32(rowsU_.get(), std::max<long long>(total_upper_, 1) * strideU_, -1, stream_));

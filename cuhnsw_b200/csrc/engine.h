@@ -181,7 +181,8 @@ class Engine {
 
   DevBuf<float> vec_;
   DevBuf<int> rows0_, rowsU_, levels_d_, upper_base_d_, labels_d_;
-  DevBuf<unsigned char> build_scratch_;  // of the last build, if it was small
+  DevBuf<unsigned char> build_scratch_;  // of the last build, if it was small and not the first
+  long long builds_ = 0;
   static constexpr size_t kBuildScratchKept = 256u << 20;
   DevBuf<unsigned> records_[Pipeline::kDepth];  // pieces of an index file on their way (8 MB each, once a file was used)
   DevBuf<unsigned long long> counters_;  // [0] search ticket, [1..2] build tickets, [4..7] stats, [8..] tickets of the search lanes
