@@ -408,6 +408,10 @@ int Engine::AllocGraph() {
 int Engine::SetRandomLevels(const int* levels) {
   if (!has_data_) return Fail(kBadState, "set_data() must be called first");
   if (!levels && n_ > 0) return Fail(kInvalidArgument, "null levels");
+  int rc = EnsureDevice();
+  if (rc) return rc;
+  // searches still running on other streams read the graph whose arrays are written over from here on
+  if ((rc = WaitForSearches()) != kOk) return rc;
   levels_h_.assign((size_t)n_, 0);
   max_level_ = 0;
   enter_point_ = 0;
@@ -419,8 +423,7 @@ int Engine::SetRandomLevels(const int* levels) {
       enter_point_ = (int)i;
     }
   }
-  int rc = AllocGraph();
-  if (rc) return rc;
+  if ((rc = AllocGraph()) != kOk) return rc;
   has_levels_ = true;
   has_graph_ = false;
   Log(3, "max level: %d, enter point: %d", max_level_, enter_point_);

@@ -108,6 +108,30 @@ def test_a_rebuild_waits_for_searches_in_flight_and_a_destroyed_stream_does_no_h
   assert int(eng.search_knn(q[:100], 10, 64)[0].max()) < 5000
 
 
+def test_a_second_build_of_the_same_rows_waits_for_searches_in_flight():
+  """The second build writes over the graph arrays that are in place: set_random_levels alone, and the whole of
+  build(), must leave a search on another stream the graph it walks."""
+  import torch
+  eng, q = _engine(20000, 7000)
+  want = eng.search_knn(q, 10, 400)
+  dq = torch.from_numpy(q).cuda()
+  levels = eng.obj.get_graph()[0]
+  for again in (lambda: eng.obj.set_random_levels(levels), eng.build):
+    out = (torch.empty((len(q), 10), dtype=torch.int32, device="cuda"), torch.empty((len(q), 10), device="cuda"),
+           torch.empty(len(q), dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    eng.obj.set_stream(side.cuda_stream)
+    eng.obj.search_knn_device(dq.data_ptr(), len(q), 10, 400, out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr())
+    eng.obj.set_stream(0)
+    again()
+    torch.cuda.synchronize()
+    assert (out[0].cpu().numpy() == want[0]).all() and (out[2].cpu().numpy() == want[2]).all()
+    assert_same_bits(out[1].cpu().numpy(), want[1])
+    eng.build()  # (the same graph again)
+  assert (eng.search_knn(q, 10, 400)[0] == want[0]).all()
+
+
 @pytest.mark.parametrize("in_flight", [1, 3])
 def test_python_batch_generator_gives_the_blocking_answers_in_order(in_flight):
   """CuHNSW.search_knn_batches: batches of different sizes (a single 1-d query and an empty batch among them)
