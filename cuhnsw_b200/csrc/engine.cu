@@ -1022,7 +1022,8 @@ int Engine::SaveIndex(const char* path) {
   if (rc) return rc;
   CU(cudaStreamSynchronize(stream_));
   // An existing file is overwritten in place and cut to its new length at the end: its cached pages are used again
-  // instead of being freed and allocated anew.
+  // instead of being freed and allocated anew.  Until then zeros stand for its header, which no reader takes for an
+  // index: a save that is cut short never leaves new records in front of old ones in a file that loads.
   const int fd = ::open(path, O_WRONLY | O_CREAT | O_CLOEXEC, 0666);
   if (fd < 0) return Fail(kIoError, std::string("cannot open ") + path + " for writing");
   // closes the file on every way out; a file that was not written to the end is removed
@@ -1051,7 +1052,11 @@ int Engine::SaveIndex(const char* path) {
   h.m = (uint64_t)m;
   h.mult = opt_.level_mult;
   h.ef_construction = (uint64_t)opt_.ef_construction;
-  bool ok = WriteAll(fd, &h, sizeof(h));
+  struct stat st;
+  const bool regular = ::fstat(fd, &st) == 0 && S_ISREG(st.st_mode);
+  FileHeader none;
+  std::memset(&none, 0, sizeof(none));
+  bool ok = WriteAll(fd, regular ? &none : &h, sizeof(h));
   // Level-0 records are put together on the device, piece by piece, exactly as they lie in the file: one
   // kernel packs the adjacency rows into degree word + neighbour slots and writes the labels, another moves
   // the vectors out of their padded (fp32 or 16-bit) rows; a piece comes down into a page-locked buffer while the
@@ -1123,10 +1128,10 @@ int Engine::SaveIndex(const char* path) {
     fill += 4 + nbytes;
   }
   flush();
-  struct stat st;
-  if (ok && ::fstat(fd, &st) == 0 && S_ISREG(st.st_mode)) {
+  if (ok && regular) {
     const off_t end = ::lseek(fd, 0, SEEK_CUR);
-    ok = end >= 0 && (st.st_size == end || ::ftruncate(fd, end) == 0);
+    ok = end >= 0 && (st.st_size <= end || ::ftruncate(fd, end) == 0) && ::lseek(fd, 0, SEEK_SET) == 0 &&
+         WriteAll(fd, &h, sizeof(h));
   }
   guard.fd = -1;
   ok = (::close(fd) == 0) && ok;

@@ -1,6 +1,10 @@
 """Transfers between ordinary host arrays and the device go through page-locked buffers of 8 MB, in pieces: sizes
 around the edges of a piece and of the in-place path (256 KB), against the device-buffer search and the numpy reader of
 index files."""
+import concurrent.futures
+import os
+import resource
+
 import numpy as np
 import pytest
 
@@ -65,6 +69,38 @@ def test_rows_graph_and_files_of_several_pieces(n, d, row_dtype, max_m0, tmp_pat
   other.save_index(again)
   assert open(path, "rb").read() == open(again, "rb").read()
   assert (other.obj.get_graph()[1] == rows0).all()
+
+
+def test_an_interrupted_save_over_an_index_leaves_nothing_that_loads(tmp_path):
+  """The write fails half way through a file of the same shape; a second name keeps what was written so far."""
+  eng, _, _ = _index(30_000, 50)
+  path, kept = str(tmp_path / "x.index"), str(tmp_path / "kept.index")
+  eng.save_index(path)
+  os.link(path, kept)
+  whole = open(path, "rb").read()
+  soft, hard = resource.getrlimit(resource.RLIMIT_FSIZE)
+  resource.setrlimit(resource.RLIMIT_FSIZE, (len(whole) // 2, hard))
+  try:
+    with pytest.raises(RuntimeError, match="short write"):
+      eng.save_index(path)
+  finally:
+    resource.setrlimit(resource.RLIMIT_FSIZE, (soft, hard))
+  assert not os.path.exists(path) and os.path.getsize(kept) == len(whole)
+  with pytest.raises(RuntimeError, match="index file"):
+    CuHNSW(engine_options(dict(dist_type="l2"))).load_index(kept)
+  eng.save_index(kept)
+  assert open(kept, "rb").read() == whole
+
+
+def test_an_index_saved_into_a_pipe_is_the_file_byte_for_byte(tmp_path):
+  eng, _, _ = _index(30_000, 50)
+  path, pipe = str(tmp_path / "x.index"), str(tmp_path / "pipe")
+  eng.save_index(path)
+  os.mkfifo(pipe)
+  with concurrent.futures.ThreadPoolExecutor(1) as pool:
+    got = pool.submit(lambda: open(pipe, "rb").read())
+    eng.save_index(pipe)
+    assert got.result() == open(path, "rb").read()
 
 
 @pytest.mark.parametrize("rows,d", [(1, 3), (40_000, 50), (42_000, 50), (70_001, 33)])

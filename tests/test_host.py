@@ -115,9 +115,10 @@ def test_call_order_and_argument_checks():
     with pytest.raises(RuntimeError, match="shorter than its header"):
       b.load_index(short)
     bad = os.path.join(tmp, "bad.index")
-    open(bad, "wb").write(b"\xff" * 200)
-    with pytest.raises(RuntimeError, match="index file"):
-      b.load_index(bad)
+    for contents in (b"\xff" * 200, b"\0" * 96 + b"\xff" * 200):  # zeros: the header of an unfinished save
+      open(bad, "wb").write(contents)
+      with pytest.raises(RuntimeError, match="index file"):
+        b.load_index(bad)
 
 
 @pytest.mark.skipif(has_gpu(), reason="checks the failure mode of a machine without a GPU")
