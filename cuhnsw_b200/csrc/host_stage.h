@@ -48,13 +48,11 @@ class HostStage {
       for (void* p : free_) cudaFreeHost(p);
       made_ -= (int)free_.size();
       free_.clear();
-      quit_ = true;
+      ++generation_;
       threads.swap(threads_);
     }
     work_.notify_all();
     for (std::thread& t : threads) t.join();
-    std::lock_guard<std::mutex> lock(mu_);
-    quit_ = false;
   }
 
   // A buffer, or nullptr: page-locked memory cannot be had, or, without `wait`, all buffers are in use.  A thread that
@@ -100,7 +98,7 @@ class HostStage {
     {
       std::lock_guard<std::mutex> lock(mu_);
       const int want = std::min({n - 1, kMaxThreads, (int)std::thread::hardware_concurrency() - 1});
-      while ((int)threads_.size() < want && !quit_) threads_.emplace_back([this] { Serve(); });
+      while ((int)threads_.size() < want) threads_.emplace_back([this, mine = generation_] { Serve(mine); });
       jobs_.push_back(job);
     }
     work_.notify_all();
@@ -138,9 +136,10 @@ class HostStage {
       if (++job.done == job.n) job.over.notify_all();
     }
   }
-  void Serve() {
+  // until the users that this thread was started for are gone; others may have come and gone since
+  void Serve(long long mine) {
     std::unique_lock<std::mutex> lock(mu_);
-    for (;;) {
+    while (mine == generation_) {
       std::shared_ptr<Job> job;
       for (auto& j : jobs_)
         if (j->next < j->n) {
@@ -148,7 +147,6 @@ class HostStage {
           break;
         }
       if (!job) {
-        if (quit_) return;
         work_.wait(lock);
         continue;
       }
@@ -164,7 +162,7 @@ class HostStage {
   std::vector<std::thread> threads_;
   std::deque<std::shared_ptr<Job>> jobs_;
   int users_ = 0, made_ = 0;
-  bool quit_ = false;
+  long long generation_ = 0;  // counts the times the last user went
 };
 
 // A buffer of the stage for the lifetime of a scope.

@@ -1,0 +1,70 @@
+// Host-only exercise of host_stage.h: the CUDA calls it makes are answered by the fakes below.
+//   host_stage_test <name>   runs one check; exit code 0 = passed
+#include "host_stage.h"
+
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <string>
+
+extern "C" {
+cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
+  *p = std::malloc(bytes);
+  return *p ? cudaSuccess : cudaErrorMemoryAllocation;
+}
+cudaError_t cudaFreeHost(void* p) {
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t*, unsigned) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+}
+
+using hnsw::HostStage;
+
+namespace {
+#define EXPECT(x)                                                  \
+  do {                                                             \
+    if (!(x)) {                                                    \
+      std::fprintf(stderr, "line %d: %s\n", __LINE__, #x);         \
+      std::exit(1);                                                \
+    }                                                              \
+  } while (0)
+
+// a parallel loop gives every part exactly one turn
+void Loop(int n) {
+  std::vector<int> turns((size_t)n, 0);
+  HostStage::Get().ParallelFor(n, [&](int i) { ++turns[(size_t)i]; });
+  for (int t : turns) EXPECT(t == 1);
+}
+
+// the last user goes, and while its threads are on their way out another one comes and goes: nobody waits for good
+void Users() {
+  for (int i = 0; i < 3000; ++i) {
+    HostStage::Get().AddUser();
+    Loop(6);
+    std::atomic<bool> go{false};
+    std::thread other([&go, i] {
+      while (!go) {
+      }
+      for (volatile int spin = 0; spin < i % 60 * 50; ++spin) {
+      }
+      HostStage::Get().AddUser();
+      HostStage::Get().DropUser();
+    });
+    go = true;
+    HostStage::Get().DropUser();
+    other.join();
+  }
+}
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::string name = argc > 1 ? argv[1] : "";
+  if (name == "users") Users();
+  else return 2;
+  return 0;
+}
