@@ -17,6 +17,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -98,7 +99,11 @@ class HostStage {
     {
       std::lock_guard<std::mutex> lock(mu_);
       const int want = std::min({n - 1, kMaxThreads, (int)std::thread::hardware_concurrency() - 1});
-      while ((int)threads_.size() < want) threads_.emplace_back([this, mine = generation_] { Serve(mine); });
+      try {
+        while ((int)threads_.size() < want) threads_.emplace_back([this, mine = generation_] { Serve(mine); });
+      } catch (const std::system_error&) {
+        // the process is at its limit of threads: the calling thread and those there are do the work
+      }
       jobs_.push_back(job);
     }
     work_.notify_all();

@@ -2,7 +2,10 @@
 //   host_stage_test <name>   runs one check; exit code 0 = passed
 #include "host_stage.h"
 
+#include <dlfcn.h>
+
 #include <atomic>
+#include <cerrno>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
@@ -21,6 +24,15 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t*, unsigned) { return cudaSucces
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+}
+
+// the process is at its limit of threads after so many more
+static std::atomic<int> g_threads_left{1 << 30};
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* attr, void* (*f)(void*), void* arg) {
+  if (g_threads_left-- <= 0) return EAGAIN;
+  using Real = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+  static const Real real = reinterpret_cast<Real>(dlsym(RTLD_NEXT, "pthread_create"));
+  return real(t, attr, f, arg);
 }
 
 using hnsw::HostStage;
@@ -60,11 +72,25 @@ void Users() {
     other.join();
   }
 }
+
+// no thread, or fewer than asked for, can be started: the work is done all the same
+void ThreadLimit() {
+  for (int left : {0, 1, 3}) {
+    HostStage::Get().AddUser();
+    g_threads_left = left;
+    for (int i = 0; i < 3; ++i) Loop(9);
+    std::vector<char> from(5u << 20, 'x'), to(from.size());
+    HostStage::Get().Copy(to.data(), from.data(), from.size());
+    EXPECT(from == to);
+    HostStage::Get().DropUser();
+  }
+}
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   if (name == "users") Users();
+  else if (name == "thread-limit") ThreadLimit();
   else return 2;
   return 0;
 }

@@ -14,10 +14,10 @@ def program(tmp_path_factory):
   cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
   subprocess.check_call(["g++", "-std=c++17", "-O1", "-g", "-Wall", "-pthread", "-I", os.path.join(cuda, "include"),
                          "-I", os.path.join(ROOT, "cuhnsw_b200", "csrc"),
-                         os.path.join(ROOT, "tests", "native", "host_stage_test.cpp"), "-o", out])
+                         os.path.join(ROOT, "tests", "native", "host_stage_test.cpp"), "-o", out, "-ldl"])
   return out
 
 
-@pytest.mark.parametrize("check", ["users"])
+@pytest.mark.parametrize("check", ["users", "thread-limit"])
 def test_host_stage(program, check):
   subprocess.run([program, check], check=True, timeout=60)
