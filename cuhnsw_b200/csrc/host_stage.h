@@ -9,6 +9,7 @@
 // of it is given back when the last handle is destroyed.  Any number of threads may use it at once.
 #pragma once
 #include <cuda_runtime.h>
+#include <pthread.h>
 
 #include <algorithm>
 #include <condition_variable>
@@ -17,6 +18,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -33,7 +35,11 @@ class HostStage {
 
   // (never destroyed: handles that outlive main() may still use it)
   static HostStage& Get() {
-    static HostStage* one = new HostStage;
+    static HostStage* one = [] {
+      auto* stage = new HostStage;
+      pthread_atfork([] { Get().mu_.lock(); }, [] { Get().mu_.unlock(); }, [] { Get().Forked(); });
+      return stage;
+    }();
     return *one;
   }
 
@@ -159,6 +165,17 @@ class HostStage {
       Run(*job);
       lock.lock();
     }
+  }
+
+  // In a forked child: the threads are not there, so nobody may wait for them, or on what they waited on.  Their objects
+  // are left behind (a destructor would wait).
+  void Forked() {
+    new (&threads_) std::vector<std::thread>;
+    new (&jobs_) std::deque<std::shared_ptr<Job>>;
+    new (&work_) std::condition_variable;
+    new (&room_) std::condition_variable;
+    ++generation_;
+    mu_.unlock();
   }
 
   std::mutex mu_;

@@ -3,6 +3,8 @@
 #include "host_stage.h"
 
 #include <dlfcn.h>
+#include <sys/wait.h>
+#include <unistd.h>
 
 #include <atomic>
 #include <cerrno>
@@ -85,12 +87,29 @@ void ThreadLimit() {
     HostStage::Get().DropUser();
   }
 }
+
+// a forked child, which has none of the threads, can use what it inherited and give it back
+void Fork() {
+  HostStage::Get().AddUser();
+  Loop(9);
+  const pid_t child = fork();
+  if (child == 0) {
+    alarm(20);
+    Loop(9);
+    HostStage::Get().DropUser();
+    _exit(0);
+  }
+  int status = -1;
+  EXPECT(waitpid(child, &status, 0) == child && status == 0);
+  HostStage::Get().DropUser();
+}
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string name = argc > 1 ? argv[1] : "";
   if (name == "users") Users();
   else if (name == "thread-limit") ThreadLimit();
+  else if (name == "fork") Fork();
   else return 2;
   return 0;
 }
