@@ -750,7 +750,7 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
   const bool small = (size_t)nq * per_query <= kInPlaceBytes;
   if (pieces == 1 && !small) return kOk;
   struct Piece {
-    std::unique_ptr<StageBuffer> buffer;
+    StreamBuffer buffer;
     cudaStream_t stream = nullptr;
     long long first = 0, count = 0;
     float *q = nullptr, *dist = nullptr;
@@ -759,8 +759,7 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
   int nslots = 0;
   for (; nslots < (int)std::min<long long>(pieces, kPieces); ++nslots) {
     Piece& s = slots[nslots];
-    s.buffer.reset(new StageBuffer(nslots == 0));
-    if (!s.buffer->get()) break;
+    if (!s.buffer.Open(nslots == 0)) break;
     if (pieces == 1) {
       s.stream = stream_;
     } else {
@@ -770,7 +769,12 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
   }
   if (nslots == 0) return kOk;
   *handled = true;
-  const cudaStream_t own = stream_;
+  // the pieces are enqueued on their own streams; the handle's is back on every way out
+  struct OwnStream {
+    cudaStream_t* at;
+    cudaStream_t own;
+    ~OwnStream() { *at = own; }
+  } own_stream{&stream_, stream_};
   // every stream's scratch before the first launch: an allocation waits for what runs
   for (int i = 0; i < nslots && pieces > 1 && !rc; ++i) {
     SearchLane* lane = nullptr;
@@ -782,7 +786,7 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
   if (rc) return rc;
   // waits for a piece and hands its results to the caller
   auto collect = [&](Piece& s) -> cudaError_t {
-    const cudaError_t e = cudaStreamSynchronize(s.stream);
+    const cudaError_t e = s.buffer.Wait();
     if (e == cudaSuccess) {
       const size_t words = (size_t)s.count * topk, at = (size_t)s.first * topk;
       // ids, distances and counts as one row of words, shared out in equal parts
@@ -812,17 +816,18 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
     s.first = at;
     s.count = nq * (i + 1) / pieces - at;
     at += s.count;
-    s.q = reinterpret_cast<float*>(s.buffer->get());
+    s.q = reinterpret_cast<float*>(s.buffer.get());
     s.ids = reinterpret_cast<int*>(s.q + ((size_t)s.count * d_ + 63) / 64 * 64);
     s.dist = reinterpret_cast<float*>(s.ids + ((size_t)s.count * topk + 31) / 32 * 32);
     s.found = reinterpret_cast<int*>(s.dist + ((size_t)s.count * topk + 31) / 32 * 32);
     stage.Copy(s.q, q + (size_t)s.first * d_, (size_t)s.count * d_ * 4);
     stream_ = s.stream;
+    s.buffer.Use(s.stream);
     rc = small ? SearchGraphDevice(s.q, s.count, topk, ef, s.ids, s.dist, s.found)
                : SearchGraphCopied(s.q, s.count, topk, ef, s.ids, s.dist, s.found);
-    stream_ = own;
+    stream_ = own_stream.own;
     if (rc) {
-      cudaStreamSynchronize(s.stream);  // a copy from the buffer may be under way
+      s.buffer.Wait();  // a copy from the buffer may be under way
       s.count = 0;
     }
   }

@@ -200,6 +200,38 @@ class StageBuffer {
   void* p_;
 };
 
+// A staging buffer that the work of a stream reads and writes: it goes back when that work is over, also when an
+// exception takes the scope down.
+class StreamBuffer {
+ public:
+  StreamBuffer() = default;
+  StreamBuffer(const StreamBuffer&) = delete;
+  StreamBuffer& operator=(const StreamBuffer&) = delete;
+  ~StreamBuffer() { Wait(); }
+  // false: none to be had
+  bool Open(bool wait) {
+    buffer_.reset(new StageBuffer(wait));
+    if (!buffer_->get()) buffer_.reset();
+    return buffer_ != nullptr;
+  }
+  unsigned char* get() const { return buffer_->get(); }
+  // from here on `stream` may have work on the buffer
+  void Use(cudaStream_t stream) {
+    stream_ = stream;
+    busy_ = true;
+  }
+  cudaError_t Wait() {
+    if (!busy_) return cudaSuccess;
+    busy_ = false;
+    return cudaStreamSynchronize(stream_);
+  }
+
+ private:
+  std::unique_ptr<StageBuffer> buffer_;
+  cudaStream_t stream_ = nullptr;
+  bool busy_ = false;
+};
+
 // A ring of staging buffers for a transfer in pieces: fill or drain one while the device works on the others.
 class Pipeline {
  public:

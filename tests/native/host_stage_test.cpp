@@ -25,6 +25,9 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t*, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+static int g_waits = 0;
+static bool g_held = true;  // the buffers were all in use whenever a stream was waited for
+cudaError_t cudaStreamSynchronize(cudaStream_t);
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 }
 
@@ -38,6 +41,14 @@ extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* attr, void* (*
 }
 
 using hnsw::HostStage;
+
+cudaError_t cudaStreamSynchronize(cudaStream_t) {
+  ++g_waits;
+  void* p = HostStage::Get().Acquire(false);
+  if (p) g_held = false;
+  HostStage::Get().Release(p);
+  return cudaSuccess;
+}
 
 namespace {
 #define EXPECT(x)                                                  \
@@ -75,6 +86,31 @@ void Users() {
   }
 }
 
+// a buffer that a stream works on goes back behind that work, also when an exception takes its scope down
+void Unwinding() {
+  HostStage::Get().AddUser();
+  void* others[HostStage::kMaxBuffers - 1];
+  for (void*& p : others) EXPECT((p = HostStage::Get().Acquire(false)) != nullptr);
+  try {
+    hnsw::StreamBuffer b;
+    EXPECT(b.Open(false));
+    b.Use(nullptr);
+    throw std::bad_alloc();
+  } catch (const std::bad_alloc&) {
+  }
+  EXPECT(g_waits == 1 && g_held);
+  {
+    hnsw::StreamBuffer b;
+    EXPECT(b.Open(false));
+    EXPECT(!hnsw::StreamBuffer().Open(false));
+    b.Use(nullptr);
+    EXPECT(b.Wait() == cudaSuccess && b.Wait() == cudaSuccess);
+  }
+  EXPECT(g_waits == 2 && g_held);
+  for (void* p : others) HostStage::Get().Release(p);
+  HostStage::Get().DropUser();
+}
+
 // no thread, or fewer than asked for, can be started: the work is done all the same
 void ThreadLimit() {
   for (int left : {0, 1, 3}) {
@@ -110,6 +146,7 @@ int main(int argc, char** argv) {
   if (name == "users") Users();
   else if (name == "thread-limit") ThreadLimit();
   else if (name == "fork") Fork();
+  else if (name == "unwinding") Unwinding();
   else return 2;
   return 0;
 }

@@ -18,6 +18,6 @@ def program(tmp_path_factory):
   return out
 
 
-@pytest.mark.parametrize("check", ["users", "thread-limit", "fork"])
+@pytest.mark.parametrize("check", ["users", "thread-limit", "fork", "unwinding"])
 def test_host_stage(program, check):
   subprocess.run([program, check], check=True, timeout=60)
