@@ -100,6 +100,7 @@ Engine::~Engine() {
     }
   for (cudaStream_t s : piece_streams_)
     if (s) cudaStreamDestroy(s);
+  if (pieces_after_) cudaEventDestroy(pieces_after_);
   HostStage::Get().DropUser();
 }
 
@@ -153,7 +154,7 @@ int Engine::EnsureDevice() {
   sm_count_ = prop.multiProcessorCount;
   smem_optin_ = prop.sharedMemPerBlockOptin;
   smem_per_sm_ = prop.sharedMemPerMultiprocessor;
-  CU(counters_.alloc(8 + kSearchLanes));
+  CU(counters_.alloc(8 + kSearchLanes + kPieces));
   CU(cudaMemset(counters_.get(), 0, counters_.size() * sizeof(unsigned long long)));
   Log(3, "device %d: %s, sm_%d%d, %d SMs, %zu B shared memory per block", dev, prop.name, prop.major, prop.minor,
       sm_count_, smem_optin_);
@@ -653,12 +654,12 @@ int Engine::LaneFor(cudaStream_t stream, SearchLane** out) {
   for (SearchLane& l : lanes_)
     if (l.used && l.stream == stream) pick = &l;
   if (!pick) {
-    for (SearchLane& l : lanes_)
-      if (!l.used && !pick) pick = &l;
+    for (int i = 0; i < kSearchLanes; ++i)
+      if (!lanes_[i].used && !pick) pick = &lanes_[i];
     if (!pick) {
       pick = &lanes_[0];
-      for (SearchLane& l : lanes_)
-        if (l.stamp < pick->stamp) pick = &l;
+      for (int i = 1; i < kSearchLanes; ++i)
+        if (lanes_[i].stamp < pick->stamp) pick = &lanes_[i];
       if (pick->pending) CU(cudaEventSynchronize(pick->done));  // its last search is over before another stream uses it
       pick->pending = false;
     }
@@ -763,8 +764,11 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
     if (pieces == 1) {
       s.stream = stream_;
     } else {
+      SearchLane& lane = lanes_[kSearchLanes + nslots];
       if (!piece_streams_[nslots]) CU(cudaStreamCreateWithFlags(&piece_streams_[nslots], cudaStreamNonBlocking));
-      s.stream = piece_streams_[nslots];
+      if (!lane.done) CU(cudaEventCreateWithFlags(&lane.done, cudaEventDisableTiming));
+      s.stream = lane.stream = piece_streams_[nslots];
+      lane.used = true;
     }
   }
   if (nslots == 0) return kOk;
@@ -784,6 +788,12 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
       rc = PrepareSchedule(most, lane, &sched);
   }
   if (rc) return rc;
+  // like the one search it stands for, the pieces come behind whatever the caller has put on the handle's stream
+  if (pieces > 1) {
+    if (!pieces_after_) CU(cudaEventCreateWithFlags(&pieces_after_, cudaEventDisableTiming));
+    CU(cudaEventRecord(pieces_after_, stream_));
+    for (int i = 0; i < nslots; ++i) CU(cudaStreamWaitEvent(slots[i].stream, pieces_after_, 0));
+  }
   // waits for a piece and hands its results to the caller
   auto collect = [&](Piece& s) -> cudaError_t {
     const cudaError_t e = s.buffer.Wait();

@@ -185,14 +185,15 @@ class Engine {
   long long builds_ = 0;
   static constexpr size_t kBuildScratchKept = 256u << 20;
   DevBuf<unsigned> records_[Pipeline::kDepth];  // pieces of an index file on their way (8 MB each, once a file was used)
-  DevBuf<unsigned long long> counters_;  // [0] search ticket, [1..2] build tickets, [4..7] stats, [8..] tickets of the search lanes
+  DevBuf<unsigned long long> counters_;  // [1..3] build tickets, [4..7] stats, [8..] tickets of the search lanes
   bool stats_on_ = false;
   // Scratch of one search in flight: its ticket counter and the grow-only arrays of the
   // longest-first schedule (four words per query; six and the sort's storage for large batches).  A search uses the set that belongs to the
   // stream it is enqueued on, so searches enqueued on different streams can run at the same time: the tail of
   // one batch (a launch lasts as long as its longest walk) overlaps with the next batch.  A stream beyond
   // kSearchLanes takes over the least recently used set after waiting for the search that used it last (through
-  // the set's own event, which outlives a stream the caller has destroyed since).
+  // the set's own event, which outlives a stream the caller has destroyed since).  The pieces of a large host-buffer
+  // search have kPieces sets behind those, so that they never take one from a caller's stream.
   struct SearchLane {
     cudaStream_t stream = nullptr;
     bool used = false;
@@ -210,8 +211,9 @@ class Engine {
   };
   LaneIo IoOf(long long nq, int topk) const;
   int ReserveIo(SearchLane* lane, const LaneIo& io);
-  static constexpr int kSearchLanes = 8;
-  SearchLane lanes_[kSearchLanes];
+  static constexpr int kSearchLanes = 8;  // for the caller's streams
+  static constexpr int kPieces = 4;       // pieces of one large host-buffer search in flight, with sets of their own
+  SearchLane lanes_[kSearchLanes + kPieces];
   unsigned long long lane_clock_ = 0;
   int LaneFor(cudaStream_t stream, SearchLane** lane);
   int MarkLane(SearchLane* lane);  // records `done` on the engine's stream
@@ -220,8 +222,9 @@ class Engine {
                         bool* handled);
   int SearchGraphCopied(const float* q, long long nq, int topk, int ef, int* nns, float* dist, int* found);
   static constexpr size_t kInPlaceBytes = 256u << 10;  // queries and results of a search that are staged in place
-  static constexpr int kPieces = 4;          // pieces of one search in flight
-  cudaStream_t piece_streams_[kPieces] = {};  // created when a search first needs them
+  // created when a search first needs them, with the event by which they wait for what is on the engine's stream
+  cudaStream_t piece_streams_[kPieces] = {};
+  cudaEvent_t pieces_after_ = nullptr;
   int WaitForSearches();           // every search enqueued so far, on whatever stream, is over
   int PrepareSchedule(long long nq, SearchLane* lane, SearchSchedule* s);
   double last_build_seconds_ = 0.0;

@@ -47,6 +47,30 @@ def test_host_searches_around_the_edges_of_the_staging_sizes(d, topk):
     assert_same_bits(got[1], want[1][:nq])
 
 
+@pytest.mark.parametrize("queries", [300, 60_000])
+def test_a_blocking_host_search_comes_behind_the_work_on_the_handles_stream(queries):
+  """In place and in pieces, on a stream of the caller's and on the legacy default stream."""
+  import torch
+  eng, _, rng = _index(3000, 20)
+  q = rng.standard_normal((queries, 20)).astype(np.float32)
+  want = eng.search_knn(q, 10, 40)
+  a = torch.randn((4096, 4096), device="cuda")
+  for stream in (torch.cuda.Stream(), torch.cuda.default_stream()):
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+      for _ in range(100):  # some tens of ms
+        a = a @ a * 1e-2
+      before = torch.cuda.Event()
+      before.record(stream)
+    eng.obj.set_stream(stream.cuda_stream)
+    got = eng.search_knn(q, 10, 40)
+    assert before.query()
+    assert eng.obj.current_stream() == stream.cuda_stream
+    assert (got[0] == want[0]).all() and (got[2] == want[2]).all()
+    assert_same_bits(got[1], want[1])
+  eng.obj.set_stream(0)
+
+
 @pytest.mark.parametrize("n,d,row_dtype,max_m0", [(40_000, 104, "f32", 8), (33_001, 77, "f32", 64),
                                                   (50_001, 50, "f16", 33), (300, 9, "bf16", 8)])
 def test_rows_graph_and_files_of_several_pieces(n, d, row_dtype, max_m0, tmp_path):
