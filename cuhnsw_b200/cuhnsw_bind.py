@@ -136,6 +136,9 @@ class CuHNSWBind:
     arr = np.ascontiguousarray(levels, dtype=np.int32)
     if arr.ndim != 1:
       raise RuntimeError("levels must be 1d array")
+    num_data = self.describe()["num_data"]  # the engine reads this many
+    if arr.shape[0] < num_data:
+      raise RuntimeError(f"{arr.shape[0]} levels for {num_data} rows")
     self._check(self._lib.cuhnsw_set_random_levels(self._h, arr.ctypes.data))
 
   def build_graph(self):

@@ -338,6 +338,17 @@ def _rounded(x, row_dtype="f16"):
   return x.astype(np.float16).astype(np.float32)
 
 
+def test_levels_for_fewer_rows_than_there_are_are_refused():
+  eng = CuHNSW(engine_options(dict(dist_type="l2")))
+  eng.set_data(np.arange(300, dtype=np.float32).reshape(100, 3))
+  with pytest.raises(RuntimeError, match="99 levels for 100 rows"):
+    eng.obj.set_random_levels(np.zeros(99, np.int32))
+  for count in (100, 101):
+    eng.obj.set_random_levels(np.zeros(count, np.int32))
+  eng.obj.build_graph()
+  assert (eng.obj.get_graph()[0] == 0).all()
+
+
 @pytest.mark.parametrize("d,dist_type,row_dtype", [(50, "dot", "f16"), (33, "l2", "f16"), (128, "l2", "f16"),
                                                    (200, "dot", "f16"), (960, "l2", "f16"), (50, "dot", "bf16"),
                                                    (97, "l2", "bf16"), (960, "l2", "bf16")])
