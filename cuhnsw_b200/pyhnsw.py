@@ -10,7 +10,6 @@ over once, and every search is one call into the device-resident index.
 import concurrent.futures
 import json
 import os
-import sys
 import tempfile
 
 import numpy as np
@@ -93,11 +92,7 @@ class CuHNSW:
       self.logger.warning("it is not common to set nrz = True and dist_type = l2")
     data = np.asarray(data)
     if data.ndim == 2 and data.size > 0:
-      rows, self.data = self.data, None
-      # the copy of the previous corpus is written over if nobody else holds it
-      if rows is None or rows.shape != data.shape or sys.getrefcount(rows) > 2 or np.may_share_memory(rows, data):
-        rows = np.empty(data.shape, np.float32)
-      self.data = rows
+      self.data = rows = np.empty(data.shape, np.float32)
       self.logger.info("data shape: %d x %d", *rows.shape)
       if (not self.opt.nrz and data.dtype == np.float32 and data.flags.c_contiguous and
           rows.nbytes >= _SHARED_ROWS_BYTES):

@@ -5,6 +5,7 @@ import json
 import math
 import os
 import re
+import sys
 import tempfile
 
 import numpy as np
@@ -193,6 +194,34 @@ def test_python_api_constructor_semantics():
     CuHNSW({"dist_type": "hamming"})
   with pytest.raises(AssertionError):
     CuHNSW({"block_dim": 48})
+
+
+class _Engine:
+  """Stands in for the binding of a CuHNSW: takes the rows, refuses them if told to."""
+  refuse = False
+
+  def set_data(self, rows):
+    if self.refuse:
+      raise RuntimeError("refused")
+    self.rows = np.array(rows)
+
+  def __call__(self, **opt):
+    from cuhnsw_b200 import CuHNSW
+    index = CuHNSW(dict(py_log_level=1, c_log_level=0, **opt))
+    index.obj = self
+    return index
+
+
+def test_set_data_never_writes_over_an_array_it_handed_out(monkeypatch):
+  """Also where the interpreter counts references to a local differently."""
+  real = sys.getrefcount
+  monkeypatch.setattr(sys, "getrefcount", lambda x: real(x) - 2)
+  for n in (5, 50_000):
+    index = _Engine()(dist_type="l2")
+    index.set_data(np.ones((n, 50), np.float32))
+    kept = index.data
+    index.set_data(np.zeros((n, 50), np.float32))
+    assert (kept == 1).all() and (index.data == 0).all()
 
 
 def test_benchmark_arithmetic():
