@@ -92,17 +92,22 @@ class CuHNSW:
       self.logger.warning("it is not common to set nrz = True and dist_type = l2")
     data = np.asarray(data)
     if data.ndim == 2 and data.size > 0:
-      self.data = rows = np.empty(data.shape, np.float32)
-      self.logger.info("data shape: %d x %d", *rows.shape)
+      rows = np.empty(data.shape, np.float32)
       if (not self.opt.nrz and data.dtype == np.float32 and data.flags.c_contiguous and
           rows.nbytes >= _SHARED_ROWS_BYTES):
         # the device gets the caller's rows as they are, while the copy is made
+        self.logger.info("data shape: %d x %d", *rows.shape)
         with concurrent.futures.ThreadPoolExecutor(1) as beside:
           copied = beside.submit(_fill_rows, rows, data, False)
-          self.obj.set_data(data)
-          copied.result()
+          try:
+            self.obj.set_data(data)
+          finally:
+            copied.result()
+            self.data = rows
       else:
         _fill_rows(rows, data, self.opt.nrz)
+        self.data = rows  # (values that do not convert leave everything as it was)
+        self.logger.info("data shape: %d x %d", *rows.shape)
         self.obj.set_data(rows)
       return
     rows = np.array(data, dtype=np.float32, copy=True)

@@ -224,6 +224,27 @@ def test_set_data_never_writes_over_an_array_it_handed_out(monkeypatch):
     assert (kept == 1).all() and (index.data == 0).all()
 
 
+@pytest.mark.parametrize("n", [5, 50_000])
+def test_rows_that_do_not_convert_leave_the_corpus_in_place(n):
+  index = _Engine()(dist_type="l2")
+  index.set_data(np.ones((n, 50), np.float32))
+  bad = np.full((n + 1, 50), 2, object)
+  bad[n // 2, 7] = "seven"
+  for rows in (bad, bad[:n]):
+    with pytest.raises(ValueError):
+      index.set_data(rows)
+    assert index.data.shape == (n, 50) and (index.data == 1).all() and (index.obj.rows == 1).all()
+
+
+@pytest.mark.parametrize("n", [5, 50_000])
+def test_rows_that_the_engine_refuses_are_a_whole_copy(n):
+  index = _Engine()(dist_type="l2")
+  index.obj.refuse = True
+  with pytest.raises(RuntimeError, match="refused"):
+    index.set_data(np.ones((n, 50), np.float32))
+  assert (index.data == 1).all()
+
+
 def test_benchmark_arithmetic():
   import bench
   assert bench.algorithmic_bytes_per_query(10, 2, 1, 50, 12, 24, 10) == 10 * 200 + 2 * 100 + 52 + 200 + 80
