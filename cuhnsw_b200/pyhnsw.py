@@ -91,10 +91,10 @@ class CuHNSW:
     if self.opt.nrz and self.opt.dist_type == "l2":
       self.logger.warning("it is not common to set nrz = True and dist_type = l2")
     data = np.asarray(data)
-    if data.ndim == 2 and data.size > 0:
+    # (a copy in another order has its rows' squares summed in another order: those are left to numpy as a whole)
+    if data.ndim == 2 and data.size > 0 and data.flags.c_contiguous:
       rows = np.empty(data.shape, np.float32)
-      if (not self.opt.nrz and data.dtype == np.float32 and data.flags.c_contiguous and
-          rows.nbytes >= _SHARED_ROWS_BYTES):
+      if not self.opt.nrz and data.dtype == np.float32 and rows.nbytes >= _SHARED_ROWS_BYTES:
         # the device gets the caller's rows as they are, while the copy is made
         self.logger.info("data shape: %d x %d", *rows.shape)
         with concurrent.futures.ThreadPoolExecutor(1) as beside:

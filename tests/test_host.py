@@ -237,6 +237,22 @@ def test_rows_that_do_not_convert_leave_the_corpus_in_place(n):
 
 
 @pytest.mark.parametrize("n", [5, 50_000])
+@pytest.mark.parametrize("order", ["C", "F", "every other column", "every other row", "backwards"])
+def test_rows_in_any_memory_order_get_numpys_bits(n, order):
+  x = np.random.default_rng(n).standard_normal((n, 50))
+  if order == "every other column":
+    x = np.random.default_rng(n).standard_normal((n, 100))[:, ::2]
+  x = {"F": np.asfortranarray(x), "every other row": np.repeat(x, 2, axis=0)[::2], "backwards": x[::-1]}.get(order, x)
+  for dtype in (np.float64, np.float32):
+    index = _Engine()(dist_type="dot", nrz=True)
+    index.set_data(x.astype(dtype, copy=False))
+    want = np.array(x, dtype=np.float32, copy=True)
+    want /= np.linalg.norm(want, axis=1, keepdims=True)
+    assert (np.ascontiguousarray(index.data).view(np.uint32) == np.ascontiguousarray(want).view(np.uint32)).all()
+    assert (index.data == index.obj.rows).all()
+
+
+@pytest.mark.parametrize("n", [5, 50_000])
 def test_rows_that_the_engine_refuses_are_a_whole_copy(n):
   index = _Engine()(dist_type="l2")
   index.obj.refuse = True
