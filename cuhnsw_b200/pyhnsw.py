@@ -7,10 +7,12 @@ import.  The implementation is this project's own: the options travel to the C A
 file (the binding's ``init`` takes a path, cuhnsw/bindings.cc:22-24), the vectors are handed
 over once, and every search is one call into the device-resident index.
 """
-import concurrent.futures
+import collections
+import contextvars
 import json
 import os
 import tempfile
+import threading
 
 import numpy as np
 
@@ -27,10 +29,37 @@ _THREADS = 8
 _BLOCK_BYTES = 1 << 20
 
 
-def _fill_rows(rows, data, normalise):
+def _run_beside(work, count):
+  """Calls work() on up to `count` threads of its own, in the caller's context (numpy.errstate is part of it), and on the
+  calling thread; a process at its limit of threads does with those there are."""
+  failed = []
+
+  def guarded():
+    try:
+      work()
+    except BaseException as err:  # pylint: disable=broad-except
+      failed.append(err)
+
+  threads = []
+  for _ in range(count):
+    thread = threading.Thread(target=contextvars.copy_context().run, args=(guarded,))
+    try:
+      thread.start()
+    except RuntimeError:
+      break
+    threads.append(thread)
+  guarded()
+  for thread in threads:
+    thread.join()
+  if failed:
+    raise failed[0]
+
+
+def _fill_rows(rows, data, normalise, before=None):
   """rows[...] = data as float32, each row divided by its norm if asked for.  Large corpora by several threads in blocks
   that stay in a core's cache: a row's norm does not depend on the rows around it, so the values are the same.  (512 MB
-  in one thread: 100 ms, mostly page faults of the fresh copy.)"""
+  in one thread: 100 ms, mostly page faults of the fresh copy.)  before: what the calling thread does first, while the
+  others copy."""
   def block(lo, hi):
     part = rows[lo:hi]
     part[...] = data[lo:hi]
@@ -41,9 +70,22 @@ def _fill_rows(rows, data, normalise):
     block(0, len(rows))
     return
   step = max(1, _BLOCK_BYTES // (4 * rows.shape[1]))
-  with concurrent.futures.ThreadPoolExecutor(_THREADS) as pool:
-    for done in [pool.submit(block, lo, min(lo + step, len(rows))) for lo in range(0, len(rows), step)]:
-      done.result()
+  starts = collections.deque(range(0, len(rows), step))
+  caller = threading.current_thread()
+
+  def blocks():
+    try:
+      if before and threading.current_thread() is caller:
+        before()
+    finally:
+      while starts:
+        try:
+          lo = starts.popleft()
+        except IndexError:
+          break
+        block(lo, min(lo + step, len(rows)))
+
+  _run_beside(blocks, _THREADS)
 
 
 def normalize_rows(x):
@@ -97,13 +139,10 @@ class CuHNSW:
       if not self.opt.nrz and data.dtype == np.float32 and rows.nbytes >= _SHARED_ROWS_BYTES:
         # the device gets the caller's rows as they are, while the copy is made
         self.logger.info("data shape: %d x %d", *rows.shape)
-        with concurrent.futures.ThreadPoolExecutor(1) as beside:
-          copied = beside.submit(_fill_rows, rows, data, False)
-          try:
-            self.obj.set_data(data)
-          finally:
-            copied.result()
-            self.data = rows
+        try:
+          _fill_rows(rows, data, False, before=lambda: self.obj.set_data(data))
+        finally:
+          self.data = rows
       else:
         _fill_rows(rows, data, self.opt.nrz)
         self.data = rows  # (values that do not convert leave everything as it was)

@@ -7,6 +7,7 @@ import os
 import re
 import sys
 import tempfile
+import threading
 
 import numpy as np
 import pytest
@@ -259,6 +260,37 @@ def test_rows_that_the_engine_refuses_are_a_whole_copy(n):
   with pytest.raises(RuntimeError, match="refused"):
     index.set_data(np.ones((n, 50), np.float32))
   assert (index.data == 1).all()
+
+
+@pytest.mark.parametrize("n", [5, 50_000])
+def test_a_caller_that_wants_an_error_for_a_row_of_zeros_gets_it(n):
+  rows = np.ones((n, 50), np.float32)
+  rows[n - 1] = 0
+  index = _Engine()(dist_type="dot", nrz=True)
+  with np.errstate(invalid="raise"), pytest.raises(FloatingPointError):
+    index.set_data(rows)
+  with np.errstate(invalid="ignore"):
+    index.set_data(rows)
+  assert np.isnan(index.data[n - 1]).all() and not np.isnan(index.data[:n - 1]).any()
+
+
+@pytest.mark.parametrize("left", [0, 1, 3])
+@pytest.mark.parametrize("nrz", [False, True])
+def test_set_data_at_the_limit_of_threads(monkeypatch, left, nrz):
+  start = threading.Thread.start
+  started = []
+
+  def limited(thread):
+    if len(started) == left:
+      raise RuntimeError("can't start new thread")
+    started.append(thread)
+    start(thread)
+
+  monkeypatch.setattr(threading.Thread, "start", limited)
+  index = _Engine()(dist_type="dot", nrz=nrz)
+  index.set_data(np.ones((50_000, 64), np.float32))
+  want = np.float32(1) / np.float32(8) if nrz else 1
+  assert (index.data == want).all() and (index.obj.rows == want).all() and not any(t.is_alive() for t in started)
 
 
 def test_benchmark_arithmetic():
