@@ -1257,23 +1257,45 @@ int Engine::LoadIndex(const char* path) {
   levels_h_.assign((size_t)n, 0);
   std::vector<int> rowsU;
   const long long lists_at = (long long)sizeof(h) + n * (long long)rec;
-  std::vector<unsigned char> lists((size_t)(fsize - lists_at));
-  if (!ReadRecords(fd, lists.data(), 1, (long long)lists.size(), lists_at, [](long long, long long) {}))
-    return Fail(kIoError, "index file: short read");
-  size_t pos = 0;
+  // through a buffer of bounded size, filled by several threads (a file may be longer than its lists)
+  std::vector<unsigned char> piece((size_t)std::min<long long>(fsize - lists_at, 4 << 20));
+  long long next = lists_at;  // first byte of the file that has not been read
+  size_t pos = 0, end = 0;    // the part of the buffer that has not been taken
+  bool unreadable = false;
+  // the next bytes, at most a node's lists (17 KB); null: the file ends before them
+  const auto take = [&](size_t bytes) -> const unsigned char* {
+    if (end - pos < bytes) {
+      std::memmove(piece.data(), piece.data() + pos, end - pos);
+      end -= pos;
+      pos = 0;
+      const long long more = std::min<long long>((long long)(piece.size() - end), fsize - next);
+      if ((long long)end + more < (long long)bytes) return nullptr;
+      if (!ReadRecords(fd, piece.data() + end, 1, more, next, [](long long, long long) {})) {
+        unreadable = true;
+        return nullptr;
+      }
+      end += (size_t)more;
+      next += more;
+    }
+    const unsigned char* at = piece.data() + pos;
+    pos += bytes;
+    return at;
+  };
+  const auto ended = [&] {
+    return Fail(kIoError, unreadable ? "index file: short read" : "index file: truncated link lists");
+  };
   for (long long i = 0; i < n; ++i) {
     uint32_t nbytes;
-    if (lists.size() - pos < 4) return Fail(kIoError, "index file: truncated link lists");
-    std::memcpy(&nbytes, lists.data() + pos, 4);
-    pos += 4;
+    const unsigned char* size = take(4);
+    if (!size) return ended();
+    std::memcpy(&nbytes, size, 4);
     if (nbytes % per_link || nbytes / per_link > 64) return Fail(kParseError, "index file: bad link list size");
     const int lv = (int)(nbytes / per_link);
     if (lv > h.maxlevel) return Fail(kParseError, "index file: a node lies above the file's top level");
     levels_h_[(size_t)i] = lv;
     if (!nbytes) continue;
-    if (lists.size() - pos < nbytes) return Fail(kIoError, "index file: truncated link lists");
-    const unsigned char* list = lists.data() + pos;
-    pos += nbytes;
+    const unsigned char* list = take(nbytes);
+    if (!list) return ended();
     for (int l = 0; l < lv; ++l) {
       const unsigned char* o = list + per_link * (size_t)l;
       uint32_t deg;

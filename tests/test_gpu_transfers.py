@@ -127,6 +127,32 @@ def test_an_index_saved_into_a_pipe_is_the_file_byte_for_byte(tmp_path):
     assert got.result() == open(path, "rb").read()
 
 
+def test_what_trails_an_index_in_its_file_is_not_read(tmp_path):
+  """Link lists of several pieces of 4 MB, and a file with a hole of 6 GB behind them; cut within the lists it is
+  refused."""
+  rng = np.random.default_rng(3)
+  n = 70_000
+  eng = CuHNSW(engine_options(dict(dist_type="l2", max_m=32, max_m0=32, ef_construction=8, batch_max=4096)))
+  eng.set_data(rng.integers(-8, 9, (n, 3)).astype(np.float32))
+  eng.obj.set_random_levels((np.arange(n) % 2).astype(np.int32))
+  eng.obj.build_graph()
+  path = str(tmp_path / "x.index")
+  eng.save_index(path)
+  size, want = os.path.getsize(path), eng.obj.get_graph()
+  assert size - 96 - n * (4 * 32 + 4 * 3 + 12) > (4 << 20)
+  os.truncate(path, size + (6 << 30))
+  other = CuHNSW(engine_options(dict(dist_type="l2")))
+  before = resource.getrusage(resource.RUSAGE_SELF).ru_maxrss
+  other.load_index(path)
+  assert resource.getrusage(resource.RUSAGE_SELF).ru_maxrss - before < (1 << 20)  # kB
+  for a, b in zip(other.obj.get_graph(), want):
+    assert (a == b).all()
+  for cut in (1, (4 << 20) + 5):
+    os.truncate(path, size - cut)
+    with pytest.raises(RuntimeError, match="truncated"):
+      other.load_index(path)
+
+
 @pytest.mark.parametrize("rows,d", [(1, 3), (40_000, 50), (42_000, 50), (70_001, 33)])
 def test_set_data_copies_and_normalises_like_one_thread(rows, d):
   """Below and above the size from which several threads share the work; a second corpus over the first."""
