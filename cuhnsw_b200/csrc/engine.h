@@ -71,10 +71,10 @@ class DevBuf {
     p_ = nullptr;
     n_ = room_ = 0;
   }
-  // n elements of undefined content; what is there already is used again unless most of it would lie idle (handing 100
-  // MB back to the driver and taking it again costs 4 ms)
+  // n elements of undefined content; what is there already is used again if little of it would lie idle, an eighth or 64
+  // MB at the most (handing 100 MB back to the driver and taking it again costs 4 ms)
   cudaError_t alloc(size_t n) {
-    if (n > 0 && n <= room_ && room_ / 2 <= n) {
+    if (n > 0 && n <= room_ && room_ - n <= room_ / 8 && (room_ - n) * sizeof(T) <= (64u << 20)) {
       n_ = n;
       return cudaSuccess;
     }

@@ -153,6 +153,22 @@ def test_what_trails_an_index_in_its_file_is_not_read(tmp_path):
       other.load_index(path)
 
 
+def test_a_smaller_corpus_hands_device_memory_back():
+  import torch
+  eng = CuHNSW(engine_options(dict(dist_type="l2")))
+  rows = np.zeros((500_000, 104), np.float32)
+  eng.set_data(rows)
+  torch.cuda.synchronize()
+  held = 500_000  # rows there is room for
+  for n, room in ((500_000, 500_000), (300_000, 300_000), (280_000, 300_000), (240_000, 240_000)):
+    before = torch.cuda.mem_get_info()[0]
+    eng.set_data(rows[:n])
+    torch.cuda.synchronize()
+    given = torch.cuda.mem_get_info()[0] - before
+    assert abs(given - (held - room) * 416) <= (4 << 20), (n, given)
+    held = room
+
+
 @pytest.mark.parametrize("rows,d", [(1, 3), (40_000, 50), (42_000, 50), (70_001, 33)])
 def test_set_data_copies_and_normalises_like_one_thread(rows, d):
   """Below and above the size from which several threads share the work; a second corpus over the first."""
