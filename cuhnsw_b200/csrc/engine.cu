@@ -373,7 +373,7 @@ int Engine::AllocRows(long long num_data, int num_dims) {
   has_data_ = has_levels_ = has_graph_ = labelled_ = false;
   labels_h_.clear();
   labels_d_.release();
-  CU(vec_.alloc(((size_t)n_ * vstride_ * (rows16_ ? 2 : 4) + 3) / 4));
+  CU(Alloc(vec_, ((size_t)n_ * vstride_ * (rows16_ ? 2 : 4) + 3) / 4));
   return kOk;
 }
 
@@ -388,10 +388,10 @@ int Engine::AllocGraph() {
     if (acc > (1ll << 30)) return Fail(kUnsupported, "too many upper-layer rows");
   }
   total_upper_ = acc;
-  CU(rows0_.alloc((size_t)n_ * stride0_));
-  CU(rowsU_.alloc((size_t)std::max<long long>(total_upper_, 1) * strideU_));
-  CU(levels_d_.alloc((size_t)std::max<long long>(n_, 1)));
-  CU(upper_base_d_.alloc((size_t)std::max<long long>(n_, 1)));
+  CU(Alloc(rows0_, (size_t)n_ * stride0_));
+  CU(Alloc(rowsU_, (size_t)std::max<long long>(total_upper_, 1) * strideU_));
+  CU(Alloc(levels_d_, (size_t)std::max<long long>(n_, 1)));
+  CU(Alloc(upper_base_d_, (size_t)std::max<long long>(n_, 1)));
   CU(launch_fill_i32(rows0_.get(), n_ * stride0_, -1, stream_));
   CU(launch_fill_i32(rowsU_.get(), std::max<long long>(total_upper_, 1) * strideU_, -1, stream_));
   if (n_ > 0) {
@@ -522,7 +522,7 @@ int Engine::BuildGraph() {
   const size_t at_vals = part(items * 8), at_vals2 = part(items * 8);
   const size_t at_tmp = part(tmp_bytes + 256);
   const size_t at_nodes = part(std::max<size_t>(max_upper_nodes, 1) * 4);
-  CU(build_scratch_.alloc(total));
+  CU(Alloc(build_scratch_, total));
   unsigned char* const base = build_scratch_.get();
   // on every way out
   struct GiveBack {
@@ -693,8 +693,8 @@ int Engine::PrepareSchedule(long long nq, SearchLane* lane, SearchSchedule* s) {
   if (nq > lane->capacity) {
     lane->capacity = 0;  // (what there is goes back first)
     const long long cap = std::max<long long>(nq, 1024);
-    CU(lane->sched.reserve((size_t)cap * (large ? 6 : 4)));
-    if (large) CU(lane->sched_tmp.reserve(search_schedule_tmp_bytes(cap)));
+    CU(Reserve(lane->sched, (size_t)cap * (large ? 6 : 4)));
+    if (large) CU(Reserve(lane->sched_tmp, search_schedule_tmp_bytes(cap)));
     lane->capacity = cap;
   }
   unsigned* base = lane->sched.get();
@@ -892,7 +892,7 @@ Engine::LaneIo Engine::IoOf(long long nq, int topk) const {
   return io;
 }
 int Engine::ReserveIo(SearchLane* lane, const LaneIo& io) {
-  CU(lane->io.reserve(io.bytes));
+  CU(Reserve(lane->io, io.bytes));
   return kOk;
 }
 
@@ -1030,6 +1030,19 @@ int Engine::GetGraph(int* levels, int* rows0, int* rows_upper) {
 // ---------------------------------------------------------------------------
 // hnswlib-compatible file (layout: cpp/src/cuhnsw_base.cu:159-247 / 250-365)
 // ---------------------------------------------------------------------------
+// (as Alloc, which must not give back the arrays that are being made)
+int Engine::ReserveRecords(int pieces, size_t words) {
+  cudaError_t e = cudaSuccess;
+  for (int turn = 0; turn < 2; ++turn) {
+    e = cudaSuccess;
+    for (int i = 0; i < pieces && e == cudaSuccess; ++i) e = records_[i].reserve(words);
+    if (e != cudaErrorMemoryAllocation) break;
+    cudaGetLastError();
+    build_scratch_.release();
+  }
+  return e == cudaSuccess ? kOk : FailCuda(e, "the buffers of an index file");
+}
+
 int Engine::SaveIndex(const char* path) {
   if (!has_graph_) return Fail(kBadState, "no graph to save");
   if (!path) return Fail(kInvalidArgument, "null path");
@@ -1085,7 +1098,7 @@ int Engine::SaveIndex(const char* path) {
   std::vector<unsigned char> pageable;  // one record above the size of a staging buffer, or no page-locked memory
   if (rec > HostStage::kBufferBytes || !pipe.Open(std::max<long long>(pieces, 1))) pageable.resize(chunk_rows * rec);
   const int depth = pageable.empty() ? pipe.depth() : 1;
-  for (int i = 0; i < depth; ++i) CU(records_[i].reserve(chunk_rows * (size_t)rec_words));
+  if ((rc = ReserveRecords(depth, chunk_rows * (size_t)rec_words)) != kOk) return rc;
   auto host = [&](long long i) { return pageable.empty() ? pipe.At(i).host() : pageable.data(); };
   for (long long i = 0; i < pieces + depth - 1 && ok; ++i) {
     if (i < pieces) {
@@ -1200,8 +1213,8 @@ int Engine::LoadIndex(const char* path) {
   if (rc) return rc;
   stride0_ = round_up(m0, 8);
   strideU_ = round_up(m, 8);
-  CU(rows0_.alloc((size_t)std::max<long long>(n, 1) * stride0_));
-  CU(labels_d_.alloc((size_t)std::max<long long>(n, 1)));
+  CU(Alloc(rows0_, (size_t)std::max<long long>(n, 1) * stride0_));
+  CU(Alloc(labels_d_, (size_t)std::max<long long>(n, 1)));
   std::vector<long long> labels((size_t)n);
   const long long rec_words = (long long)(rec / 4);
   {
@@ -1214,7 +1227,7 @@ int Engine::LoadIndex(const char* path) {
     std::vector<unsigned char> pageable;  // one record above the size of a staging buffer, or no page-locked memory
     if (rec > HostStage::kBufferBytes || !pipe.Open(std::max<long long>(pieces, 1))) pageable.resize(rows_in_chunk * rec);
     const int depth = pageable.empty() ? pipe.depth() : 1;
-    for (int i = 0; i < depth; ++i) CU(records_[i].reserve(rows_in_chunk * (size_t)rec_words));
+    if ((rc = ReserveRecords(depth, rows_in_chunk * (size_t)rec_words)) != kOk) return rc;
     CU(bad.alloc(1));
     CU(cudaMemsetAsync(bad.get(), 0xff, sizeof(unsigned long long), stream_));
     for (long long i = 0; i < pieces; ++i) {
@@ -1334,9 +1347,9 @@ int Engine::LoadIndex(const char* path) {
     if (acc > (1ll << 30)) return Fail(kUnsupported, "too many upper-layer rows");
   }
   total_upper_ = acc;
-  CU(rowsU_.alloc((size_t)std::max<long long>(total_upper_, 1) * strideU_));
-  CU(levels_d_.alloc((size_t)std::max<long long>(n, 1)));
-  CU(upper_base_d_.alloc((size_t)std::max<long long>(n, 1)));
+  CU(Alloc(rowsU_, (size_t)std::max<long long>(total_upper_, 1) * strideU_));
+  CU(Alloc(levels_d_, (size_t)std::max<long long>(n, 1)));
+  CU(Alloc(upper_base_d_, (size_t)std::max<long long>(n, 1)));
   if (total_upper_ > 0)
     CU(cudaMemcpy(rowsU_.get(), rowsU.data(), (size_t)total_upper_ * strideU_ * sizeof(int), cudaMemcpyHostToDevice));
   else
@@ -1379,17 +1392,17 @@ int Engine::CloneFrom(const Engine& src) {
     return bytes ? cudaMemcpyPeer(dst, device_, from, src.device_, bytes) : cudaSuccess;
   };
   const size_t one = (size_t)std::max<long long>(n_, 1);
-  CU(rows0_.alloc(one * stride0_));
-  CU(rowsU_.alloc((size_t)std::max<long long>(total_upper_, 1) * strideU_));
-  CU(levels_d_.alloc(one));
-  CU(upper_base_d_.alloc(one));
+  CU(Alloc(rows0_, one * stride0_));
+  CU(Alloc(rowsU_, (size_t)std::max<long long>(total_upper_, 1) * strideU_));
+  CU(Alloc(levels_d_, one));
+  CU(Alloc(upper_base_d_, one));
   CU(copy(vec_.get(), src.vec_.get(), vec_.size() * sizeof(float)));
   CU(copy(rows0_.get(), src.rows0_.get(), rows0_.size() * sizeof(int)));
   CU(copy(rowsU_.get(), src.rowsU_.get(), rowsU_.size() * sizeof(int)));
   CU(copy(levels_d_.get(), src.levels_d_.get(), levels_d_.size() * sizeof(int)));
   CU(copy(upper_base_d_.get(), src.upper_base_d_.get(), upper_base_d_.size() * sizeof(int)));
   if (src.labelled_) {
-    CU(labels_d_.alloc(one));
+    CU(Alloc(labels_d_, one));
     CU(copy(labels_d_.get(), src.labels_d_.get(), labels_d_.size() * sizeof(int)));
   }
   CU(cudaDeviceSynchronize());

@@ -148,6 +148,22 @@ class Engine {
   int FailCuda(cudaError_t e, const char* what);
   int EnsureDevice();
   int AllocRows(long long num_data, int num_dims);
+  // n elements as by buf.alloc; when the device is out of memory, once more without what the engine keeps between calls
+  // only to save time
+  template <class T>
+  cudaError_t Alloc(DevBuf<T>& buf, size_t n) {
+    cudaError_t e = buf.alloc(n);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    build_scratch_.release();
+    for (DevBuf<unsigned>& r : records_) r.release();
+    return buf.alloc(n);
+  }
+  template <class T>
+  cudaError_t Reserve(DevBuf<T>& buf, size_t n) {
+    return n <= buf.size() ? cudaSuccess : Alloc(buf, n);
+  }
+  int ReserveRecords(int pieces, size_t words);
   int UploadRows(const float* data, int num_dims);
   int DownloadRows(int* dst, const int* src, int stride, int width, long long count);
   int AllocGraph();

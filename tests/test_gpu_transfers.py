@@ -169,6 +169,25 @@ def test_a_smaller_corpus_hands_device_memory_back():
     held = room
 
 
+def test_what_a_build_keeps_goes_back_when_the_device_is_out_of_memory():
+  """The scratch of the second build stays for a third; rows that fit the device only without it must still fit."""
+  import torch
+  eng, base, _ = _index(400_000, 8, max_m=12, max_m0=24)
+  eng.build()
+  graph = eng.obj.get_graph()
+  torch.cuda.synchronize()
+  fill = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+  try:
+    eng.set_data(np.tile(base, 4))  # 51 MB, 13 of them in the place of the former rows
+  finally:
+    del fill
+    torch.cuda.empty_cache()
+  eng.set_data(base)
+  eng.build()
+  for a, b in zip(eng.obj.get_graph(), graph):
+    assert (a == b).all()
+
+
 @pytest.mark.parametrize("rows,d", [(1, 3), (40_000, 50), (42_000, 50), (70_001, 33)])
 def test_set_data_copies_and_normalises_like_one_thread(rows, d):
   """Below and above the size from which several threads share the work; a second corpus over the first."""
