@@ -760,7 +760,7 @@ int Engine::SearchGraphStaged(const float* q, long long nq, int topk, int ef, in
   int nslots = 0;
   for (; nslots < (int)std::min<long long>(pieces, kPieces); ++nslots) {
     Piece& s = slots[nslots];
-    if (!s.buffer.Open(nslots == 0)) break;
+    if (!s.buffer.Open()) break;
     if (pieces == 1) {
       s.stream = stream_;
     } else {

@@ -62,35 +62,30 @@ class HostStage {
     for (std::thread& t : threads) t.join();
   }
 
-  // A buffer, or nullptr: page-locked memory cannot be had, or, without `wait`, all buffers are in use.  A thread that
-  // holds a buffer asks for more without waiting, so that threads never wait for each other in a circle.
-  void* Acquire(bool wait) {
-    std::unique_lock<std::mutex> lock(mu_);
-    for (;;) {
+  // A buffer, or nullptr: page-locked memory cannot be had, or all buffers are in use.  Nobody waits for one: the others
+  // may be held for as long as somebody's file takes to write, and every transfer has another way.
+  void* Acquire() {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
       if (!free_.empty()) {
         void* p = free_.back();
         free_.pop_back();
         return p;
       }
-      if (made_ < kMaxBuffers) break;
-      if (!wait) return nullptr;
-      room_.wait(lock);
+      if (made_ >= kMaxBuffers) return nullptr;
+      ++made_;
     }
-    ++made_;
-    lock.unlock();
     void* p = nullptr;
     if (cudaHostAlloc(&p, kBufferBytes, cudaHostAllocPortable) == cudaSuccess) return p;
     cudaGetLastError();
-    lock.lock();
+    std::lock_guard<std::mutex> lock(mu_);
     --made_;
-    room_.notify_one();
     return nullptr;
   }
   void Release(void* p) {
     if (!p) return;
     std::lock_guard<std::mutex> lock(mu_);
     free_.push_back(p);
-    room_.notify_one();
   }
 
   // f(0) ... f(n - 1) on the calling thread and the pool's; returns when all are done.  f must not throw.
@@ -173,13 +168,12 @@ class HostStage {
     new (&threads_) std::vector<std::thread>;
     new (&jobs_) std::deque<std::shared_ptr<Job>>;
     new (&work_) std::condition_variable;
-    new (&room_) std::condition_variable;
     ++generation_;
     mu_.unlock();
   }
 
   std::mutex mu_;
-  std::condition_variable work_, room_;
+  std::condition_variable work_;
   std::vector<void*> free_;
   std::vector<std::thread> threads_;
   std::deque<std::shared_ptr<Job>> jobs_;
@@ -190,7 +184,7 @@ class HostStage {
 // A buffer of the stage for the lifetime of a scope.
 class StageBuffer {
  public:
-  explicit StageBuffer(bool wait) : p_(HostStage::Get().Acquire(wait)) {}
+  StageBuffer() : p_(HostStage::Get().Acquire()) {}
   ~StageBuffer() { HostStage::Get().Release(p_); }
   StageBuffer(const StageBuffer&) = delete;
   StageBuffer& operator=(const StageBuffer&) = delete;
@@ -209,8 +203,8 @@ class StreamBuffer {
   StreamBuffer& operator=(const StreamBuffer&) = delete;
   ~StreamBuffer() { Wait(); }
   // false: none to be had
-  bool Open(bool wait) {
-    buffer_.reset(new StageBuffer(wait));
+  bool Open() {
+    buffer_.reset(new StageBuffer);
     if (!buffer_->get()) buffer_.reset();
     return buffer_ != nullptr;
   }
@@ -260,7 +254,7 @@ class Pipeline {
   bool Open(long long pieces) {
     for (; depth_ < kDepth && depth_ < pieces; ++depth_) {
       Slot& s = slots_[depth_];
-      s.buffer_.reset(new StageBuffer(depth_ == 0));
+      s.buffer_.reset(new StageBuffer);
       if (!s.buffer_->get() || cudaEventCreateWithFlags(&s.done_, cudaEventDisableTiming) != cudaSuccess) {
         s.buffer_.reset();
         cudaGetLastError();

@@ -44,7 +44,7 @@ using hnsw::HostStage;
 
 cudaError_t cudaStreamSynchronize(cudaStream_t) {
   ++g_waits;
-  void* p = HostStage::Get().Acquire(false);
+  void* p = HostStage::Get().Acquire();
   if (p) g_held = false;
   HostStage::Get().Release(p);
   return cudaSuccess;
@@ -90,10 +90,10 @@ void Users() {
 void Unwinding() {
   HostStage::Get().AddUser();
   void* others[HostStage::kMaxBuffers - 1];
-  for (void*& p : others) EXPECT((p = HostStage::Get().Acquire(false)) != nullptr);
+  for (void*& p : others) EXPECT((p = HostStage::Get().Acquire()) != nullptr);
   try {
     hnsw::StreamBuffer b;
-    EXPECT(b.Open(false));
+    EXPECT(b.Open());
     b.Use(nullptr);
     throw std::bad_alloc();
   } catch (const std::bad_alloc&) {
@@ -101,8 +101,8 @@ void Unwinding() {
   EXPECT(g_waits == 1 && g_held);
   {
     hnsw::StreamBuffer b;
-    EXPECT(b.Open(false));
-    EXPECT(!hnsw::StreamBuffer().Open(false));
+    EXPECT(b.Open());
+    EXPECT(!hnsw::StreamBuffer().Open());
     b.Use(nullptr);
     EXPECT(b.Wait() == cudaSuccess && b.Wait() == cudaSuccess);
   }

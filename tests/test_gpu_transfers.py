@@ -4,6 +4,7 @@ index files."""
 import concurrent.futures
 import os
 import resource
+import time
 
 import numpy as np
 import pytest
@@ -125,6 +126,42 @@ def test_an_index_saved_into_a_pipe_is_the_file_byte_for_byte(tmp_path):
     got = pool.submit(lambda: open(pipe, "rb").read())
     eng.save_index(pipe)
     assert got.result() == open(path, "rb").read()
+
+
+def test_calls_of_other_threads_do_not_wait_for_a_file_that_is_slow_to_write(tmp_path):
+  """Three saves into pipes that nobody reads yet hold all page-locked buffers; everything else takes another way."""
+  slow = [_index(150_000, 50)[0] for _ in range(3)]  # 37 MB, five pieces
+  eng, base, rng = _index(60_000, 50)
+  q = rng.standard_normal((40_000, 50)).astype(np.float32)
+  path = str(tmp_path / "x.index")
+  eng.save_index(path)
+  want = eng.search_knn(q, 10, 40), eng.obj.get_graph()
+  pipes = [str(tmp_path / f"pipe{i}") for i in range(3)]
+  for p in pipes:
+    os.mkfifo(p)
+  with concurrent.futures.ThreadPoolExecutor(7) as pool:
+    saves = [pool.submit(e.save_index, p) for e, p in zip(slow, pipes)]
+    readers = [open(p, "rb") for p in pipes]  # returns when the save has opened its end
+
+    def everything():
+      time.sleep(1)
+      eng.set_data(base)
+      eng.build()
+      few, many = eng.search_knn(q[:100], 10, 40), eng.search_knn(q, 10, 40)
+      assert (few[0] == want[0][0][:100]).all() and (many[0] == want[0][0]).all()
+      assert all((a == b).all() for a, b in zip(eng.obj.get_graph(), want[1]))
+      eng.save_index(path + "2")
+      eng.load_index(path + "2")
+
+    try:
+      pool.submit(everything).result(timeout=30)
+      assert not any(s.done() for s in saves)
+    finally:
+      read = [pool.submit(r.read) for r in readers]
+      for r, s in zip(read, saves):
+        s.result()
+        assert len(r.result()) > 4 * PIECE
+  assert open(path, "rb").read() == open(path + "2", "rb").read()
 
 
 def test_what_trails_an_index_in_its_file_is_not_read(tmp_path):
