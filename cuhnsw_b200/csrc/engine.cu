@@ -409,24 +409,23 @@ int Engine::AllocGraph() {
 int Engine::SetRandomLevels(const int* levels) {
   if (!has_data_) return Fail(kBadState, "set_data() must be called first");
   if (!levels && n_ > 0) return Fail(kInvalidArgument, "null levels");
+  for (long long i = 0; i < n_; ++i)  // (a refused call leaves the graph that is there as it was)
+    if (levels[i] < 0 || levels[i] > 64) return Fail(kInvalidArgument, "levels must lie in 0..64");
   int rc = EnsureDevice();
   if (rc) return rc;
   // searches still running on other streams read the graph whose arrays are written over from here on
   if ((rc = WaitForSearches()) != kOk) return rc;
-  levels_h_.assign((size_t)n_, 0);
+  has_graph_ = has_levels_ = false;
+  levels_h_.assign(levels, levels + n_);
   max_level_ = 0;
   enter_point_ = 0;
-  for (long long i = 0; i < n_; ++i) {
-    if (levels[i] < 0 || levels[i] > 64) return Fail(kInvalidArgument, "levels must lie in 0..64");
-    levels_h_[i] = levels[i];
+  for (long long i = 0; i < n_; ++i)
     if (levels[i] > max_level_) {
       max_level_ = levels[i];
       enter_point_ = (int)i;
     }
-  }
   if ((rc = AllocGraph()) != kOk) return rc;
   has_levels_ = true;
-  has_graph_ = false;
   Log(3, "max level: %d, enter point: %d", max_level_, enter_point_);
   return kOk;
 }

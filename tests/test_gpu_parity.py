@@ -338,6 +338,21 @@ def _rounded(x, row_dtype="f16"):
   return x.astype(np.float16).astype(np.float32)
 
 
+def test_refused_levels_leave_the_graph_as_it_was():
+  base, q, opt = small_workload("angular_toy", 3000, 50)
+  eng = CuHNSW(engine_options(opt))
+  eng.set_data(base)
+  eng.build()
+  want, levels = eng.search_knn(q, 10, 40), eng.obj.get_graph()[0]
+  for wrong in (-1, 65):
+    bad = levels.copy()
+    bad[7], bad[2999] = 60, wrong
+    with pytest.raises(RuntimeError, match="levels must lie"):
+      eng.obj.set_random_levels(bad)
+    got = eng.search_knn(q, 10, 40)
+    assert (got[0] == want[0]).all() and (eng.obj.get_graph()[0] == levels).all()
+
+
 def test_levels_for_fewer_rows_than_there_are_are_refused():
   eng = CuHNSW(engine_options(dict(dist_type="l2")))
   eng.set_data(np.arange(300, dtype=np.float32).reshape(100, 3))
