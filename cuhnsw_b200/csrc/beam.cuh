@@ -109,8 +109,7 @@ struct VisitedTable {
 };
 
 // Per-warp shared-memory state.  Loop bounds and branch conditions come from ballots, shuffles and reductions rather than
-// from loads, so that the compiler knows them to be the same in every lane: a warp-wide operation under a condition it
-// cannot be sure of costs a divergence check and a register move each (27 of 374 instructions per expansion).
+// from loads, so that the compiler knows them to be the same in every lane (figures in smem.cuh).
 struct WarpList : VisitedTable {
   unsigned keys;  // shared-memory address of `cap` 64-bit keys, ascending (distance, id)
   unsigned spos;  // 32 words of scratch

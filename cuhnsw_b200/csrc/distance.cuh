@@ -363,7 +363,7 @@ struct Pick {
   using D128 = DistSmall<4, Row>;
   using Wide = DistLargeT<4, 8, Row>;
   using WideDeep = DistLargeT<8, 4, Row>;
-  // a warp of a four-warp CTA per query sees one or two rows of most requests: two rows, eight columns of
+  // one CTA per query: each of its four or eight warps gets one to five rows of a round.  Two rows, eight columns of
   // each in flight (a 3840-byte row in one round trip) measured 8 % faster there than four rows of four
   using Team = DistLargeT<8, 8, Row, 2>;
 };

@@ -453,12 +453,13 @@ int Engine::ResolveVsize(int cap, long long nq, int* vsize) const {
   if (opt_.visited_table_size > 0) {
     v = std::min(32768, std::max(64, next_pow2(opt_.visited_table_size)));
   } else {
-    // Largest table that still lets the kernel keep its target number of warps resident per SM
+    // Largest table that still lets the warp kernel keep its target number of warps resident per SM
     // (the walk is latency bound: resident warps matter more than a few repeated evaluations),
-    // but never below ~4 entries per list slot, where repeats explode.
-    // Wide rows and few queries: the kernel chosen there keeps 4 CTAs per SM resident whatever the table
-    // size, and a repeated evaluation re-reads kilobytes.  Measured on 1M x 960, 1000 queries, ef 500:
-    // 3576 evaluations per query with 2048 entries, 2099 with 16384.
+    // but never below ~4 entries per list slot, where repeats explode.  Wide rows and few queries: few warps
+    // are resident whatever the table's size, and a repeated evaluation re-reads kilobytes (1 M x 960, 1000
+    // queries, ef 500: 3576 evaluations per query with 2048 entries, 2099 with 16384).
+    // One CTA per query: its launcher sizes the table (walk_table_entries); what is found here only says
+    // that ef fits.
     const int kind = nq < 0 ? kSearchWarp
                             : search_kernel_kind(d_, cap, nq, opt_.search_team, opt_.reverse_cand ? 1 : 0, sm_count_);
     const int warps = d_ <= 128 ? 32 : kind == kSearchWarpDeep ? 8 : 16;

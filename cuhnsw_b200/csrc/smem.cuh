@@ -1,6 +1,6 @@
-// Shared memory by 32-bit address.  A generic pointer into shared memory that is kept in a struct makes the compiler
-// build the shared window's base again at every access (a special-register read, a move and an add, 10 % of the
-// instructions of a walk); an address taken once is a register plus an immediate offset.
+// Shared memory by 32-bit address, taken once, instead of generic pointers kept in structs.  Counters of the warp kernel
+// (20 000 queries, 1.18 M x 50, ef 200): 374 warp instructions per expansion with pointers, 325 with addresses, conditions
+// that are the same in every lane (beam.cuh) and the descent in a kernel of its own (search.cu).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -30,7 +30,7 @@ namespace hnsw {
 // flag in the lowest bit keys compare as they stand.  A group of up to 32 keys is merged at once: places by binary
 // search (the same number of steps in every lane), ranks among the group, then one bit per place of the new list
 // says whether it holds a newcomer; the old key of a place is the one that many places further down, so that the list
-// moves 32 keys per 11 instructions whatever the group's size.
+// moves 32 keys at a time whatever the group's size.
 struct KeyList {
   unsigned keys;   // shared-memory address of cap + 1 keys; those from `size` on read ~0
   unsigned marks;  // a bit per place
