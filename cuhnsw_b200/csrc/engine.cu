@@ -461,7 +461,8 @@ int Engine::ResolveVsize(int cap, long long nq, int* vsize) const {
     // One CTA per query: its launcher sizes the table (walk_table_entries); what is found here only says
     // that ef fits.
     const int kind = nq < 0 ? kSearchWarp
-                            : search_kernel_kind(d_, cap, nq, opt_.search_team, opt_.reverse_cand ? 1 : 0, sm_count_);
+                            : search_kernel_kind(d_, rows16_, stride0_, cap, nq, opt_.search_team,
+                                                 opt_.reverse_cand ? 1 : 0, sm_count_);
     const int warps = d_ <= 128 ? 32 : kind == kSearchWarpDeep ? 8 : 16;
     const int top = kind == kSearchWarpDeep ? 8192 : 4096;
     const long long budget = (long long)smem_optin_ / warps - 640;

@@ -79,7 +79,7 @@ cudaError_t launch_search(const SearchParams& p, int sm_count, cudaStream_t stre
 size_t search_smem_per_cta(int d, int ef, int vsize, long long n);
 // which search kernel a batch gets: one warp per query (narrow rows; wide rows; wide rows, few queries) or one CTA
 enum SearchKernelKind { kSearchWarpSmall = 0, kSearchWarp = 1, kSearchWarpDeep = 2, kSearchTeam = 3 };
-int search_kernel_kind(int d, int ef, long long nq, int team, int reverse_cand, int sm_count);
+int search_kernel_kind(int d, int rows16, int links, int ef, long long nq, int team, int reverse_cand, int sm_count);
 // one CTA per query (search_walk.cuh), by row type
 cudaError_t launch_search_walk_f32(const SearchParams& p, int sm_count, cudaStream_t stream,
                                    const SearchSchedule* sched);

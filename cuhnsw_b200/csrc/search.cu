@@ -255,23 +255,46 @@ size_t search_smem_per_cta(int d, int ef, int vsize, long long n) {
   return per_warp * kWarpsPerCta;
 }
 
-// One CTA per query while that is the faster way: up to so many queries per SM.  Narrow rows: the longer the walks, the
-// longer a launch waits for its last ones (ef 50: 14 queries per SM; in between in proportion; ef 170 and more: 36).  Wide
-// rows: 10, very wide ones 14.  Measured, one warp / one CTA per query, ms: 300 000 x 96 f16, 4000 queries, ef 50: 0.33 /
-// 0.36, ef 128: 0.76 / 0.64, ef 400: 2.13 / 1.60, 6000: 0.39 / 0.49, 0.79 / 0.84, 2.19 / 1.94; 200 000 x 300 f16, ef 100,
-// 1000 queries: 0.75 / 0.53, 2000: 0.73 / 0.74; 150 000 x 960, ef 500, 2000: 3.56 / 3.16, 3000: 4.12 / 4.43.  More figures
-// are in search_walk.cuh.  Expanding the farthest key first knows no next nodes to prepare: always one warp.
-static long long team_limit(int d, int ef, int sm_count) {
-  const int per_sm = d > 512 ? 14 : d > 128 ? 10 : ef * 27 / 128 < 14 ? 14 : ef * 27 / 128 > 36 ? 36 : ef * 27 / 128;
-  return (long long)sm_count * per_sm;
+// One CTA per query while that is the faster way: up to so many queries per SM, which no rule on sizes hits for all data.
+// Measured with tables of 200 000 to 500 000 rows of 16 to 48 links, time of one CTA / one warp per query (device buffers,
+// medians of five launches):
+//   short walks end before rounds and, from a wave on, the entry kernel and the sort pay: 300 000 x 50, 6 and 8 queries per
+//   SM: ef 10 0.87 and 1.38, ef 30 0.81 and 1.07, ef 50 0.73 and 0.90; fp32 rows of 65 values and more, whose evaluations
+//   four warps share, hold out longer: 300 000 x 128, 12 and 20: ef 20 0.77 and 1.04, ef 50 0.61 and 0.86, but with 16
+//   links x 96, 20 per SM, 1.29 at ef 40.
+//   walks of 200 to 400: 0.5 to 0.95 up to 28 per SM, 0.8 to 1.2 at 36, 0.9 to 1.35 at 44.  Rows of up to 32 values leave the
+//   commit's one warp as the longer part if it has many links to merge: 200 000 x 32 with 32 links, ef 250, 8, 12 and 18 per
+//   SM 0.87 1.10 1.32, with 20 links at 20 per SM 1.4 (300 000 with 16 links, ef 300: 0.70 to 0.87 up to 36).
+//   long lists leave an SM 4 to 8 CTAs, each of which merges on one warp: 300 000 x 128, 14 and 26 per SM: ef 600 0.73 and
+//   1.24, ef 800 0.78 and 1.42, ef 1200 1.07 and 1.29; 24 links x 50, ef 1200: 0.86 and 1.04; ef 1000, 14 and 24 per SM: 20
+//   links x 48 1.08 and 1.41, 32 links x 48 1.01 and 1.31.  Once a list is so long that hardly more warps than CTAs fit
+//   either, CTAs win again: ef 4800 0.65 to 1.0.
+static int narrow_walks_per_sm(int d, int rows16, int links, int ef) {
+  const bool long_rows = d > 64 && !rows16, many_links = links > 24;
+  if (ef >= 4000) return 36;
+  if (ef < 40) return long_rows ? (ef < 16 ? 4 : 14) : 6;
+  if (d <= 32 && links > 16) return std::min({16, std::max(8, ef / 8), 11000 / ef});
+  const int few = d <= 32 ? ef / 5 : std::max(14, ef * 27 / 128);
+  const int many = d <= 64 ? (many_links ? 11000 : 15000) / ef
+                           : long_rows && ef >= 2000 ? 24 : std::max(14, 14000 / ef);
+  return std::min({d <= 64 && many_links ? 30 : 36, few, many});
 }
-// Otherwise one warp per query; for few queries over wide rows with 32 float4 loads in flight instead of 16 (1 M x 960,
-// 1000 queries: 6.0 against 8.5 ms at ef 500).
-int search_kernel_kind(int d, int ef, long long nq, int team, int reverse_cand, int sm_count) {
-  if (!reverse_cand && (team == 1 || (team < 0 && nq <= team_limit(d, ef, sm_count)))) return kSearchTeam;
+// Wide rows: warps keep 16 float4 in flight each and win once 8 to 16 of them fill an SM; when, depends on the data more than
+// on the sizes.  One CTA / one warp per query at 7, 8 and 10 queries per SM: 100 000 x 200: ef 250 1.06 1.19 1.36, ef 400 1.24
+// 1.37 1.57, ef 700 1.39 1.56 1.72, ef 3000 0.80 0.88 1.03; 200 000 x 150: ef 250 0.75 0.86 0.92, ef 400 0.91 0.98 1.14, ef 700
+// 0.80 0.84 0.99.  60 000 x 960 at 10 and 14: ef 50 0.87 1.01, ef 200 0.99 1.20, ef 400 1.06 1.28, ef 1600 0.72 0.91.
+static int wide_walks_per_sm(int d, int ef) {
+  if (d > 512) return ef > 200 && ef < 1200 ? 10 : 14;
+  return ef > 300 && ef < 2000 ? 7 : 10;
+}
+// Otherwise one warp per query; for few queries over rows above 512 floats with 32 float4 loads in flight instead of 16
+// (60 000 x 960, 8 and 10 queries per SM: ef 100 0.84 and 0.89, ef 400 0.77 and 1.12).  Expanding the farthest key first
+// knows no next nodes to prepare: always one warp.
+int search_kernel_kind(int d, int rows16, int links, int ef, long long nq, int team, int reverse_cand, int sm_count) {
+  const int walks = d <= 128 ? narrow_walks_per_sm(d, rows16, links, ef) : wide_walks_per_sm(d, ef);
+  if (!reverse_cand && (team == 1 || (team < 0 && nq <= (long long)sm_count * walks))) return kSearchTeam;
   if (d <= 128) return kSearchWarpSmall;
-  if (nq <= (long long)sm_count * 10) return kSearchWarpDeep;
-  return kSearchWarp;
+  return d > 512 && nq <= (long long)sm_count * 10 ? kSearchWarpDeep : kSearchWarp;
 }
 
 template <class Row>
@@ -283,14 +306,14 @@ static cudaError_t launch_search_rows(const SearchParams& p, int sm_count, cudaS
   if (d <= 64) return launch_search_t<typename E::D64>(p, sm_count, stream, sched);
   if (d <= 96) return launch_search_t<typename E::D96>(p, sm_count, stream, sched);
   if (d <= 128) return launch_search_t<typename E::D128>(p, sm_count, stream, sched);
-  if (search_kernel_kind(d, p.ef, p.nq, p.team, p.reverse_cand, sm_count) == kSearchWarpDeep)
+  if (search_kernel_kind(d, p.g.rows16, p.g.stride0, p.ef, p.nq, p.team, p.reverse_cand, sm_count) == kSearchWarpDeep)
     return launch_search_t<typename E::WideDeep>(p, sm_count, stream, sched);
   return launch_search_t<typename E::Wide>(p, sm_count, stream, sched);
 }
 
 cudaError_t launch_search(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   if (p.nq <= 0) return cudaSuccess;
-  if (search_kernel_kind(p.g.d, p.ef, p.nq, p.team, p.reverse_cand, sm_count) == kSearchTeam)
+  if (search_kernel_kind(p.g.d, p.g.rows16, p.g.stride0, p.ef, p.nq, p.team, p.reverse_cand, sm_count) == kSearchTeam)
     return p.g.rows16 == kRowsF16    ? launch_search_walk_f16(p, sm_count, stream, sched)
            : p.g.rows16 == kRowsBF16 ? launch_search_walk_bf16(p, sm_count, stream, sched)
                                      : launch_search_walk_f32(p, sm_count, stream, sched);

@@ -120,8 +120,8 @@ int cuhnsw_search_knn_async_on(cuhnsw_handle* h, int32_t replica, void* cuda_str
  *  - The first call on a device looks up the array's device address (a one-time set-up per device); make that
  *    first call before any stream capture is started.
  *  - The CUDA runtime loads a kernel into device memory the first time it is launched.  Which search kernel runs
- *    depends on the row width class (<= 32, 64, 96, 128 floats, wider), row_dtype, reverse_cand, ef_search and
- *    the batch size class; the first call of each combination therefore takes that memory and
+ *    depends on the row width class (<= 32, 64, 96, 128, 512 floats, wider), row_dtype, reverse_cand, max_m0, ef_search
+ *    and the batch size class; the first call of each combination therefore takes that memory and
  *    belongs in the warm-up of a process that later runs with its pool full.
  *  - The array is shared by all handles and calls of the process on that device and keeps the previous call's
  *    contents; the call clears the one word that has to start at zero.  Calls that overlap on the GPU (two

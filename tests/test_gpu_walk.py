@@ -42,11 +42,29 @@ def test_walk_equals_the_oracle(d, max_m0, dist_type, values):
 @pytest.mark.parametrize("d,ef,nq", [(20, 40, 2072), (50, 200, 3996), (50, 200, 5328), (140, 40, 1480),
                                      (600, 120, 592), (600, 120, 2072)])
 def test_batches_on_both_sides_of_a_change_of_kernel(d, ef, nq):
-  """A batch of the largest size of one kernel and one query more (148 SMs), against one warp per query."""
+  """Batches around sizes at which kernel, shape or order of service change, against one warp per query."""
+  _same_as_one_warp_per_query(d, ef, nq)
+
+
+@pytest.mark.parametrize("row_dtype,d,max_m0,ef,per_sm", [
+  ("f32", 20, 16, 10, 6), ("f32", 20, 16, 40, 8), ("f32", 20, 24, 100, 12), ("f32", 20, 32, 1000, 11),
+  ("f32", 50, 16, 100, 21), ("f32", 50, 24, 1500, 10), ("f32", 50, 25, 300, 30), ("f32", 50, 32, 1000, 11),
+  ("f32", 50, 16, 4000, 36), ("f32", 100, 16, 15, 4), ("f32", 100, 16, 30, 14), ("f32", 100, 16, 50, 14),
+  ("f32", 100, 16, 800, 17), ("f32", 100, 16, 2000, 24), ("f16", 100, 16, 30, 6), ("f16", 100, 16, 60, 14),
+  ("bf16", 100, 16, 2000, 14), ("f32", 140, 16, 300, 10), ("f32", 140, 16, 301, 7), ("f32", 140, 16, 2000, 10),
+  ("f32", 600, 16, 100, 2), ("f16", 600, 16, 200, 14), ("f32", 600, 16, 201, 10), ("f32", 600, 16, 1200, 14)])
+def test_batches_at_the_lines_of_the_choice(row_dtype, d, max_m0, ef, per_sm):
+  """The largest batch of one kernel (queries per SM) and one query more, against one warp per query."""
+  import torch
+  _same_as_one_warp_per_query(d, ef, per_sm * torch.cuda.get_device_properties(0).multi_processor_count, row_dtype,
+                               max_m0)
+
+
+def _same_as_one_warp_per_query(d, ef, nq, row_dtype="f32", max_m0=16):
   rng = np.random.default_rng(nq)
   base = rng.standard_normal((4000, d)).astype(np.float32)
   q = rng.standard_normal((nq + 1, d)).astype(np.float32)
-  opt = dict(dist_type="l2", max_m=8, max_m0=16, ef_construction=32, seed=4, batch_max=1024)
+  opt = dict(dist_type="l2", max_m=8, max_m0=max_m0, ef_construction=32, seed=4, batch_max=1024, row_dtype=row_dtype)
   engines = []
   for team in (-1, 0):
     engines.append(CuHNSW(engine_options(dict(opt, search_team=team))))
