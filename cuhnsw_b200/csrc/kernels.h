@@ -88,7 +88,7 @@ cudaError_t launch_search_walk_f16(const SearchParams& p, int sm_count, cudaStre
 cudaError_t launch_search_walk_bf16(const SearchParams& p, int sm_count, cudaStream_t stream,
                                     const SearchSchedule* sched);
 // first stage of a scheduled search: descent of every query + sort; fills p.order / entry_node / entry_dist
-cudaError_t schedule_search(SearchParams& p, const SearchSchedule& sched, int sm_count, cudaStream_t stream);
+cudaError_t schedule_search(SearchParams& p, const SearchSchedule& sched, cudaStream_t stream);
 // search whose device staging and work ticket live in a fixed file-scope device array (no allocation)
 size_t search_static_capacity();
 size_t search_static_bytes(long long nq, int d, int topk);

@@ -175,8 +175,7 @@ size_t search_schedule_tmp_bytes(long long nq) {
   return bytes;
 }
 
-cudaError_t schedule_search(SearchParams& p, const SearchSchedule& s, int sm_count, cudaStream_t stream) {
-  (void)sm_count;
+cudaError_t schedule_search(SearchParams& p, const SearchSchedule& s, cudaStream_t stream) {
   if (p.nq > s.capacity || p.nq > 0x7fffffffll) return cudaErrorInvalidValue;  // the sort counts items in an int
 #define CALL(R) launch_entry_rows<R>(p, s, stream)
   cudaError_t e = HNSW_WITH_ROWS(p.g.rows16, CALL);
@@ -237,7 +236,7 @@ static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaSt
   if (e != cudaSuccess) return e;
   // more queries than resident warps: start the long walks first
   if (sched && p.nq > grid * kWarpsPerCta && p.nq <= sched->capacity && p.nq <= 0x7fffffffll) {
-    e = schedule_search(p, *sched, sm_count, stream);
+    e = schedule_search(p, *sched, stream);
     if (e != cudaSuccess) return e;
     e = residents(knn_search_kernel<Dist, kReverse, true>, smem, &per_sm);
     if (e != cudaSuccess) return e;

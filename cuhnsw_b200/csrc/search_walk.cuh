@@ -115,7 +115,7 @@ cudaError_t launch_walk_t(const SearchParams& p0, int table_top, int sm_count, c
   const long long grid = std::max(1ll, std::min((long long)per_sm * sm_count, p.nq));
   // more queries than resident walks: start the long ones first
   if (sched && p.nq > grid && p.nq <= sched->capacity && p.nq <= 0x7fffffffll) {
-    e = schedule_search(p, *sched, sm_count, stream);
+    e = schedule_search(p, *sched, stream);
     if (e != cudaSuccess) return e;
   }
   if (p.nq <= grid) p.ticket = nullptr;  // a CTA for every query: nothing to hand out, and no counter to clear
