@@ -13,6 +13,7 @@ import json
 import os
 import tempfile
 import threading
+import weakref
 
 import numpy as np
 
@@ -114,6 +115,7 @@ class CuHNSW:
     self.opt = cfg
     self.logger = aux.get_logger("cuhnsw", cfg.py_log_level)
     self.data = None
+    self._last_rows = lambda: None  # the array under `data` if _rows_of_shape made it and it is still there
     self._batch_slots = []  # streams and page-locked buffers of search_knn_batches, kept between calls
     self._batches_running = False
     self.obj = CuHNSWBind()
@@ -135,15 +137,16 @@ class CuHNSW:
     data = np.asarray(data)
     # (a copy in another order has its rows' squares summed in another order: those are left to numpy as a whole)
     if data.ndim == 2 and data.size > 0 and data.flags.c_contiguous:
-      rows = np.empty(data.shape, np.float32)
-      if not self.opt.nrz and data.dtype == np.float32 and rows.nbytes >= _SHARED_ROWS_BYTES:
+      if not self.opt.nrz and data.dtype == np.float32 and data.nbytes >= _SHARED_ROWS_BYTES:
         # the device gets the caller's rows as they are, while the copy is made
+        rows = self._rows_of_shape(data.shape)
         self.logger.info("data shape: %d x %d", *rows.shape)
         try:
           _fill_rows(rows, data, False, before=lambda: self.obj.set_data(data))
         finally:
           self.data = rows
       else:
+        rows = np.empty(data.shape, np.float32)
         _fill_rows(rows, data, self.opt.nrz)
         self.data = rows  # (values that do not convert leave everything as it was)
         self.logger.info("data shape: %d x %d", *rows.shape)
@@ -155,6 +158,24 @@ class CuHNSW:
     self.data = rows
     self.logger.info("data shape: %d x %d", *rows.shape)
     self.obj.set_data(rows)
+
+  def _rows_of_shape(self, shape):
+    """A float32 array for a copy that cannot fail.  It takes the memory of the copy before if that one's array is gone once
+    ``data`` is (1 M x 128: 11 ms of page faults less).  Every view, tensor or buffer of the array refers to the one over
+    the bare memory, whose base is no array: while a reference to that one lives, somebody holds the rows."""
+    memory, last, data = None, self._last_rows(), self.data
+    same = last is not None and getattr(data, "base", None) is last
+    if same and last.nbytes == data.nbytes == 4 * shape[0] * shape[1]:
+      memory, former = last.base.obj, data.shape
+      self.data = data = last = None
+      last = self._last_rows()
+      if last is not None:
+        memory, self.data = None, last.reshape(former)
+    if memory is None:
+      memory = np.empty(4 * shape[0] * shape[1], np.uint8)
+    whole = np.frombuffer(memoryview(memory), np.float32)
+    self._last_rows = weakref.ref(whole)
+    return whole.reshape(shape)
 
   def set_random_levels(self):
     """level(i) = int32(-ln(max(U_i, 1e-10)) * level_mult) with U from numpy's legacy generator seeded

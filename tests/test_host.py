@@ -225,6 +225,34 @@ def test_set_data_never_writes_over_an_array_it_handed_out(monkeypatch):
     assert (kept == 1).all() and (index.data == 0).all()
 
 
+@pytest.mark.parametrize("hold", ["nothing", "the array", "a row of a view", "a buffer", "a tensor", "an engine call"])
+def test_the_memory_of_a_former_copy_is_used_again_when_nobody_can_see_it(hold):
+  import torch
+  n = 50_000
+  index = _Engine()(dist_type="l2")
+  index.set_data(np.ones((n, 50), np.float32))
+  first = index.data.ctypes.data
+  kept = {"nothing": lambda x: None, "the array": lambda x: x, "a row of a view": lambda x: x.T[3][5:].view(np.uint32),
+          "a buffer": memoryview, "a tensor": torch.from_numpy, "an engine call": lambda x: x.ctypes}[hold](index.data)
+  index.set_data(np.zeros((n // 2, 100), np.float32))
+  assert index.data.shape == (n // 2, 100) and (index.data == 0).all()
+  assert (index.data.ctypes.data == first) == (hold == "nothing")
+  if hold == "a row of a view":
+    assert (kept == np.float32(1).view(np.uint32)).all()
+  elif hold != "nothing":
+    assert (np.asarray(kept if hold != "an engine call" else kept._arr) == 1).all()
+  # its own rows as the next corpus; an array put in the place of `data`
+  index.set_data(index.data[::1])
+  assert (index.data == 0).all()
+  index.data = mine = np.full((n, 50), 3, np.float32)
+  index.set_data(np.ones((n, 50), np.float32))
+  assert (mine == 3).all() and (index.data == 1).all()
+  for own in (None, index.data[:7]):
+    index.data = own
+    index.set_data(np.zeros((n, 50), np.float32))
+    assert (index.data == 0).all() and index.data.shape == (n, 50)
+
+
 @pytest.mark.parametrize("n", [5, 50_000])
 def test_rows_that_do_not_convert_leave_the_corpus_in_place(n):
   index = _Engine()(dist_type="l2")
