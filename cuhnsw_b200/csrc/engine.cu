@@ -1276,40 +1276,34 @@ int Engine::LoadIndex(const char* path) {
   long long next = lists_at;  // first byte of the file that has not been read
   size_t pos = 0, end = 0;    // the part of the buffer that has not been taken
   bool unreadable = false;
-  // the next bytes, at most a node's lists (17 KB); null: the file ends before them
-  const auto take = [&](size_t bytes) -> const unsigned char* {
-    if (end - pos < bytes) {
-      std::memmove(piece.data(), piece.data() + pos, end - pos);
-      end -= pos;
-      pos = 0;
-      const long long more = std::min<long long>((long long)(piece.size() - end), fsize - next);
-      if ((long long)end + more < (long long)bytes) return nullptr;
-      if (!ReadRecords(fd, piece.data() + end, 1, more, next, [](long long, long long) {})) {
-        unreadable = true;
-        return nullptr;
-      }
-      end += (size_t)more;
-      next += more;
-    }
-    const unsigned char* at = piece.data() + pos;
-    pos += bytes;
-    return at;
+  // are there so many more bytes, at most a node's lists (17 KB), in the buffer or else in the file?
+  const auto more = [&](size_t bytes) {
+    std::memmove(piece.data(), piece.data() + pos, end - pos);
+    end -= pos;
+    pos = 0;
+    const long long room = std::min<long long>((long long)(piece.size() - end), fsize - next);
+    if ((long long)end + room < (long long)bytes) return false;
+    unreadable = !ReadRecords(fd, piece.data() + end, 1, room, next, [](long long, long long) {});
+    end += (size_t)room;
+    next += room;
+    return !unreadable;
   };
   const auto ended = [&] {
     return Fail(kIoError, unreadable ? "index file: short read" : "index file: truncated link lists");
   };
   for (long long i = 0; i < n; ++i) {
     uint32_t nbytes;
-    const unsigned char* size = take(4);
-    if (!size) return ended();
-    std::memcpy(&nbytes, size, 4);
+    if (end - pos < 4 && !more(4)) return ended();
+    std::memcpy(&nbytes, piece.data() + pos, 4);
+    pos += 4;
     if (nbytes % per_link || nbytes / per_link > 64) return Fail(kParseError, "index file: bad link list size");
     const int lv = (int)(nbytes / per_link);
     if (lv > h.maxlevel) return Fail(kParseError, "index file: a node lies above the file's top level");
     levels_h_[(size_t)i] = lv;
     if (!nbytes) continue;
-    const unsigned char* list = take(nbytes);
-    if (!list) return ended();
+    if (end - pos < nbytes && !more(nbytes)) return ended();
+    const unsigned char* list = piece.data() + pos;
+    pos += nbytes;
     for (int l = 0; l < lv; ++l) {
       const unsigned char* o = list + per_link * (size_t)l;
       uint32_t deg;
