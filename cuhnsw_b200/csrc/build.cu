@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32) init_level_kernel(InitParams
       int cur = L.g.enter_point;
       float dcur = de.eval(cur, 1);
       dcur = __shfl_sync(FULL, dcur, 0);
-      greedy_descent(de, wl.spos, L.g.rowsU, L.g.strideU, L.g.upper_base, L.g.max_level, l, cur, dcur, wc);
+      greedy_descent(de, L.g.rowsU, L.g.strideU, L.g.upper_base, L.g.max_level, l, cur, dcur, wc);
       for (int j = lane; j < L.stride; j += 32) {
         row[j] = (j == 0) ? cur : -1;
         drow[j] = (j == 0) ? dcur : 0.0f;

@@ -30,7 +30,7 @@ namespace hnsw {
 
 struct VecTable {
   const unsigned char* vec;  // n rows
-  size_t row_bytes;          // row stride
+  unsigned row_bytes;        // row stride (32 bits: a row's address is one multiplication and addition)
   int nchunk;                // ceil(d / 4): chunks that hold data
   int d;
   int dist_type;
@@ -172,7 +172,7 @@ struct DistSmall {
   }
   // query = stored (padded) row `id`
   __device__ __forceinline__ void load_query_row(int id) {
-    Row::template load<C, 8>(t.vec + (size_t)id * t.row_bytes, lane_id() & 7, 0, t.nchunk, q);
+    Row::template load<C, 8>(t.vec + (size_t)(unsigned)id * t.row_bytes, lane_id() & 7, 0, t.nchunk, q);
   }
 
   // Lane r (r < n <= 32, n >= 1) holds a row id; returns the distance to it in lane r.
@@ -196,7 +196,7 @@ struct DistSmall {
         const int r = r0 + 4 * u + team;
         const int rid = __shfl_sync(FULL, id, r < n ? r : 0);
         // only the last chunk column can lie past the end of the row
-        Row::template load<C, 8, true>(t.vec + (size_t)rid * t.row_bytes, tl, 0, t.nchunk, v[u]);
+        Row::template load<C, 8, true>(t.vec + (size_t)(unsigned)rid * t.row_bytes, tl, 0, t.nchunk, v[u]);
       }
 #pragma unroll
       for (int u = 0; u < kB; ++u) {
@@ -285,7 +285,7 @@ struct DistLargeT {
     __syncwarp();
   }
   __device__ __forceinline__ void load_query_row(int id) {
-    const unsigned char* row = t.vec + (size_t)id * t.row_bytes;
+    const unsigned char* row = t.vec + (size_t)(unsigned)id * t.row_bytes;
     for (int c0 = 0; c0 < C; c0 += 2) {
       float4 v[2];
       Row::template load<2, 32>(row, lane_id(), c0, t.nchunk, v);
@@ -311,7 +311,7 @@ struct DistLargeT {
 #pragma unroll
         for (int u = 0; u < kRows; ++u) {
           // rows past n are folded onto row 0: a harmless repeated load whose result nobody selects
-          Row::template load<kChunks, 32>(t.vec + (size_t)(rid[u] >= 0 ? rid[u] : 0) * t.row_bytes, lane, c0, t.nchunk,
+          Row::template load<kChunks, 32>(t.vec + (size_t)(unsigned)(rid[u] >= 0 ? rid[u] : 0) * t.row_bytes, lane, c0, t.nchunk,
                                           v[u]);
         }
 #pragma unroll

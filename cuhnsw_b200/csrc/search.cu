@@ -53,7 +53,7 @@ knn_search_kernel(SearchParams p) {
       dcur = de.eval(cur, 1);
       dcur = __shfl_sync(FULL, dcur, 0);
       wc.evals += 1;
-      greedy_descent(de, wl.spos, p.g.rowsU, p.g.strideU, p.g.upper_base, p.g.max_level, 0, cur, dcur, wc);
+      greedy_descent(de, p.g.rowsU, p.g.strideU, p.g.upper_base, p.g.max_level, 0, cur, dcur, wc);
     }
     // layer 0: list = {entry}, visited = {entry} (cuda_search_kernels.cuh:108-112)
     wl.seed(mkkey(dcur, cur));
@@ -91,7 +91,6 @@ knn_search_kernel(SearchParams p) {
 template <class Dist>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) entry_kernel(SearchParams p, SearchSchedule s) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int scratch[kWarpsPerCta][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long qi = (long long)blockIdx.x * kWarpsPerCta + warp;
   if (qi >= p.nq) return;
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) entry_kernel(SearchParams p
   float dcur = de.eval(cur, 1);
   dcur = __shfl_sync(FULL, dcur, 0);
   wc.evals += 1;
-  greedy_descent(de, smem_addr(scratch[warp]), p.g.rowsU, p.g.strideU, p.g.upper_base, p.g.max_level, 0, cur, dcur, wc);
+  greedy_descent(de, p.g.rowsU, p.g.strideU, p.g.upper_base, p.g.max_level, 0, cur, dcur, wc);
   if (lane == 0) {
     s.entry_node[qi] = cur;
     s.entry_dist[qi] = dcur;

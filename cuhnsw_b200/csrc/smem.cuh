@@ -24,6 +24,11 @@ __device__ __forceinline__ uint2 lds64(unsigned at) {
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(at) : "memory");
   return v;
 }
+__device__ __forceinline__ uint4 lds128(unsigned at) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+  return v;
+}
 __device__ __forceinline__ void sts32(unsigned at, unsigned v) {
   asm volatile("st.shared.u32 [%0], %1;" : : "r"(at), "r"(v) : "memory");
 }
