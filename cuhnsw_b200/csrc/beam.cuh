@@ -51,9 +51,9 @@ __host__ __device__ inline int visited_tag_bits(long long n, int buckets) {
 // Lossy set of node ids in shared memory with no false positives.  id -> h = id * odd mod 2^B is a bijection on B-bit
 // numbers.  Bucket b, of any number of buckets, holds the range of h with floor(h * buckets / 2^B) = b, whose low bits, the
 // tag, differ, so (bucket, tag) identifies the id exactly and only the tag has to be stored, with one more bit that says that
-// there is one.  Each bucket keeps its four most recent tags; a displaced id can only cause a repeated distance
-// evaluation, never a different result, because duplicates are rejected when merging into the list and a key that left the
-// list can never re-enter.
+// there is one.  Each bucket keeps its four most recent tags; a displaced id is evaluated again when it comes
+// back, which is never a different result: WarpList turns it down when merging, Frontier looks it up (an id that is not in
+// the table can only have been there if its bucket is full), and a key that left the list can never re-enter.
 // Four tags per bucket instead of two in the same space, tested two at a time: evaluations per query at 1.18 M x 50, ef 200
 // and 400, 1173 -> 1075 and 1545 -> 1288 (1027 distinct rows at ef 200), at 1 M x 128, ef 256, 3887 -> 3624.
 struct VisitedTable {
@@ -102,24 +102,67 @@ struct VisitedTable {
     const unsigned t = tag | 0x80000000u;
     return w.x == t || w.y == t || w.z == t || w.w == t;
   }
-  // the same, and an id that is not there enters if `on`
-  __device__ __forceinline__ bool test_and_set(int id, bool on = true) {
+  // What the table said of an id: `full`: if it is not known, it may have been forgotten.
+  struct Seen {
+    unsigned at, tag;
+    bool known, full;
+  };
+  // an id that is not there enters if `on`
+  __device__ __forceinline__ Seen enter(int id, bool on) {
     const unsigned g = (unsigned)id * mul, b = __umulhi(g, buckets);
     const unsigned tag = (g >> shift) & tag_mask;
+    Seen s;
     if (!wide) {
-      const unsigned at = vt + 8 * b, one = tag | 0x8000u, t = one * 0x10001u;
-      const uint2 w = lds64(at);
-      const bool known = (zero_half(w.x ^ t) | zero_half(w.y ^ t)) != 0u;
-      if (on && !known) sts64(at, (w.x << 16) | one, __funnelshift_l(w.x, w.y, 16));
-      return known;
+      s.at = vt + 8 * b;
+      s.tag = tag | 0x8000u;
+      const uint2 w = lds64(s.at);
+      const unsigned t = s.tag * 0x10001u;
+      s.known = (zero_half(w.x ^ t) | zero_half(w.y ^ t)) != 0u;
+      s.full = w.y >> 31;
+      if (on && !s.known) put(s, w);
+    } else {
+      s.at = vt + 16 * b;
+      s.tag = tag | 0x80000000u;
+      const uint4 w = lds128(s.at);
+      s.known = w.x == s.tag || w.y == s.tag || w.z == s.tag || w.w == s.tag;
+      s.full = w.w != 0u;
+      if (on && !s.known) sts128(s.at, s.tag, w.x, w.y, w.z);
     }
-    const unsigned at = vt + 16 * b, t = tag | 0x80000000u;
-    const uint4 w = lds128(at);
-    const bool known = w.x == t || w.y == t || w.z == t || w.w == t;
-    if (on && !known) sts128(at, t, w.x, w.y, w.z);
-    return known;
+    return s;
   }
+  __device__ __forceinline__ void put(const Seen& s, uint2 w) const {
+    sts64(s.at, (w.x << 16) | s.tag, __funnelshift_l(w.x, w.y, 16));
+  }
+  // Behind a __syncwarp: ids that entered a bucket together with others, of which one was stored, enter again until they
+  // are there or their bucket is full.
+  __device__ __forceinline__ void settle(const Seen& s, bool entered) {
+    const unsigned newest = lds32(s.at);
+    if (!__any_sync(FULL, entered && (wide ? newest : newest & 0xffffu) != s.tag)) return;
+    for (;;) {
+      bool missing;
+      if (!wide) {
+        const uint2 w = lds64(s.at);
+        const unsigned t = s.tag * 0x10001u;
+        missing = entered && (zero_half(w.x ^ t) | zero_half(w.y ^ t)) == 0u && !(w.y >> 31);
+        if (!__any_sync(FULL, missing)) return;
+        if (missing) put(s, w);
+      } else {
+        const uint4 w = lds128(s.at);
+        missing = entered && w.x != s.tag && w.y != s.tag && w.z != s.tag && w.w == 0u;
+        if (!__any_sync(FULL, missing)) return;
+        if (missing) sts128(s.at, s.tag, w.x, w.y, w.z);
+      }
+      __syncwarp();
+    }
+  }
+  __device__ __forceinline__ bool test_and_set(int id, bool on = true) { return enter(id, on).known; }
 };
+
+// key i of an array of keys in shared memory
+__device__ __forceinline__ unsigned long long key_at(unsigned keys, int i) {
+  const uint2 w = lds64(keys + 8 * i);
+  return ((unsigned long long)w.y << 32) | w.x;
+}
 
 // Per-warp shared-memory state.  Loop bounds and branch conditions come from ballots, shuffles and reductions rather than
 // from loads, so that the compiler knows them to be the same in every lane (figures in smem.cuh).
@@ -430,6 +473,35 @@ __device__ __forceinline__ void beam_layer(Dist& de, WarpList& wl, const int* __
     k = wl.low_words(wl.cursor);
   }
 }
+
+// The adjacency rows of one layer, for a warp whose lanes read a slot each.
+struct LayerRows {
+  const char* mine;  // this lane's slot of row 0
+  unsigned bytes;    // of a row
+  int stride;        // slots
+  const int* upper_base;
+  int level;
+  int lane;
+
+  __device__ __forceinline__ LayerRows() {}
+  __device__ __forceinline__ LayerRows(const int* rows, int stride_, const int* upper_base_, int level_) {
+    lane = lane_number();
+    mine = reinterpret_cast<const char*>(rows + lane);
+    bytes = 4u * (unsigned)stride_;
+    stride = stride_;
+    upper_base = upper_base_;
+    level = level_;
+  }
+  // (row numbers have 32 bits, so an address is one multiplication and addition)
+  __device__ __forceinline__ const int* row(int id) const {
+    const unsigned r = level == 0 ? (unsigned)id : (unsigned)(__ldg(upper_base + id) + (level - 1));
+    return reinterpret_cast<const int*>(mine + (size_t)r * bytes);
+  }
+  // slot base + lane of the row at p
+  __device__ __forceinline__ int read(const int* p, int base) const {
+    return base + lane < stride ? __ldg(p + base) : -1;
+  }
+};
 
 // reverse_cand variant (cuda_utils_kernels.cuh:113-124 of the reference): every step expands
 // the FARTHEST unexpanded key of the list; the walk ends when every key is expanded.

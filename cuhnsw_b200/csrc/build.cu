@@ -21,7 +21,7 @@
 
 #include "kernels.h"
 #include "beam.cuh"
-#include "walk.cuh"
+#include "frontier_walk.cuh"
 
 namespace hnsw {
 
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_s
   }
 }
 
-// The same selection (select_neighbors with no newcomer) by the W warps of a CTA over the ascending keys of a KeyList:
+// The same selection (select_neighbors with no newcomer) by the W warps of a CTA over ascending keys:
 // each warp tests one of the next W candidates against the accepted neighbours and against the candidates before its
 // own; which of those were accepted is known once all have reported, so the outcome is that of one candidate after the
 // other.  ids, dist, flags: shared-memory addresses (kMaxLinks words each, W words).  Every warp returns the degree.
@@ -307,16 +307,16 @@ __device__ __forceinline__ int select_team(Dist& de, unsigned keys, int nc, int 
   int head = min(nn_num, max_head);
   for (int j = threadIdx.x; j < head; j += 32 * W) {
     const uint2 k = lds64(keys + 8 * j);
-    sts32(ids + 4 * j, k.y >> 1);
-    sts32(dist + 4 * j, __float_as_uint(ord2f(k.x)));
+    sts32(ids + 4 * j, k.x);
+    sts32(dist + 4 * j, __float_as_uint(ord2f(k.y)));
   }
   __syncthreads();
   for (int j0 = head; j0 < nc && head < m; j0 += W) {
     unsigned flag = 0;
     if (j0 + w < nc) {
       const uint2 k = lds64(keys + 8 * (j0 + w));
-      const float cd = ord2f(__shfl_sync(FULL, k.x, 0));
-      de.load_query_row((int)(__shfl_sync(FULL, k.y, 0) >> 1));
+      const float cd = ord2f(__shfl_sync(FULL, k.y, 0));
+      de.load_query_row((int)__shfl_sync(FULL, k.x, 0));
       for (int base = 0; base < head && flag == 0; base += 8) {
         const int n = min(8, head - base);
         const int id = lane < n ? (int)lds32(ids + 4 * (base + lane)) : 0;
@@ -325,7 +325,7 @@ __device__ __forceinline__ int select_team(Dist& de, unsigned keys, int nc, int 
         if (__any_sync(FULL, lane < n && cd > dd)) flag = kTurnedDown;
       }
       if (w > 0 && flag == 0) {
-        const int id = lane < w ? (int)(lds64(keys + 8 * (j0 + lane)).y >> 1) : 0;
+        const int id = lane < w ? (int)lds64(keys + 8 * (j0 + lane)).x : 0;
         const float dd = de.eval_eight(id, w);
         wc.evals += w;
         flag = __ballot_sync(FULL, lane < w && cd > dd);
@@ -345,8 +345,8 @@ __device__ __forceinline__ int select_team(Dist& de, unsigned keys, int nc, int 
       }
       if (threadIdx.x == 0 && at >= 0) {
         const uint2 k = lds64(keys + 8 * (j0 + u));
-        sts32(ids + 4 * at, k.y >> 1);
-        sts32(dist + 4 * at, __float_as_uint(ord2f(k.x)));
+        sts32(ids + 4 * at, k.x);
+        sts32(dist + 4 * at, __float_as_uint(ord2f(k.y)));
       }
     }
     __syncthreads();
@@ -355,7 +355,7 @@ __device__ __forceinline__ int select_team(Dist& de, unsigned keys, int nc, int 
 }
 
 // Phase A for batches that leave the machine idle (the first of every level, and small corpora): one CTA per node, whose
-// walk prepares several nodes at a time (walk.cuh) and whose warps share the selection.
+// walk prepares several nodes at a time (frontier_walk.cuh) and whose warps share the selection.
 constexpr int kTeamWarps = 4, kTeamNodes = 8;
 constexpr int kTeamTable = 4096;          // entries of its visited table
 // largest batch, in nodes per SM (whole builds with 0 / 10 / 20 / 40: 100 000 x 50 24.6 / 23.6 / 24.1 / 25.0 ms,
@@ -363,15 +363,16 @@ constexpr int kTeamTable = 4096;          // entries of its visited table
 constexpr int kTeamPerSm = 10;
 constexpr size_t kTeamSmem = 56u << 10;   // more shared memory than this leaves fewer than four CTAs per SM
 template <class Dist>
-using BuildWalk = Walk<Dist, kTeamWarps, kTeamNodes>;
+using BuildWalk = FrontierWalk<Dist, kTeamWarps, kTeamNodes>;
 // walk, the selection's arrays, and for wide rows a query for each warp's candidate
 template <class Dist>
-inline size_t build_team_smem(const BuildLevel& L, int vsize) {
+inline size_t build_team_smem(const BuildLevel& L, int entries) {
   return (Dist::smem_bytes(L.g.d) * (1 + kTeamWarps) +
-          BuildWalk<Dist>::smem_bytes(L.ef_construction, L.stride, vsize, L.g.n) + kMaxLinks * 8 + 16 + 15) / 16 * 16;
+          BuildWalk<Dist>::smem_bytes(Frontier::slots_for(L.ef_construction), L.stride, entries, L.g.n) +
+          kMaxLinks * 8 + 16 + 15) / 16 * 16;
 }
 template <class Dist>
-__global__ void __launch_bounds__(32 * kTeamWarps, Dist::kTeamMinCtas) build_search_team_kernel(BatchParams p, int vsize) {
+__global__ void __launch_bounds__(32 * kTeamWarps, Dist::kTeamMinCtas) build_search_team_kernel(BatchParams p, int entries) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = lane_number();
   const BuildLevel& L = p.L;
@@ -386,16 +387,14 @@ __global__ void __launch_bounds__(32 * kTeamWarps, Dist::kTeamMinCtas) build_sea
   at += Dist::smem_bytes(L.g.d) * kTeamWarps;
   const unsigned ids = kept(smem_addr(at)), dist = ids + 4 * kMaxLinks, flags = dist + 4 * kMaxLinks;
   at += kMaxLinks * 8 + 16;
-  walk.bind(at, L.ef_construction, L.stride, vsize, L.g.n);
-  walk.rows = L.rows;
-  walk.upper_base = L.g.upper_base;
-  walk.level = L.level;
+  walk.bind(at, L.ef_construction, Frontier::slots_for(L.ef_construction), L.stride, entries, L.g.n);
+  walk.rows = LayerRows(L.rows, L.stride, L.g.upper_base, L.level);
   const auto select = [&](int nc) {
-    return select_team<Dist, kTeamWarps>(Dist::kSharedQuery ? own : walk.de, walk.list.keys, nc, L.max_m, p.nn_num,
+    return select_team<Dist, kTeamWarps>(Dist::kSharedQuery ? own : walk.de, walk.fr.slots, nc, L.max_m, p.nn_num,
                                          L.save_remains, ids, dist, flags, w, walk.wc);
   };
   if (w > 0) {
-    while (walk.help(nullptr) != kWalkOver) select(walk.posted(WalkBoard<kTeamNodes>::kPool));
+    while (walk.help(nullptr) != kWalkOver) select(walk.posted(FrontierBoard<kTeamNodes>::kPool));
     if (p.S.stats && lane == 0) atomicAdd(p.S.stats + 0, (unsigned long long)walk.wc.evals);
     return;
   }
@@ -407,11 +406,13 @@ __global__ void __launch_bounds__(32 * kTeamWarps, Dist::kTeamMinCtas) build_sea
     const int s = L.nodes ? __ldg(L.nodes + p.first + t) : (int)(p.first + t);
     walk.start(kWalkNode, nullptr, s);
     // seeds: the node's current row (cuda_build_kernels.cuh:203-212)
-    walk.seed_row(walk.row_of(s));
+    walk.seed_row(s);
     walk.run();
-    if (lane == 0) sts32(walk.board + WalkBoard<kTeamNodes>::kPool, walk.list.size);
+    walk.fr.sort_done();
+    const int nc = min(walk.fr.done, L.ef_construction);
+    if (lane == 0) sts32(walk.board + FrontierBoard<kTeamNodes>::kPool, nc);
     walk.post(kWalkSelect);
-    const int deg = select(walk.list.size);
+    const int deg = select(nc);
     int* so = p.S.st_ids + (size_t)t * L.stride;
     float* sd = p.S.st_dist + (size_t)t * L.stride;
     for (int j = lane; j < L.stride; j += 32) {
@@ -613,14 +614,14 @@ static cudaError_t build_batch_t(const BuildLevel& L, const BuildScratch& S, lon
   p.nn_num = (int)(L.max_m * (double)L.heuristic_coef);
   cudaError_t e = cudaMemsetAsync(S.ticket, 0, 2 * sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return e;
-  const int team_vsize = L.vsize_fixed ? L.vsize : L.vsize > kTeamTable ? L.vsize : kTeamTable;
-  const size_t team_smem = build_team_smem<Dist>(L, team_vsize);
+  const int team_entries = L.vsize_fixed ? L.vsize : kTeamTable;
+  const size_t team_smem = build_team_smem<Dist>(L, team_entries);
   if (!L.reverse_cand && count <= (long long)sm_count * kTeamPerSm && team_smem <= kTeamSmem) {
     auto kern = build_search_team_kernel<Dist>;
     int grid = 1;
     e = grid_for(kern, team_smem, 32 * kTeamWarps, sm_count, count, &grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, 32 * kTeamWarps, team_smem, stream>>>(p, team_vsize);
+    kern<<<grid, 32 * kTeamWarps, team_smem, stream>>>(p, team_entries);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   } else {
     size_t per_warp = build_smem_per_warp<Dist>(L.g.d, p.cap, L.vsize, L.g.n);

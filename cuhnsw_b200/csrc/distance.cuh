@@ -121,6 +121,14 @@ __device__ __forceinline__ float4 first4(const float4& a, const float4& b) {
   return make_float4(__fmul_rn(dx, dx), __fmul_rn(dy, dy), __fmul_rn(dz, dz), __fmul_rn(dw, dw));
 }
 
+// see eval_pool
+template <bool kLeast>
+__device__ __forceinline__ void put_evaluated(uint2 e, float dist, unsigned least) {
+  const unsigned image = f2ord(dist);
+  sts64(kLeast ? e.y & 0xffffffu : e.y, image, e.x);
+  if (kLeast) atomic_min_shared(least + 4 * (e.y >> 24), image);
+}
+
 __device__ __forceinline__ float fold4(const float4& a) { return (a.x + a.y) + (a.z + a.w); }
 
 // ---------------------------------------------------------------------------
@@ -146,6 +154,7 @@ struct DistSmall {
   static constexpr int kBuildMinCtas = C <= 3 ? 16 : 12;
   static constexpr int kWarpsPerSmTarget = 32;
   static constexpr int kTeamMinCtas = 5;  // construction with one CTA of four warps per node
+  static constexpr bool kDeepPool = C <= 3;    // eval_pool with two eights of rows under way without spills
   static constexpr bool kSharedQuery = false;  // every warp keeps its own copy of the query
   __host__ __device__ static constexpr size_t smem_bytes(int) { return 0; }
 
@@ -217,37 +226,60 @@ struct DistSmall {
     return result;
   }
 
-  // Rows r = 8 w .. 8 w + 7, 8 (w + warps) ..., below n, of a pool of (id, address) pairs in shared memory: the words
-  // (distance image, id) of row r go to its address.  A team takes two rows at a time, whose lane sums are folded together: the first exchange of
-  // the butterfly leaves one row in each half of the team (the pairs that are added are the same, so are the
-  // sums), and eight rows cost 5 shuffles instead of the 16 of two passes of eval().
-  __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps) {
-    if (t.dist_type == DIST_DOT) eval_pool_t<true>(pool, n, w, warps);
-    else eval_pool_t<false>(pool, n, w, warps);
+  // Rows a and b of a team, as lane sums: the first exchange of the butterfly leaves a's in the lower half of the team and
+  // b's in the upper one.  The pairs that are added are those of eval(), so the sums are the same.
+  __device__ __forceinline__ float fold_two(float a, float b) const {
+    const bool second = lane_no & 4;
+    float s = (second ? b : a) + __shfl_xor_sync(FULL, second ? a : b, 4);
+    s += __shfl_xor_sync(FULL, s, 2);
+    s += __shfl_xor_sync(FULL, s, 1);
+    return s;
   }
-  template <bool kDot>
-  __device__ __forceinline__ void eval_pool_t(unsigned pool, int n, int w, int warps) {
+  // The rows of a pool of n (id, place) pairs in shared memory, eight at a time for each of the `warps` warps: the words
+  // (distance image, id) of a row go to its place, an address.  kLeast: the address has 24 bits, and the smallest image of the
+  // rows with the same upper 8 bits b goes to word b at `least`.  A team takes two rows at a time, whose lane sums are folded together:
+  // the first exchange of the butterfly leaves one row in each half of the team (the pairs that are added are the same, so
+  // are the sums), and eight rows cost 5 shuffles instead of the 16 of two passes of eval().  kPairs: such eights whose
+  // loads are issued together.
+  template <int kPairs, bool kLeast>
+  __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps, unsigned least) {
+    if (t.dist_type == DIST_DOT) eval_pool_t<true, kPairs, kLeast>(pool, n, w, warps, least);
+    else eval_pool_t<false, kPairs, kLeast>(pool, n, w, warps, least);
+  }
+  template <bool kDot, int kPairs, bool kLeast>
+  __device__ __forceinline__ void eval_pool_t(unsigned pool, int n, int w, int warps, unsigned least) {
     const int team = lane_no >> 3, tl = lane_no & 7;
     const bool second = tl & 4;
-    for (int r0 = 8 * w; r0 < n; r0 += 8 * warps) {
-      const int ra = r0 + team, rb = ra + 4;
-      // rows past n are folded onto the last one: a harmless repeated load whose result nobody writes
-      const uint2 ea = lds64(pool + 8 * min(ra, n - 1)), eb = lds64(pool + 8 * min(rb, n - 1));
-      float4 va[C], vb[C];
-      Row::template load<C, 8, true>(t.vec + (size_t)ea.x * t.row_bytes, tl, 0, t.nchunk, va);
-      Row::template load<C, 8, true>(t.vec + (size_t)eb.x * t.row_bytes, tl, 0, t.nchunk, vb);
-      float4 aa = first4<kDot>(q[0], va[0]), ab = first4<kDot>(q[0], vb[0]);
+    for (int r0 = 8 * w; r0 < n; r0 += 8 * kPairs * warps) {
+      uint2 ea[kPairs], eb[kPairs];
+      float4 va[kPairs][C], vb[kPairs][C];
 #pragma unroll
-      for (int c = 1; c < C; ++c) {
-        fma4(aa, q[c], va[c], kDot ? DIST_DOT : DIST_L2);
-        fma4(ab, q[c], vb[c], kDot ? DIST_DOT : DIST_L2);
+      for (int u = 0; u < kPairs; ++u) {
+        // rows past n are folded onto the last one: a harmless repeated load whose result nobody writes
+        const int ra = r0 + 8 * u * warps + team;
+        ea[u] = lds64(pool + 8 * min(ra, n - 1));
+        eb[u] = lds64(pool + 8 * min(ra + 4, n - 1));
       }
-      const float sa = fold4(aa), sb = fold4(ab);
-      float s = (second ? sb : sa) + __shfl_xor_sync(FULL, second ? sa : sb, 4);
-      s += __shfl_xor_sync(FULL, s, 2);
-      s += __shfl_xor_sync(FULL, s, 1);
-      if (kDot) s = -s;
-      if ((tl & 3) == 0 && (second ? rb : ra) < n) sts64(second ? eb.y : ea.y, f2ord(s), second ? eb.x : ea.x);
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) {
+        if (u > 0 && r0 + 8 * u * warps >= n) break;  // warp-uniform
+        Row::template load<C, 8, true>(t.vec + (size_t)ea[u].x * t.row_bytes, tl, 0, t.nchunk, va[u]);
+        Row::template load<C, 8, true>(t.vec + (size_t)eb[u].x * t.row_bytes, tl, 0, t.nchunk, vb[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) {
+        if (u > 0 && r0 + 8 * u * warps >= n) break;
+        float4 aa = first4<kDot>(q[0], va[u][0]), ab = first4<kDot>(q[0], vb[u][0]);
+#pragma unroll
+        for (int c = 1; c < C; ++c) {
+          fma4(aa, q[c], va[u][c], kDot ? DIST_DOT : DIST_L2);
+          fma4(ab, q[c], vb[u][c], kDot ? DIST_DOT : DIST_L2);
+        }
+        float s = fold_two(fold4(aa), fold4(ab));
+        if (kDot) s = -s;
+        const int r = r0 + 8 * u * warps + team + (second ? 4 : 0);
+        if ((tl & 3) == 0 && r < n) put_evaluated<kLeast>(second ? eb[u] : ea[u], s, least);
+      }
     }
   }
 };
@@ -267,6 +299,7 @@ struct DistLargeT {
   static constexpr int kBuildMinCtas = 8;
   static constexpr int kWarpsPerSmTarget = 16;
   static constexpr int kTeamMinCtas = 4;
+  static constexpr bool kDeepPool = false;
   static constexpr bool kSharedQuery = true;   // one copy in shared memory
   __host__ __device__ static constexpr size_t smem_bytes(int d) { return (size_t)((d + 127) / 128) * 128 * sizeof(float); }
 
@@ -338,15 +371,15 @@ struct DistLargeT {
     return result;
   }
   __device__ __forceinline__ float eval_eight(int id, int n) { return eval(id, n); }
-  // Rows r = w, w + warps, ... below n of a pool of (id, address) pairs in shared memory: the words (distance image,
-  // id) of row r go to its address.
-  __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps) {
+  // The same, with rows w, w + warps, ... for warp w.
+  template <int, bool kLeast>
+  __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps, unsigned least) {
     const int lane = lane_id();
     for (int r0 = w; r0 < n; r0 += 32 * warps) {
       const int cnt = min(32, (n - r0 + warps - 1) / warps);
       const uint2 e = lds64(pool + 8 * min(r0 + lane * warps, n - 1));
       const float s = eval((int)e.x, cnt);
-      if (lane < cnt) sts64(e.y, f2ord(s), e.x);
+      if (lane < cnt) put_evaluated<kLeast>(e, s, least);
     }
   }
 };

@@ -30,7 +30,8 @@ struct SearchParams {
   long long nq;
   int topk;
   int ef;
-  int vsize;             // visited table entries per warp (power of two); one CTA per query: chosen by its launcher
+  int vsize;             // visited table entries per warp (power of two); one CTA per query: chosen by its launcher, like
+  int slots = 0;         // its key slots
   int table_request = 0; // the option visited_table_size: entries per query the caller wants, 0 = by size
   size_t smem_optin = 0; // shared memory a CTA / an SM can have
   size_t smem_per_sm = 0;

@@ -48,6 +48,15 @@ __device__ __forceinline__ void atomic_or_shared(unsigned at, unsigned v) {
   asm volatile("red.shared.or.b32 [%0], %1;" : : "r"(at), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void atomic_min_shared(unsigned at, unsigned v) {
+  asm volatile("red.shared.min.u32 [%0], %1;" : : "r"(at), "r"(v) : "memory");
+}
+
+// where `on`, the cache line of global memory at p on its way to the L2 cache
+__device__ __forceinline__ void prefetch_l2_if(bool on, const void* p) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n @p prefetch.global.L2 [%0];\n}" : : "l"(p), "r"((unsigned)on));
+}
+
 // The lane number, read once: the compiler does not fetch it again where registers are short.
 __device__ __forceinline__ int lane_number() {
   unsigned v;

@@ -315,7 +315,7 @@ struct Walk {
           filter_posted(w);
           __syncthreads();
         }
-        de.eval_pool(pool, posted(Board::kPool), w, W);
+        de.template eval_pool<1, false>(pool, posted(Board::kPool), w, W, 0);
       }
       __syncthreads();
     }
@@ -336,7 +336,7 @@ struct Walk {
   __device__ __forceinline__ void evaluate_rows(int n) {
     if (lane == 0) sts32(board + Board::kPool, n);
     post(kWalkRows);
-    de.eval_pool(pool, n, 0, W);
+    de.template eval_pool<1, false>(pool, n, 0, W, 0);
     __syncthreads();
     wc.evals += n;
   }
@@ -518,7 +518,7 @@ struct Walk {
         filter_posted(0);
         __syncthreads();
         const int total = posted(Board::kPool);
-        de.eval_pool(pool, total, 0, W);
+        de.template eval_pool<1, false>(pool, total, 0, W, 0);
         __syncthreads();
         if (chosen) mine.count = (int)lds32(board + Board::kCount + 4 * (lane - c));
         wc.evals += total;

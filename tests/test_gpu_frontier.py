@@ -1,0 +1,40 @@
+"""One CTA per query on a frontier (frontier.cuh, frontier_walk.cuh), for few queries: every shape of the kernel at the batch sizes
+where the choice changes, rows of one and two chunks of links, visited tables so small that most ids are forgotten and have
+to be looked up, lists that run out of slots, results ranked in registers and sorted in place, data full of exact ties."""
+import numpy as np
+import pytest
+
+import oracle
+from conftest import assert_same_bits, engine_options, oracle_graph_of
+from cuhnsw_b200 import CuHNSW
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d,max_m0,dist_type,values,table", [
+  (9, 64, "l2", 2, 64), (50, 24, "dot", 1000, 0), (64, 33, "l2", 3, 512), (96, 48, "dot", 2, 0), (128, 16, "l2", 1000, 64),
+  (200, 64, "dot", 3, 0), (600, 24, "l2", 2, 64), (1000, 40, "dot", 1000, 0)])
+def test_frontier_equals_the_oracle(d, max_m0, dist_type, values, table):
+  import torch
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  rng = np.random.default_rng(d + table)
+  n = 2500
+  base = rng.integers(-values, values + 1, (n, d)).astype(np.float32)
+  opt = dict(dist_type=dist_type, max_m=max(max_m0 // 2, 4), max_m0=max_m0, ef_construction=max(48, max_m0), seed=5,
+             batch_max=512, search_team=1, visited_table_size=table)
+  eng = CuHNSW(engine_options(opt))
+  eng.set_data(base)
+  eng.build()
+  g = oracle_graph_of(eng, base, opt)
+  q = (base[rng.integers(0, n, 3 * sms + 1)] + rng.integers(-1, 2, (3 * sms + 1, d))).astype(np.float32)
+  # the last one: more keys than the index reaches
+  for nq, ef, topk in ((1, 1, 1), (3, 2, 2), (sms, 32, 32), (sms + 1, 33, 33), (2 * sms, 100, 10), (2 * sms + 1, 101, 100),
+                       (sms, 300, 33), (3 * sms, 300, 1), (3 * sms + 1, 60, 60), (20, 2600, 2600)):
+    want = oracle.search(g, q[:nq], topk, ef, counters=True)
+    eng.obj.enable_stats(True)
+    got = eng.search_knn(q[:nq], topk, ef)
+    stats = eng.obj.get_stats()
+    eng.obj.enable_stats(False)
+    assert (got[0] == want[0]).all() and (got[2] == want[2]).all(), (nq, ef)
+    assert_same_bits(got[1], want[1])
+    assert stats["expansions"] == int(want[3][:, 1].sum()) and stats["sweeps"] == int(want[3][:, 2].sum()), (nq, ef)
