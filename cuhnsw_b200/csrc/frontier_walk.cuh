@@ -1,4 +1,5 @@
-// The graph walk of one CTA per query for few queries, on a Frontier instead of a list of the ef closest keys.
+// The graph walk of one CTA per query for few queries and for long walks, on a Frontier instead of a list of the ef closest
+// keys.
 //
 // Rounds as in walk.cuh: select up to P unexpanded nodes, prepare them together, commit those whose turn it is.  There every
 // commit ends in a merge into the sorted list, 1500 cycles of one warp, half to two thirds of a round.  Here
@@ -11,9 +12,9 @@
 //
 // Bound: the chain of a round, two memory round trips and a commit of about 2500 cycles.  One B200, ms, with the list / so: one
 // query of 100 000 x 50, ef 300: 0.261 / 0.181; 148 of 1.18 M x 50, ef 200: 0.477 / 0.350; 37 of 1 M x 96 bfloat16, ef 128: 0.302 / 0.256;
-// one of 150 000 x 960, ef 300: 0.326 / 0.253.  It helps less the more neighbours a node brings, as a commit costs by the
-// neighbour and a merge by the key that is close enough, and does not where a launch waits for the SMs rather than for its
-// longest walk (search_walk.cuh).
+// one of 150 000 x 960, ef 300: 0.326 / 0.253.  It helps the more the longer the list would be (1500 keys: 1.5 to 2.3 times as fast), and the
+// less the more neighbours a node brings, as a commit costs by the neighbour and a merge by the key that is close enough
+// (search_walk.cuh).
 #pragma once
 #include "frontier.cuh"
 #include "walk.cuh"

@@ -125,7 +125,7 @@ cudaError_t launch_walk_t(const SearchParams& p0, int table_top, int sm_count, c
   return cudaGetLastError();
 }
 
-// The same on a frontier (frontier_walk.cuh), for few queries.
+// The same on a frontier (frontier_walk.cuh), for few queries and long walks.
 template <class Dist, int W, int P, int kMinCtas>
 __global__ void __launch_bounds__(32 * W, kMinCtas) knn_frontier_kernel(SearchParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -223,32 +223,46 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
 //   150 000 x 960, ef 300 (the former CTA-per-query kernel / now): 1: 0.338 / 0.251, 300: 1.12 / 0.83, 1000: 1.22 / 1.07
 // Short walks prepare four nodes at a time: their later nodes are less certain and their neighbours overlap more (20 000 x
 // 50, ef 100: 1.6 evaluations for each distinct row with eight, 1.3 with four).
-// Few queries walk on a frontier.  ms, list / frontier, at up to one query per SM, 16 warps x 16 nodes: 148 of 1.18 M x 50, ef 60
-// 0.251 / 0.225, ef 200 0.477 / 0.350; 37 of 1 M x 128 whole numbers, ef 64 0.274 / 0.244; 37 of 1 M x 96, ef 64 0.204 / 0.186.  At up to
-// three, 8 x 8 in three CTAs per SM: 300 of 300 000 x 96 whole numbers, ef 128 0.443 / 0.369; 300 of 300 000 x 64 f16 0.357 /
-// 0.291; 200 of 500 000 x 64 whole numbers 0.483 / 0.416.  At seven it is the data that decides (500 000 x 64 whole numbers, ef 64
-// 0.339 / 0.380, ef 256 0.848 / 0.739; 300 000 x 64 f16, ef 60 0.250 / 0.308; 1.18 M x 50, ef 200 0.677 / 0.566).
-constexpr int kShortWalk = 100;  // largest ef of a short walk
+//
+// List or frontier, ms.  Up to one query per SM 16 warps x 16 nodes: one of 100 000 x 50, ef 300 0.261 / 0.181; 148 of 1.18 M x 50,
+// ef 60 0.251 / 0.225, ef 200 0.477 / 0.350; 37 of 1 M x 128 whole numbers, ef 64 0.274 / 0.244; one and 148 of 600 000 x 50, ef 1500 1.27 /
+// 0.72 and 3.01 / 1.60; but ef 10 0.049 / 0.055 and 0.080 / 0.092, ef 25 the same.  Up to three 8 x 8 in three CTAs per SM: 300 of 300 000 x
+// 96 whole numbers, ef 128 0.443 / 0.369; 300 of 300 000 x 64 f16 0.357 / 0.291; 444 of 200 000 x 128 whole numbers, ef 40 0.240 / 0.236.
+// Beyond, short and middling walks are faster on the one or on the other by the data (1000 of 500 000 x 64 whole numbers, ef 64
+// 0.339 / 0.408, ef 128 0.485 / 0.529; of 300 000 x 96 0.400 / 0.394, 0.540 / 0.499) and get the list, long ones are not slower on the
+// frontier on any of nine tables: 600, 1000 and 2000 of 1.18 M x 50, ef 200 0.67 / 0.55, 0.67 / 0.61, 0.76 / 0.66, ef 400 1.19 / 0.89; of
+// 300 000 x 64 f16 0.43 / 0.36, 0.49 / 0.42, 0.58 / 0.56, ef 400 0.95 / 0.83; of 1 M x 128 whole numbers 0.84 / 0.83, 0.95 / 0.95, 1.12 / 1.08, 1.92 /
+// 1.94 (4000: 1.95 / 2.20); 1000 of 50 000 x 40, ef 700 1.20 / 0.80; rows of up to 32 values 0.515 / 0.595 at 2000, ef 200.
+constexpr int kShortWalk = 100;      // largest ef of a short walk
+constexpr int kRoundsFrom = 32;      // smallest ef of few walks on a frontier
+constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 template <class Dist, int kCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
-  if (p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
-  if (p.nq <= (long long)sm_count * 3) return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
+  if (p.ef >= kRoundsFrom) {
+    if (p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
+    if (p.nq <= (long long)sm_count * 3) return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
+  }
   if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, kCtas>(p, 8192, sm_count, stream, sched);
+  if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14)
+    return launch_frontier_t<Dist, 4, 8, kCtas>(p, 8192, sm_count, stream, sched);
   if (p.nq <= (long long)sm_count * 27) return launch_walk_t<Dist, 4, 8, kCtas>(p, 8192, sm_count, stream, sched);
   return launch_walk_t<Dist, 2, 8, 10>(p, 8192, sm_count, stream, sched);
 }
+// Wide rows, list / frontier: one of 150 000 x 960, ef 300 0.326 / 0.253 (16 x 16); 300 of them 0.890 / 0.679 (8 x 8); one and 148 of 200 000 x
+// 200, ef 1500 1.44 / 0.93 and 3.28 / 1.48; with ef 25 and 10 the frontier is the slower one by 6 to 20 %, with ef 100 they are equal
+// (300 000 x 300).  4 x 8: 1000 of 120 000 x 960, ef 200 0.75 / 0.76, ef 300 1.09 / 0.96, ef 400 1.45 / 1.22; of 300 000 x 300 0.73 / 0.74, 1.01 / 0.94,
+// 1.28 / 1.12; of 200 000 x 150 f16 0.75 / 0.71, 0.94 / 0.81, 1.26 / 0.98; 600 of them, ef 1000 2.62 / 1.78; 400 of 120 000 x 960, ef 200 0.59 / 0.61.
 template <class Dist>
 cudaError_t launch_walk_wide(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
-  // on a frontier while the SMs hold all queries at once.  ms, list / frontier: 148 of 150 000 x 960, ef 60 (8 x 4) 0.305 / 0.281;
-  // 148 of 300 000 x 300, ef 100 (8 x 8) 0.310 / 0.306; 300 of 150 000 x 960, ef 300 (8 x 8) 0.890 / 0.679; one (16 x 16) 0.326 / 0.253
-  if (p.nq <= sm_count) {
-    if (p.ef > kShortWalk) return launch_frontier_t<Dist, 16, 16, 1>(p, 16384, sm_count, stream, sched);
-    if (p.g.d > 512) return launch_frontier_t<Dist, 8, 4, 2>(p, 16384, sm_count, stream, sched);
-  }
+  const bool brief = p.ef <= kShortWalk;
+  if (!brief && p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 16384, sm_count, stream, sched);
   // while two CTAs of eight warps per SM hold all queries at once; further on four CTAs of four serve more (60 000 x 960, 2,
   // 3 and 4 queries per SM, four / eight warps: ef 100 1.21 1.06 0.94, ef 200 1.12 0.96 0.78, ef 400 1.12 0.92 0.73)
-  if (p.nq <= (long long)sm_count * 2) return launch_frontier_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched);
-  if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, 4>(p, 16384, sm_count, stream, sched);
+  if (p.nq <= (long long)sm_count * 2)
+    return brief ? launch_walk_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched)
+                 : launch_frontier_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched);
+  if (brief) return launch_walk_t<Dist, 4, 4, 4>(p, 16384, sm_count, stream, sched);
+  if (p.ef >= kLongWide) return launch_frontier_t<Dist, 4, 8, 4>(p, 16384, sm_count, stream, sched);
   return launch_walk_t<Dist, 4, 8, 4>(p, 16384, sm_count, stream, sched);
 }
 

@@ -28,8 +28,9 @@ def test_frontier_equals_the_oracle(d, max_m0, dist_type, values, table):
   g = oracle_graph_of(eng, base, opt)
   q = (base[rng.integers(0, n, 3 * sms + 1)] + rng.integers(-1, 2, (3 * sms + 1, d))).astype(np.float32)
   # the last one: more keys than the index reaches
-  for nq, ef, topk in ((1, 1, 1), (3, 2, 2), (sms, 32, 32), (sms + 1, 33, 33), (2 * sms, 100, 10), (2 * sms + 1, 101, 100),
-                       (sms, 300, 33), (3 * sms, 300, 1), (3 * sms + 1, 60, 60), (20, 2600, 2600)):
+  for nq, ef, topk in ((1, 1, 1), (3, 31, 2), (sms, 32, 32), (sms + 1, 33, 33), (2 * sms, 100, 10), (2 * sms + 1, 101, 100),
+                       (sms, 300, 33), (3 * sms, 300, 1), (3 * sms + 1, 60, 60), (3 * sms + 1, 200, 10), (3 * sms, 250, 40),
+                       (20, 2600, 2600)):
     want = oracle.search(g, q[:nq], topk, ef, counters=True)
     eng.obj.enable_stats(True)
     got = eng.search_knn(q[:nq], topk, ef)
