@@ -211,7 +211,7 @@ struct Walk {
 
   Dist de;
   KeyList list;
-  VisitedTable vis;
+  VisitedPairs vis;
   unsigned found;  // shared-memory address of kBuffers x stride keys: the prepared nodes' new neighbours
   unsigned pool;   // of the rows to evaluate: (id, address of the key's place in `found`)
   unsigned board;
@@ -224,7 +224,7 @@ struct Walk {
   // shared memory of one walk, without the distance engine's own
   __host__ __device__ static size_t smem_bytes(int ef, int stride, int ventries, long long n) {
     return (size_t)KeyList::bytes(ef) + (size_t)kBuffers * stride * 8 + (size_t)P * stride * 8 + Board::kBytes +
-           VisitedTable::smem_bytes(ventries, n);
+           VisitedPairs::smem_bytes(ventries, n);
   }
   __device__ __forceinline__ void bind(unsigned char* smem, int ef, int stride_, int ventries, long long n) {
     unsigned at = kept(smem_addr(smem));

@@ -39,3 +39,42 @@ def test_the_table_changes_no_answer(d, max_m0, dist_type, values, table):
     assert (got[0] == want[0]).all() and (got[2] == want[2]).all(), ef
     assert_same_bits(got[1], want[1])
     assert stats["expansions"] == int(want[3][:, 1].sum()), ef
+
+
+def _check(eng, g, q, sizes, label):
+  """Searches of the first nq queries with every (nq, ef, topk) against the oracle, expansions included."""
+  for nq, ef, topk in sizes:
+    want = oracle.search(g, q[:nq], topk, ef, counters=True)
+    eng.obj.enable_stats(True)
+    got = eng.search_knn(q[:nq], topk, ef)
+    stats = eng.obj.get_stats()
+    eng.obj.enable_stats(False)
+    assert (got[0] == want[0]).all() and (got[2] == want[2]).all(), (label, nq, ef)
+    assert_same_bits(got[1], want[1])
+    assert stats["expansions"] == int(want[3][:, 1].sum()), (label, nq, ef)
+
+
+# 64 entries: 16 buckets of four tags or 32 of two.  524 289 to 1 048 576 rows: 16 bits tell the ids of a bucket apart in
+# buckets of four (tags of 32 bits), 15 in buckets of two; above both need 32.
+@pytest.mark.parametrize("n,d,row", [(600_000, 8, "f32"), (1_100_000, 8, "f32"), (600_000, 70, "f32"), (1_100_000, 70, "f16"),
+                                     (600_000, 130, "f16"), (1_100_000, 130, "f32")])
+def test_tags_of_16_and_of_32_bits(n, d, row):
+  """Tables of 64 entries over so many rows that a tag does not fit into 15 bits, in every search kernel: one warp, one CTA on
+  a list and one CTA on a frontier per query."""
+  rng = np.random.default_rng(n + d)
+  base = rng.integers(-3, 4, (n, d), dtype=np.int8).astype(np.float32)
+  opt = dict(dist_type="l2", max_m=8, max_m0=16, ef_construction=24, seed=3, row_dtype=row)
+  q = (base[rng.integers(0, n, 500)] + rng.integers(-1, 2, (500, d))).astype(np.float32)
+  eng = CuHNSW(engine_options(opt))
+  eng.set_data(base)
+  eng.build()
+  graph = eng.obj.get_graph()
+  g = oracle_graph_of(eng, base, opt)
+  # the same graph behind handles of each kind: construction does not depend on the table
+  for team in (0, 1):
+    one = CuHNSW(engine_options(opt, search_team=team, visited_table_size=64))
+    one.set_data(base)
+    one.build()
+    for a, b in zip(one.obj.get_graph(), graph):
+      assert (a == b).all()
+    _check(one, g, q, ((40, 20, 10), (40, 120, 120), (33, 300, 10), (500, 120, 10)), (n, d, row, team))
