@@ -66,9 +66,9 @@ struct VisitedTable {
   int vbytes;
 
   // bytes for `entries` tags, a multiple of 16: 2 per tag where 15 bits tell the ids of a bucket apart, else 4
+  __host__ __device__ static bool needs_wide(int entries, long long n) { return visited_tag_bits(n, buckets_of(entries)) > 15; }
   __host__ __device__ static size_t smem_bytes(int entries, long long n) {
-    const int b = buckets_of(entries);
-    return ((size_t)b * (visited_tag_bits(n, b) <= 15 ? 8 : 16) + 15) / 16 * 16;
+    return ((size_t)buckets_of(entries) * (needs_wide(entries, n) ? 16 : 8) + 15) / 16 * 16;
   }
   __host__ __device__ static int buckets_of(int entries) { return entries >= 8 ? entries / 4 : 1; }
   __device__ __forceinline__ void bind_table(unsigned smem, int entries, long long n) {
@@ -160,8 +160,13 @@ struct VisitedTable {
 
 // The same with two tags per bucket, a power of two of buckets, and ~0 for no tag: what a walk on a list of keys needs, which
 // turns down an id that comes twice by itself.  It forgets more (evaluations per query above), but tests a bucket in one
-// word.  One CTA per query on a list, one B200, two / four tags: 1000 queries of 200 000 x 32, ef 128 and 200 0.319 / 0.362 and 0.418 / 0.467
-// ms (72 registers or 76, seven CTAs per SM or six), of 200 000 x 128 whole numbers, ef 128, 0.521 / 0.533.
+// word.  Which of the two is a matter of the registers that the rest of a kernel leaves; one B200, ms, two / four tags:
+//   one warp per query, fp32 rows of 65 to 96 values (40 000 queries, ef 128, of 620 187 x 72, 400 000 x 80, 400 000 x 96) 2.76 / 2.93,
+//   3.65 / 3.80, 2.66 / 2.81, and rows of more than 128 (8000, ef 128, of 200 000 x 150, x 300 and x 500 f16) 1.11 / 1.15, 1.25 / 1.30,
+//   1.28 / 1.36: two.  Rows of up to 64 values (40 000 of 1.18 M x 50) 2.55 / 2.49, 97 to 128 (600 000 x 128) 5.12 / 4.91, 96 bfloat16
+//   2.58 / 2.51: four.
+//   one CTA per query on a list: 1000 of 200 000 x 32, ef 128 and 200 0.318 / 0.360 and 0.415 / 0.460, of 200 000 x 128, ef 128, 0.519 /
+//   0.530: two.
 struct VisitedPairs {
   unsigned vt;     // shared-memory address: buckets of two tags (2 x 16 bit in one word, or 2 x 32 bit)
   unsigned hmask;  // 2^B - 1, B = id_bits(n)
@@ -225,7 +230,8 @@ __device__ __forceinline__ unsigned long long key_at(unsigned keys, int i) {
 
 // Per-warp shared-memory state.  Loop bounds and branch conditions come from ballots, shuffles and reductions rather than
 // from loads, so that the compiler knows them to be the same in every lane (figures in smem.cuh).
-struct WarpList : VisitedTable {
+template <class Table>
+struct WarpList : Table {
   unsigned keys;  // shared-memory address of `cap` 64-bit keys, ascending (distance, id)
   unsigned spos;  // 32 words of scratch
   int cap;
@@ -234,13 +240,13 @@ struct WarpList : VisitedTable {
   unsigned long long worst;  // largest key of a full list, KEY_MAX while there is room
 
   __host__ __device__ static size_t smem_bytes(int cap, int entries, long long n) {
-    return (size_t)((cap + 31) / 32 * 32) * 8 + 32 * 4 + VisitedTable::smem_bytes(entries, n);
+    return (size_t)((cap + 31) / 32 * 32) * 8 + 32 * 4 + Table::smem_bytes(entries, n);
   }
   __device__ __forceinline__ void bind(void* smem, int cap_, int entries, long long n) {
     keys = kept(smem_addr(smem));
     const int capr = (cap_ + 31) / 32 * 32;
     spos = keys + 8 * capr;
-    bind_table(spos + 32 * 4, entries, n);
+    this->bind_table(spos + 32 * 4, entries, n);
     cap = cap_;
     size = 0;
     cursor = 0;
@@ -267,14 +273,14 @@ struct WarpList : VisitedTable {
   // O(nodes touched); the reference resets through a touched-slot list
   // (cuda_search_kernels.cuh:145-147).
   __device__ __forceinline__ void reset() {
-    clear(0, 1);
+    this->clear(0, 1);
     size = 0;
     cursor = 0;
     worst = KEY_MAX;
     __syncwarp();
   }
   __device__ __forceinline__ void mark(int id) {
-    if (lane_id() == 0) test_and_set(id);
+    if (lane_id() == 0) this->test_and_set(id);
     __syncwarp();
   }
 
@@ -435,8 +441,8 @@ struct WarpList : VisitedTable {
 
 // One chunk of an adjacency row (lane l holds the id in slot l, -1 = unused): filter through the
 // visited table, evaluate the fresh ids, merge them.
-template <class Dist>
-__device__ __forceinline__ int expand_chunk(Dist& de, WarpList& wl, int nid, int self, WalkCounters& wc) {
+template <class Dist, class List>
+__device__ __forceinline__ int expand_chunk(Dist& de, List& wl, int nid, int self, WalkCounters& wc) {
   const int lane = lane_id();
   bool fresh = (nid >= 0) && (nid != self);
   fresh = !wl.test_and_set(nid, fresh) && fresh;
@@ -453,8 +459,8 @@ __device__ __forceinline__ int expand_chunk(Dist& de, WarpList& wl, int nid, int
 }
 
 // Whole adjacency row; `rows` is a sentinel-padded table: unused slots hold -1.
-template <class Dist>
-__device__ __forceinline__ void expand_row(Dist& de, WarpList& wl, const int* __restrict__ row, int stride,
+template <class Dist, class List>
+__device__ __forceinline__ void expand_row(Dist& de, List& wl, const int* __restrict__ row, int stride,
                                            int self, WalkCounters& wc) {
   const int lane = lane_id();
   for (int base = 0; base < stride; base += 32) {
@@ -484,8 +490,8 @@ __device__ __forceinline__ const int* row_at(const int* __restrict__ rows, unsig
 // While the neighbours of the current node are gathered, the first 32 slots of
 // the adjacency row of the likely next node (the key after the cursor) are
 // already on their way; a newcomer that overtakes it costs one ordinary load.
-template <class Dist>
-__device__ __forceinline__ void beam_layer(Dist& de, WarpList& wl, const int* __restrict__ rows, int stride,
+template <class Dist, class List>
+__device__ __forceinline__ void beam_layer(Dist& de, List& wl, const int* __restrict__ rows, int stride,
                                            const int* __restrict__ upper_base, int level, int self,
                                            WalkCounters& wc) {
   const int lane = lane_id();
@@ -564,8 +570,8 @@ struct LayerRows {
 
 // reverse_cand variant (cuda_utils_kernels.cuh:113-124 of the reference): every step expands
 // the FARTHEST unexpanded key of the list; the walk ends when every key is expanded.
-template <class Dist>
-__device__ __forceinline__ void beam_layer_reverse(Dist& de, WarpList& wl, const int* __restrict__ rows, int stride,
+template <class Dist, class List>
+__device__ __forceinline__ void beam_layer_reverse(Dist& de, List& wl, const int* __restrict__ rows, int stride,
                                                    const int* __restrict__ upper_base, int level, int self,
                                                    WalkCounters& wc) {
   const int lane = lane_id();

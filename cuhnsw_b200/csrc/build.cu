@@ -27,6 +27,7 @@ namespace hnsw {
 
 constexpr int kBuildWarps = 2;
 constexpr int kMaxLinks = 64;  // largest supported link budget (max_m0)
+using BuildList = WarpList<VisitedTable>;
 
 // Per-warp shared memory of the build kernels, after the Dist block and the WarpList block.
 struct SelBuf {
@@ -48,7 +49,7 @@ struct SelBuf {
 // sel.ids/sel.dist and returns the new degree.  The distance engine's query is
 // overwritten.
 template <class Dist>
-__device__ __forceinline__ int select_neighbors(Dist& de, const WarpList& cands, int nc, int m,
+__device__ __forceinline__ int select_neighbors(Dist& de, const BuildList& cands, int nc, int m,
                                                 int nn_num, int save_remains, SelBuf& sel, WalkCounters& wc) {
   const int lane = lane_id();
   int head = 0;
@@ -109,7 +110,7 @@ __device__ __forceinline__ int select_neighbors(Dist& de, const WarpList& cands,
 // tests use the newcomer's row as the query: two reads deep instead of one read after the other for each candidate
 // behind it.  at: the newcomer's place in cands.
 template <class Dist>
-__device__ __forceinline__ int select_with_newcomer(Dist& de, const WarpList& cands, int nc, int at, int m,
+__device__ __forceinline__ int select_with_newcomer(Dist& de, const BuildList& cands, int nc, int at, int m,
                                                     int nn_num, SelBuf& sel, WalkCounters& wc) {
   const int lane = lane_id();
   // rejected: the newcomer's own place, or none
@@ -156,19 +157,19 @@ __device__ __forceinline__ int select_with_newcomer(Dist& de, const WarpList& ca
 
 template <class Dist>
 __device__ __forceinline__ void bind_warp(unsigned char* smem, int per_warp, const GraphView& g, int cap, int vsize,
-                                          Dist& de, WarpList& wl, SelBuf& sel) {
+                                          Dist& de, BuildList& wl, SelBuf& sel) {
   unsigned char* mine = smem + (size_t)(threadIdx.x >> 5) * per_warp;
   const VecTable tab = make_table(g);
   de.init(tab, mine);
   mine += Dist::smem_bytes(g.d);
   wl.bind(mine, cap, vsize, g.n);
-  mine += WarpList::smem_bytes(cap, vsize, g.n);
+  mine += BuildList::smem_bytes(cap, vsize, g.n);
   sel.bind(mine);
 }
 
 template <class Dist>
 __host__ __device__ inline size_t build_smem_per_warp(int d, int cap, int vsize, long long n) {
-  return (Dist::smem_bytes(d) + WarpList::smem_bytes(cap, vsize, n) + SelBuf::smem_bytes() + 15) / 16 * 16;
+  return (Dist::smem_bytes(d) + BuildList::smem_bytes(cap, vsize, n) + SelBuf::smem_bytes() + 15) / 16 * 16;
 }
 
 // ---------------------------------------------------------------------------
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32) init_level_kernel(InitParams
   const int lane = threadIdx.x & 31;
   const BuildLevel& L = p.L;
   Dist de;
-  WarpList wl;
+  BuildList wl;
   SelBuf sel;
   bind_warp(smem, p.per_warp, L.g, 32, 32, de, wl, sel);
   WalkCounters wc{0, 0, 0, 0};
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_s
   const int lane = threadIdx.x & 31;
   const BuildLevel& L = p.L;
   Dist de;
-  WarpList wl;
+  BuildList wl;
   SelBuf sel;
   bind_warp(smem, p.per_warp, L.g, p.cap, L.vsize, de, wl, sel);
   // the shared-memory block is laid out for p.cap keys (at least a full row plus one, which the
@@ -458,7 +459,7 @@ __global__ void __launch_bounds__(kBuildWarps * 32, Dist::kBuildMinCtas) build_r
   const int lane = threadIdx.x & 31;
   const BuildLevel& L = p.L;
   Dist de;
-  WarpList wl;
+  BuildList wl;
   SelBuf sel;
   bind_warp(smem, p.per_warp, L.g, p.cap, 32, de, wl, sel);
   WalkCounters wc{0, 0, 0, 0};

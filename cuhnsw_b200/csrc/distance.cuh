@@ -23,6 +23,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "smem.cuh"
 
@@ -153,6 +155,8 @@ struct DistSmall {
   // rows of 128 floats are 15 % slower there (1 M x 128: 0.477 against 0.415 s)
   static constexpr int kBuildMinCtas = C <= 3 ? 16 : 12;
   static constexpr int kWarpsPerSmTarget = 32;
+  // visited table of the search with one warp per query: two tags per bucket or four (figures in beam.cuh)
+  static constexpr bool kTwoTags = C == 3 && std::is_same<Row, RowF32>::value;
   static constexpr int kTeamMinCtas = 5;  // construction with one CTA of four warps per node
   static constexpr bool kDeepPool = C <= 3;    // eval_pool with two eights of rows under way without spills
   static constexpr bool kSharedQuery = false;  // every warp keeps its own copy of the query
@@ -298,6 +302,7 @@ struct DistLargeT {
   static constexpr int kSearchMinCtas = kMinCtasT;
   static constexpr int kBuildMinCtas = 8;
   static constexpr int kWarpsPerSmTarget = 16;
+  static constexpr bool kTwoTags = true;
   static constexpr int kTeamMinCtas = 4;
   static constexpr bool kDeepPool = false;
   static constexpr bool kSharedQuery = true;   // one copy in shared memory

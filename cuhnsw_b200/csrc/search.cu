@@ -22,7 +22,7 @@ constexpr int kWarpsPerCta = 2;
 // kEntries: the batch has been scheduled, every query's descent has ended at entry_node / entry_dist.  An instance of its
 // own because the walk is cheaper without the descent beside it: 315 against 367 warp instructions per expansion by the
 // counters (20 000 queries, 600 000 x 50, ef 200: 1.76 against 1.94 ms).
-template <class Dist, bool kReverse, bool kEntries>
+template <class Dist, class Table, bool kReverse, bool kEntries>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, Dist::kSearchMinCtas)
 knn_search_kernel(SearchParams p) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -31,7 +31,7 @@ knn_search_kernel(SearchParams p) {
   Dist de;
   const VecTable tab = make_table(p.g);
   de.init(tab, mine);
-  WarpList wl;
+  WarpList<Table> wl;
   wl.bind(mine + Dist::smem_bytes(p.g.d), p.ef, p.vsize, p.g.n);
   WalkCounters wc{0, 0, 0, 0};
 
@@ -199,15 +199,21 @@ cudaError_t schedule_search(SearchParams& p, const SearchSchedule& s, cudaStream
   return cudaSuccess;
 }
 
-template <class Dist, bool kReverse>
+template <class Dist, class Table, bool kReverse>
 static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaStream_t stream,
                                     const SearchSchedule* sched);
 
+template <class Dist, class Table>
+static cudaError_t launch_search_tt(const SearchParams& p0, int sm_count, cudaStream_t stream,
+                                    const SearchSchedule* sched) {
+  return p0.reverse_cand ? launch_search_tr<Dist, Table, true>(p0, sm_count, stream, sched)
+                         : launch_search_tr<Dist, Table, false>(p0, sm_count, stream, sched);
+}
+
 template <class Dist>
-static cudaError_t launch_search_t(const SearchParams& p0, int sm_count, cudaStream_t stream,
-                                   const SearchSchedule* sched) {
-  return p0.reverse_cand ? launch_search_tr<Dist, true>(p0, sm_count, stream, sched)
-                         : launch_search_tr<Dist, false>(p0, sm_count, stream, sched);
+static cudaError_t launch_search_t(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
+  using Table = std::conditional_t<Dist::kTwoTags, VisitedPairs, VisitedTable>;
+  return launch_search_tt<Dist, Table>(p, sm_count, stream, sched);
 }
 
 // CTAs of a search kernel that an SM holds
@@ -218,16 +224,16 @@ static cudaError_t residents(K kern, size_t smem, int* per_sm) {
   return e != cudaSuccess ? e : *per_sm < 1 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }
 
-template <class Dist, bool kReverse>
+template <class Dist, class Table, bool kReverse>
 static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaStream_t stream,
                                     const SearchSchedule* sched) {
   SearchParams p = p0;
-  size_t per_warp = Dist::smem_bytes(p.g.d) + WarpList::smem_bytes(p.ef, p.vsize, p.g.n);
+  size_t per_warp = Dist::smem_bytes(p.g.d) + WarpList<Table>::smem_bytes(p.ef, p.vsize, p.g.n);
   per_warp = (per_warp + 15) / 16 * 16;
   p.smem_per_warp = (int)per_warp;
   size_t smem = per_warp * kWarpsPerCta;
   int per_sm = 0;
-  cudaError_t e = residents(knn_search_kernel<Dist, kReverse, false>, smem, &per_sm);
+  cudaError_t e = residents(knn_search_kernel<Dist, Table, kReverse, false>, smem, &per_sm);
   if (e != cudaSuccess) return e;
   const long long want = (p.nq + kWarpsPerCta - 1) / kWarpsPerCta;
   long long grid = std::max(1ll, std::min((long long)per_sm * sm_count, want));
@@ -237,19 +243,20 @@ static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaSt
   if (sched && p.nq > grid * kWarpsPerCta && p.nq <= sched->capacity && p.nq <= 0x7fffffffll) {
     e = schedule_search(p, *sched, stream);
     if (e != cudaSuccess) return e;
-    e = residents(knn_search_kernel<Dist, kReverse, true>, smem, &per_sm);
+    e = residents(knn_search_kernel<Dist, Table, kReverse, true>, smem, &per_sm);
     if (e != cudaSuccess) return e;
     grid = std::max(1ll, std::min((long long)per_sm * sm_count, want));
-    knn_search_kernel<Dist, kReverse, true><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
+    knn_search_kernel<Dist, Table, kReverse, true><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
   } else {
-    knn_search_kernel<Dist, kReverse, false><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
+    knn_search_kernel<Dist, Table, kReverse, false><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
   }
   return cudaGetLastError();
 }
 
+// (the larger table: fp32 rows of 65 to 96 values and rows above 128 may do with half of that)
 size_t search_smem_per_cta(int d, int ef, int vsize, long long n) {
   size_t dq = d <= 128 ? 0 : DistLarge::smem_bytes(d);
-  size_t per_warp = (dq + WarpList::smem_bytes(ef, vsize, n) + 15) / 16 * 16;
+  size_t per_warp = (dq + WarpList<VisitedTable>::smem_bytes(ef, vsize, n) + 15) / 16 * 16;
   return per_warp * kWarpsPerCta;
 }
 

@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(32) selftest_list_kernel(int cap, const float*
                                                            unsigned long long* out_keys, int* out_size,
                                                            int* out_minpos, int* out_cursor) {
   extern __shared__ __align__(16) unsigned char smem[];
-  WarpList wl;
+  WarpList<VisitedTable> wl;
   wl.bind(smem, cap, 64, 1 << 20);
   wl.reset();
   WalkCounters wc{0, 0, 0, 0};
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(32) selftest_list_kernel(int cap, const float*
 __global__ void __launch_bounds__(32) selftest_visited_kernel(int entries, long long n, const int* ids, int count,
                                                               int* seen) {
   extern __shared__ __align__(16) unsigned char smem[];
-  WarpList wl;
+  WarpList<VisitedTable> wl;
   wl.bind(smem, 32, entries, n);
   wl.reset();
   if (lane_id() == 0)
@@ -76,7 +76,7 @@ struct Mirror {
 cudaError_t launch_selftest_list(int cap, const float* dist, const int* ids, const int* batch_begin, int nbatches,
                                  const int* expand, unsigned long long* out_keys, int* out_size, int* out_minpos,
                                  int* out_cursor, cudaStream_t stream) {
-  const size_t smem = WarpList::smem_bytes(cap, 64, 1 << 20);
+  const size_t smem = WarpList<VisitedTable>::smem_bytes(cap, 64, 1 << 20);
   cudaError_t e = cudaFuncSetAttribute(selftest_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   selftest_list_kernel<<<1, 32, smem, stream>>>(cap, dist, ids, batch_begin, nbatches, expand, out_keys, out_size,
@@ -86,7 +86,7 @@ cudaError_t launch_selftest_list(int cap, const float* dist, const int* ids, con
 
 cudaError_t launch_selftest_visited(int entries, long long n, const int* ids, int count, int* seen,
                                     cudaStream_t stream) {
-  const size_t smem = WarpList::smem_bytes(32, entries, n);
+  const size_t smem = WarpList<VisitedTable>::smem_bytes(32, entries, n);
   cudaError_t e =
       cudaFuncSetAttribute(selftest_visited_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
