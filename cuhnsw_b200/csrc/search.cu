@@ -210,10 +210,16 @@ static cudaError_t launch_search_tt(const SearchParams& p0, int sm_count, cudaSt
                          : launch_search_tr<Dist, Table, false>(p0, sm_count, stream, sched);
 }
 
+// Which visited table: by row type (Dist::kTwoTags), but two tags per bucket also where four would need 32 bits each and two do
+// not: one factor of two of the number of rows, 16.8 to 33.5 M with 2048 entries, whose 4 KB would hold 1024.  17 M x 16, 10 000
+// queries, ef 200 and 300, and 40 000, ef 200: 1.35, 1.94 and 3.81 ms with 1024 entries of 32 bits, 1.31, 1.86 and 3.68 so.
 template <class Dist>
 static cudaError_t launch_search_t(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
-  using Table = std::conditional_t<Dist::kTwoTags, VisitedPairs, VisitedTable>;
-  return launch_search_tt<Dist, Table>(p, sm_count, stream, sched);
+  if constexpr (!Dist::kTwoTags) {
+    if (!VisitedTable::needs_wide(p.vsize, p.g.n) || VisitedPairs::needs_wide(p.vsize, p.g.n))
+      return launch_search_tt<Dist, VisitedTable>(p, sm_count, stream, sched);
+  }
+  return launch_search_tt<Dist, VisitedPairs>(p, sm_count, stream, sched);
 }
 
 // CTAs of a search kernel that an SM holds
@@ -253,10 +259,10 @@ static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaSt
   return cudaGetLastError();
 }
 
-// (the larger table: fp32 rows of 65 to 96 values and rows above 128 may do with half of that)
+// (the same for both tables where one of them is chosen: 16 bits per entry if two tags per bucket can do with that, else 32)
 size_t search_smem_per_cta(int d, int ef, int vsize, long long n) {
   size_t dq = d <= 128 ? 0 : DistLarge::smem_bytes(d);
-  size_t per_warp = (dq + WarpList<VisitedTable>::smem_bytes(ef, vsize, n) + 15) / 16 * 16;
+  size_t per_warp = (dq + WarpList<VisitedPairs>::smem_bytes(ef, vsize, n) + 15) / 16 * 16;
   return per_warp * kWarpsPerCta;
 }
 
