@@ -236,7 +236,11 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
 constexpr int kShortWalk = 100;      // largest ef of a short walk
 constexpr int kRoundsFrom = 32;      // smallest ef of few walks on a frontier
 constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
-template <class Dist, int kCtas>
+// kCtas: how many CTAs of four warps on a list an SM is to hold, said to the compiler, whose own count of registers moves with
+// every change around it: seven of rows up to 64 values, six of up to 96.  ms, so / as it came out: 1000 queries of 200 000 x 32, ef 64
+// and 100, 0.219 / 0.264 and 0.301 / 0.346 (six CTAs); 3000 of 300 000 x 64, ef 128 and 180, 0.588 / 0.625 and 0.714 / 0.764 (72 registers, six in
+// shared memory); 2000 of 300 000 x 96, ef 100 and 128, 0.521 / 0.607 and 0.569 / 0.636 (five).
+template <class Dist, int kCtas, int kFrontierCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   if (p.ef >= kRoundsFrom) {
     if (p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
@@ -244,7 +248,7 @@ cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t
   }
   if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, kCtas>(p, 8192, sm_count, stream, sched);
   if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14)
-    return launch_frontier_t<Dist, 4, 8, kCtas>(p, 8192, sm_count, stream, sched);
+    return launch_frontier_t<Dist, 4, 8, kFrontierCtas>(p, 8192, sm_count, stream, sched);
   if (p.nq <= (long long)sm_count * 27) return launch_walk_t<Dist, 4, 8, kCtas>(p, 8192, sm_count, stream, sched);
   return launch_walk_t<Dist, 2, 8, 10>(p, 8192, sm_count, stream, sched);
 }
@@ -270,10 +274,10 @@ template <class Row>
 cudaError_t launch_search_walk(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   using E = Pick<Row>;
   const int d = p.g.d;
-  if (d <= 32) return launch_walk_narrow<typename E::D32, 6>(p, sm_count, stream, sched);
-  if (d <= 64) return launch_walk_narrow<typename E::D64, 6>(p, sm_count, stream, sched);
-  if (d <= 96) return launch_walk_narrow<typename E::D96, 5>(p, sm_count, stream, sched);
-  if (d <= 128) return launch_walk_narrow<typename E::D128, 5>(p, sm_count, stream, sched);
+  if (d <= 32) return launch_walk_narrow<typename E::D32, 7, 6>(p, sm_count, stream, sched);
+  if (d <= 64) return launch_walk_narrow<typename E::D64, 7, 6>(p, sm_count, stream, sched);
+  if (d <= 96) return launch_walk_narrow<typename E::D96, 6, 5>(p, sm_count, stream, sched);
+  if (d <= 128) return launch_walk_narrow<typename E::D128, 5, 5>(p, sm_count, stream, sched);
   // a warp gets one to five rows of a round: two rows of eight columns in flight bring a 3840-byte row in one round trip;
   // rows of up to four columns have nothing for the other four to load (300 000 x 300: 0.62 against 0.73 ms)
   if (d <= 512) return launch_walk_wide<typename E::Wide>(p, sm_count, stream, sched);
