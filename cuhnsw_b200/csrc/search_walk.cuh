@@ -20,9 +20,6 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_walk_kernel(SearchParams
   walk.de.init(make_table(p.g), smem);
   walk.bind(smem + Dist::smem_bytes(p.g.d), p.ef, p.g.stride0, p.vsize, p.g.n);
   walk.rows = p.g.rows0;
-  walk.upper_base = p.g.upper_base;
-  walk.level = 0;
-  walk.self = -1;
   if (threadIdx.x >= 32) {
     walk.help(p.queries);
     return;
@@ -35,7 +32,7 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_walk_kernel(SearchParams
       if (__any_sync(FULL, qi >= p.nq)) break;
     }
     if (p.order) qi = __ldg(p.order + qi);
-    walk.start(kWalkQuery, p.queries, qi);
+    walk.start(p.queries, qi);
     int cur;
     float dcur;
     if (p.entry_node) {

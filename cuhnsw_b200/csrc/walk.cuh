@@ -63,13 +63,6 @@ struct KeyList {
     __syncwarp();
     load_worst();
   }
-  __device__ __forceinline__ void clear() {
-    for (int i = lane; i < (cap + 2) / 2; i += 32) sts128(keys + 16 * i, ~0u, ~0u, ~0u, ~0u);
-    size = 0;
-    cursor = 0;
-    worst = make_uint2(~0u, ~0u);
-    __syncwarp();
-  }
 
   // Merges the g <= 32 keys at `group` (overwritten up to the next multiple of four), keeping the ef smallest; keys
   // that are listed already or come twice enter once.
@@ -201,6 +194,7 @@ struct WalkBoard {
   static constexpr int kReq = kCount + 4 * P;     // P + 1 selected keys
   static constexpr int kBytes = (kReq + 8 * (P + 1) + 15) / 16 * 16;
 };
+// (the last two in frontier_walk.cuh only)
 enum { kWalkOver = 0, kWalkQuery = 1, kWalkRound = 2, kWalkRows = 3, kWalkNode = 4, kWalkSelect = 5 };
 
 template <class Dist, int W, int P>
@@ -215,9 +209,8 @@ struct Walk {
   unsigned found;  // shared-memory address of kBuffers x stride keys: the prepared nodes' new neighbours
   unsigned pool;   // of the rows to evaluate: (id, address of the key's place in `found`)
   unsigned board;
-  const int* rows;  // adjacency table of the searched layer
-  const int* upper_base;
-  int stride, level, self;  // ints per adjacency row (= keys per buffer); node to leave out, or -1
+  const int* rows;  // adjacency table of layer 0
+  int stride;       // ints per adjacency row (= keys per buffer)
   int lane;
   WalkCounters wc;
 
@@ -242,7 +235,7 @@ struct Walk {
   // a word of the board, known to be the same in every lane
   __device__ __forceinline__ int posted(int at) const { return __shfl_sync(FULL, (int)lds32(board + at), 0); }
   __device__ __forceinline__ const int* row_of(int id) const {
-    return rows + row_index(upper_base, level, id) * stride;
+    return rows + (size_t)id * stride;
   }
 
   // ---- parts every warp of the walk takes ----
@@ -266,7 +259,7 @@ struct Walk {
       for (int i = 0; i < N; ++i) {
         if (i < count) {
           const bool known = vis.knows(nid[i]);
-          const bool fresh = slot && nid[i] >= 0 && nid[i] != self && !known;
+          const bool fresh = slot && nid[i] >= 0 && !known;
           const unsigned m = __ballot_sync(FULL, fresh);
           const int before = __popc(m & list.lower);
           int at = 0;
@@ -298,17 +291,15 @@ struct Walk {
       if (i < count && lane == 0) sts32(board + Board::kCount + 4 * (w + W * i), (unsigned)have[i]);
   }
 
-  // Warps 1 .. W - 1: every operation starts and ends at a block barrier, as warp 0's do.  Returns, behind its first
-  // barrier, the first operation that is not the walk's own.
-  __device__ __forceinline__ int help(const float* queries) {
+  // Warps 1 .. W - 1: every operation starts and ends at a block barrier, as warp 0's do.
+  __device__ __forceinline__ void help(const float* queries) {
     const int w = warp();
     for (;;) {
       __syncthreads();
       const int op = posted(Board::kOp);
-      if (op == kWalkOver || op == kWalkSelect) return op;
-      if (op == kWalkQuery || op == kWalkNode) {
-        if (!Dist::kSharedQuery) load(op, queries);
-        if (op == kWalkNode) self = posted(Board::kQuery);
+      if (op == kWalkOver) return;
+      if (op == kWalkQuery) {
+        if (!Dist::kSharedQuery) load(queries);
         vis.clear(w, W);
       } else {
         if (op == kWalkRound) {
@@ -320,11 +311,9 @@ struct Walk {
       __syncthreads();
     }
   }
-  // the query whose number is on the board, or the stored row
-  __device__ __forceinline__ void load(int op, const float* queries) {
-    const long long qi = (unsigned)posted(Board::kQuery);
-    if (op == kWalkQuery) de.load_query(queries + (size_t)qi * de.t.d);
-    else de.load_query_row((int)qi);
+  // the query whose number is on the board
+  __device__ __forceinline__ void load(const float* queries) {
+    de.load_query(queries + (size_t)(unsigned)posted(Board::kQuery) * de.t.d);
   }
 
   // ---- warp 0 ----
@@ -340,12 +329,11 @@ struct Walk {
     __syncthreads();
     wc.evals += n;
   }
-  // query `i` of `queries` (op kWalkQuery), or stored row i, which the walk then leaves out (kWalkNode)
-  __device__ __forceinline__ void start(int op, const float* queries, long long i) {
+  // query `i` of `queries`
+  __device__ __forceinline__ void start(const float* queries, long long i) {
     if (lane == 0) sts32(board + Board::kQuery, (unsigned)i);
-    post(op);
-    load(op, queries);
-    if (op == kWalkNode) self = (int)i;
+    post(kWalkQuery);
+    load(queries);
     vis.clear(0, W);
     __syncthreads();
   }
@@ -396,30 +384,6 @@ struct Walk {
   __device__ __forceinline__ void seed(int id, float dist) {
     list.seed(f2ord(dist), (unsigned)id);
     if (lane == 0) vis.test_and_set(id);
-    __syncwarp();
-  }
-
-  // list = the neighbours in an adjacency row of the searched layer
-  __device__ __forceinline__ void seed_row(const int* row) {
-    list.clear();
-    int n = 0;
-    for (int base = 0; base < stride; base += 32) {
-      const int nid = base + lane < stride ? __ldg(row + base + lane) : -1;
-      const bool on = nid >= 0 && nid != self;
-      const unsigned m = __ballot_sync(FULL, on);
-      const int at = n + __popc(m & list.lower);
-      if (on) sts64(pool + 8 * at, (unsigned)nid, found + 8 * at);
-      vis.test_and_set(nid, on);
-      n += __popc(m);
-    }
-    if (n == 0) return;
-    evaluate_rows(n);
-    for (int i = lane; i < n; i += 32) {
-      const uint2 k = lds64(found + 8 * i);
-      sts64(pool + 8 * i, k.x, 2 * k.y);
-    }
-    __syncwarp();
-    for (int base = 0; base < n; base += 32) list.merge(pool + 8 * base, min(32, n - base));
     __syncwarp();
   }
 
