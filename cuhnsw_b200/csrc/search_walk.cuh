@@ -231,7 +231,12 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
 // 300 000 x 64 f16 0.43 / 0.36, 0.49 / 0.42, 0.58 / 0.56, ef 400 0.95 / 0.83; of 1 M x 128 whole numbers 0.84 / 0.83, 0.95 / 0.95, 1.12 / 1.08, 1.92 /
 // 1.94 (4000: 1.95 / 2.20); 1000 of 50 000 x 40, ef 700 1.20 / 0.80; rows of up to 32 values 0.515 / 0.595 at 2000, ef 200.
 constexpr int kShortWalk = 100;      // largest ef of a short walk
-constexpr int kRoundsFrom = 32;      // smallest ef of few walks on a frontier
+// Smallest ef on a frontier of up to one query per SM, of up to three, and of up to three of fp32 rows above 64 values, whose
+// evaluations a list's other warps share as well.  Time on the list over that on the frontier at ef 32, 40, 48, 56, 64, 80:
+//   148 queries: 200 000 x 50 with 24 links 1.00 1.06 1.07 1.10 1.15 1.25, with 64 links 0.94 1.04 1.11 1.08 1.10 1.17; 300 000 x 96 f16 0.92
+//   1.05 1.03 1.00 1.05 1.15; 300 000 x 128 whole numbers 1.01 1.02 1.03 1.05 1.05 1.10 (one query of them 0.95 0.97 0.95 0.98 1.01 1.05).
+//   444: 0.96 1.01 1.00 1.01 1.12 1.17, 0.98 1.09 1.09 1.09 1.12 1.16; 0.96 0.99 1.07 1.08 1.08 1.13; 0.88 0.89 0.93 0.93 0.99 1.02.
+constexpr int kFewFrom = 48, kSomeFrom = 56, kSomeFromLong = 80;
 constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 // kCtas: how many CTAs of four warps on a list an SM is to hold, said to the compiler, whose own count of registers moves with
 // every change around it: seven of rows up to 64 values, six of up to 96.  ms, so / as it came out: 1000 queries of 200 000 x 32, ef 64
@@ -239,10 +244,9 @@ constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 // shared memory); 2000 of 300 000 x 96, ef 100 and 128, 0.521 / 0.607 and 0.569 / 0.636 (five).
 template <class Dist, int kCtas, int kFrontierCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
-  if (p.ef >= kRoundsFrom) {
-    if (p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
-    if (p.nq <= (long long)sm_count * 3) return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
-  }
+  if (p.ef >= kFewFrom && p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
+  if (p.ef >= (p.g.d > 64 && !p.g.rows16 ? kSomeFromLong : kSomeFrom) && p.nq > sm_count && p.nq <= (long long)sm_count * 3)
+    return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
   if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, kCtas>(p, 8192, sm_count, stream, sched);
   if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14)
     return launch_frontier_t<Dist, 4, 8, kFrontierCtas>(p, 8192, sm_count, stream, sched);

@@ -39,3 +39,36 @@ def test_frontier_equals_the_oracle(d, max_m0, dist_type, values, table):
     assert (got[0] == want[0]).all() and (got[2] == want[2]).all(), (nq, ef)
     assert_same_bits(got[1], want[1])
     assert stats["expansions"] == int(want[3][:, 1].sum()) and stats["sweeps"] == int(want[3][:, 2].sum()), (nq, ef)
+
+
+def _index(base, opt):
+  eng = CuHNSW(engine_options(opt))
+  eng.set_data(base)
+  eng.build()
+  return eng, oracle_graph_of(eng, base, opt)
+
+
+def _equal(got, want, label):
+  assert (got[0] == want[0]).all() and (got[2] == want[2]).all(), label
+  assert_same_bits(got[1], want[1])
+
+
+@pytest.mark.parametrize("d,row", [(40, "f32"), (70, "f32"), (70, "f16"), (140, "f32")])
+def test_list_and_frontier_around_the_lines(d, row):
+  """The smallest lists that are walked on a frontier, and tables whose size the shared memory decides: a number of buckets
+  that is no power of two (three CTAs per SM at ef 6000, six or five at ef 2000)."""
+  import torch
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  rng = np.random.default_rng(d)
+  n = 9000
+  base = rng.integers(-9, 10, (n, d)).astype(np.float32)
+  opt = dict(dist_type="l2", max_m=16, max_m0=64, ef_construction=64, seed=6, search_team=1, row_dtype=row)
+  eng, g = _index(base, opt)
+  q = (base[rng.integers(0, n, 7 * sms)] + rng.integers(-1, 2, (7 * sms, d))).astype(np.float32)
+  few = 24
+  for nq, ef, topk in ((sms, 47, 10), (sms, 48, 10), (sms + 1, 55, 10), (sms + 1, 56, 10), (sms + 1, 79, 10),
+                       (sms + 1, 80, 10), (sms, 100, 10), (sms, 101, 10), (sms + 1, 6000, 100), (2 * sms + 1, 6000, 100),
+                       (7 * sms, 2000, 10), (7 * sms, 199, 10), (7 * sms, 200, 10), (7 * sms, 249, 10), (7 * sms, 250, 10)):
+    got = eng.search_knn(q[:nq], topk, ef)
+    at = np.r_[:few, nq - few:nq]
+    _equal([part[at] for part in got], oracle.search(g, q[at], topk, ef), (nq, ef))
