@@ -646,6 +646,12 @@ int Engine::SearchGraphDevice(const float* d_q, long long nq, int topk, int ef, 
   // below the smallest wave there is nothing to prepare
   const bool schedule = nq > (long long)sm_count_ * 2 && opt_.search_schedule;
   if (schedule && (rc = PrepareSchedule(nq, lane, &sched)) != kOk) return rc;
+  // A program that searches on several streams has their searches run side by side: those that came since the last one
+  // of this lane count as doing so.
+  for (int i = 0; i < kSearchLanes; ++i)
+    if (&lanes_[i] != lane && lanes_[i].searched > lane->searched) p.beside += lanes_[i].queries;
+  lane->searched = ++searches_;
+  lane->queries = nq;
   CU(launch_search(p, sm_count_, stream_, schedule ? &sched : nullptr));
   return MarkLane(lane);
 }

@@ -216,6 +216,8 @@ class Engine {
     unsigned long long stamp = 0;
     cudaEvent_t done = nullptr;  // recorded behind the last thing a search put on the stream
     bool pending = false;
+    unsigned long long searched = 0;  // number of the last search, and its queries
+    long long queries = 0;
     DevBuf<unsigned> sched;
     DevBuf<unsigned char> sched_tmp;
     long long capacity = 0;
@@ -230,7 +232,7 @@ class Engine {
   static constexpr int kSearchLanes = 8;  // for the caller's streams
   static constexpr int kPieces = 4;       // pieces of one large host-buffer search in flight, with sets of their own
   SearchLane lanes_[kSearchLanes + kPieces];
-  unsigned long long lane_clock_ = 0;
+  unsigned long long lane_clock_ = 0, searches_ = 0;
   int LaneFor(cudaStream_t stream, SearchLane** lane);
   int MarkLane(SearchLane* lane);  // records `done` on the engine's stream
   // host-buffer search through page-locked staging; *handled = false: the size or the buffers ask for another way

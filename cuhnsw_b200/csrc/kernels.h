@@ -28,6 +28,7 @@ struct SearchParams {
   GraphView g;
   const float* queries;  // nq x d, unpadded
   long long nq;
+  long long beside = 0;  // queries of the searches on other streams that this one runs beside, as far as the engine can tell
   int topk;
   int ef;
   int vsize;             // visited table entries per warp (power of two); one CTA per query: chosen by its launcher, like

@@ -238,17 +238,25 @@ constexpr int kShortWalk = 100;      // largest ef of a short walk
 //   444: 0.96 1.01 1.00 1.01 1.12 1.17, 0.98 1.09 1.09 1.09 1.12 1.16; 0.96 0.99 1.07 1.08 1.08 1.13; 0.88 0.89 0.93 0.93 0.99 1.02.
 constexpr int kFewFrom = 48, kSomeFrom = 56, kSomeFromLong = 80;
 constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
+// The walks that count are those of the searches that take turns with this one on other streams as well (p.beside): a CTA of 16
+// warps fills the registers of an SM, three of eight warps do, and what comes next waits.  32 batches through four streams, ms, by
+// the batch alone / by all: 1.18 M x 50, 148 queries each, ef 64 and 200: 3.25 / 1.97 and 5.00 / 3.52; 444: 3.33 / 2.53 and 5.73 / 4.90; 300 000 x 96
+// f16, 148: 2.95 / 1.54 and 4.50 / 2.66.  Four or more that take turns keep the chip full either way, so three CTAs of eight warps
+// do up to seven per SM (10 batches of 148, 200 and 250 of 1.18 M x 50, ef 100: 1.12, 1.11 and 1.13 times as fast as on the list; of 300 1.05, and
+// 0.9 to 1.0 at ef 60 on other tables); three batches of 200 at once do not fit (0.90).  Known loss: 100 queries of 128 floats each, ef 200 and 350, take 1.09 and 1.21 times what 16 warps took.
 // kCtas: how many CTAs of four warps on a list an SM is to hold, said to the compiler, whose own count of registers moves with
 // every change around it: seven of rows up to 64 values, six of up to 96.  ms, so / as it came out: 1000 queries of 200 000 x 32, ef 64
 // and 100, 0.219 / 0.264 and 0.301 / 0.346 (six CTAs); 3000 of 300 000 x 64, ef 128 and 180, 0.588 / 0.625 and 0.714 / 0.764 (72 registers, six in
 // shared memory); 2000 of 300 000 x 96, ef 100 and 128, 0.521 / 0.607 and 0.569 / 0.636 (five).
 template <class Dist, int kCtas, int kFrontierCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
-  if (p.ef >= kFewFrom && p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
-  if (p.ef >= (p.g.d > 64 && !p.g.rows16 ? kSomeFromLong : kSomeFrom) && p.nq > sm_count && p.nq <= (long long)sm_count * 3)
+  const long long walks = p.nq + p.beside;
+  if (p.ef >= kFewFrom && walks <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
+  const bool some = walks <= (long long)sm_count * 3 || (p.beside >= 3 * p.nq && walks <= (long long)sm_count * 7);
+  if (p.ef >= (p.g.d > 64 && !p.g.rows16 ? kSomeFromLong : kSomeFrom) && walks > sm_count && some)
     return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
   if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, kCtas>(p, 8192, sm_count, stream, sched);
-  if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14)
+  if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14 && walks <= (long long)sm_count * 20)
     return launch_frontier_t<Dist, 4, 8, kFrontierCtas>(p, 8192, sm_count, stream, sched);
   if (p.nq <= (long long)sm_count * 27) return launch_walk_t<Dist, 4, 8, kCtas>(p, 8192, sm_count, stream, sched);
   return launch_walk_t<Dist, 2, 8, 10>(p, 8192, sm_count, stream, sched);
@@ -260,7 +268,8 @@ cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t
 template <class Dist>
 cudaError_t launch_walk_wide(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   const bool brief = p.ef <= kShortWalk;
-  if (!brief && p.nq <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 16384, sm_count, stream, sched);
+  const long long walks = p.nq + p.beside;
+  if (!brief && walks <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 16384, sm_count, stream, sched);
   // while two CTAs of eight warps per SM hold all queries at once; further on four CTAs of four serve more (60 000 x 960, 2,
   // 3 and 4 queries per SM, four / eight warps: ef 100 1.21 1.06 0.94, ef 200 1.12 0.96 0.78, ef 400 1.12 0.92 0.73)
   if (p.nq <= (long long)sm_count * 2)

@@ -72,3 +72,39 @@ def test_list_and_frontier_around_the_lines(d, row):
     got = eng.search_knn(q[:nq], topk, ef)
     at = np.r_[:few, nq - few:nq]
     _equal([part[at] for part in got], oracle.search(g, q[at], topk, ef), (nq, ef))
+
+
+@pytest.mark.parametrize("d", [30, 200])
+def test_searches_in_turn_on_several_streams(d):
+  """Which kernel a small search gets depends on what the searches on other streams were; what it finds does not."""
+  import torch
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  rng = np.random.default_rng(d)
+  n, k = 6000, 10
+  base = rng.standard_normal((n, d)).astype(np.float32)
+  eng = CuHNSW(engine_options(dict(dist_type="l2", max_m=12, max_m0=24, ef_construction=64, seed=2)))
+  eng.set_data(base)
+  eng.build()
+  eng.obj.set_stream(torch.cuda.current_stream().cuda_stream)
+
+  def search(q, ef):
+    out = (torch.empty((len(q), k), dtype=torch.int32, device="cuda"), torch.empty((len(q), k), device="cuda"),
+           torch.empty((len(q),), dtype=torch.int32, device="cuda"))
+    eng.obj.search_knn_device(q.data_ptr(), len(q), k, ef, *(t.data_ptr() for t in out))
+    return out
+
+  q = torch.from_numpy(rng.standard_normal((6 * sms, d)).astype(np.float32)).cuda()
+  sizes = [1, 37, sms // 2, sms, sms + 1, 2 * sms, 3 * sms, 6 * sms]
+  alone = {(nq, ef): search(q[:nq], ef) for nq in sizes for ef in (40, 90, 300)}
+  torch.cuda.synchronize()
+  streams = [torch.cuda.Stream() for _ in range(10)]  # more than the engine keeps sets of scratch for
+  for ef in (40, 90, 300):
+    for count in (2, 4, 10):
+      for nq in sizes:
+        got = []
+        for i in range(2 * count):
+          eng.obj.set_stream(streams[i % count].cuda_stream)
+          got.append(search(q[:nq], ef))
+        torch.cuda.synchronize()
+        for out in got:
+          assert all(torch.equal(a, b) for a, b in zip(out, alone[nq, ef])), (ef, count, nq)
