@@ -253,10 +253,7 @@ struct WarpList : Table {
     worst = KEY_MAX;
   }
   // key i with its flag
-  __device__ __forceinline__ unsigned long long key(int i) const {
-    const uint2 w = lds64(keys + 8 * i);
-    return ((unsigned long long)w.y << 32) | w.x;
-  }
+  __device__ __forceinline__ unsigned long long key(int i) const { return key_at(keys, i); }
   __device__ __forceinline__ void set_key(int i, unsigned long long k) const {
     sts64(keys + 8 * i, (unsigned)k, (unsigned)(k >> 32));
   }
@@ -541,9 +538,8 @@ __device__ __forceinline__ void beam_layer(Dist& de, List& wl, const int* __rest
 
 // The adjacency rows of one layer, for a warp whose lanes read a slot each.
 struct LayerRows {
-  const char* mine;  // this lane's slot of row 0
-  unsigned bytes;    // of a row
-  int stride;        // slots
+  const int* mine;  // this lane's slot of row 0
+  int stride;       // slots
   const int* upper_base;
   int level;
   int lane;
@@ -551,16 +547,13 @@ struct LayerRows {
   __device__ __forceinline__ LayerRows() {}
   __device__ __forceinline__ LayerRows(const int* rows, int stride_, const int* upper_base_, int level_) {
     lane = lane_number();
-    mine = reinterpret_cast<const char*>(rows + lane);
-    bytes = 4u * (unsigned)stride_;
+    mine = rows + lane;
     stride = stride_;
     upper_base = upper_base_;
     level = level_;
   }
-  // (row numbers have 32 bits, so an address is one multiplication and addition)
   __device__ __forceinline__ const int* row(int id) const {
-    const unsigned r = level == 0 ? (unsigned)id : (unsigned)(__ldg(upper_base + id) + (level - 1));
-    return reinterpret_cast<const int*>(mine + (size_t)r * bytes);
+    return row_at(mine, row_number(upper_base, level, id), stride);
   }
   // slot base + lane of the row at p
   __device__ __forceinline__ int read(const int* p, int base) const {

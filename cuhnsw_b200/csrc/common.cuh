@@ -41,11 +41,4 @@ __device__ __forceinline__ unsigned long long shfl64(unsigned long long v, int s
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
-// Compacts the lanes selected by `mask`: lane r (r < popc(mask)) receives the
-// value held by the r-th selected lane, in lane order.
-__device__ __forceinline__ int compact_i32(unsigned mask, int v) {
-  int src = __fns(mask, 0, lane_id() + 1);
-  return __shfl_sync(FULL, v, src & 31);
-}
-
 }  // namespace hnsw

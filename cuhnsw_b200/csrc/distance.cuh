@@ -154,11 +154,9 @@ struct DistSmall {
   // (1.18 M x 50: 0.208 s against 0.222 s) and 2.5 % faster for 96 (2 M x 96: 0.310 against 0.318 s);
   // rows of 128 floats are 15 % slower there (1 M x 128: 0.477 against 0.415 s)
   static constexpr int kBuildMinCtas = C <= 3 ? 16 : 12;
-  static constexpr int kWarpsPerSmTarget = 32;
   // visited table of the search with one warp per query: two tags per bucket or four (figures in beam.cuh)
   static constexpr bool kTwoTags = C == 3 && std::is_same<Row, RowF32>::value;
   static constexpr int kTeamMinCtas = 5;  // construction with one CTA of four warps per node
-  static constexpr bool kDeepPool = C <= 3;    // eval_pool with two eights of rows under way without spills
   static constexpr bool kSharedQuery = false;  // every warp keeps its own copy of the query
   __host__ __device__ static constexpr size_t smem_bytes(int) { return 0; }
 
@@ -243,47 +241,32 @@ struct DistSmall {
   // (distance image, id) of a row go to its place, an address.  kLeast: the address has 24 bits, and the smallest image of the
   // rows with the same upper 8 bits b goes to word b at `least`.  A team takes two rows at a time, whose lane sums are folded together:
   // the first exchange of the butterfly leaves one row in each half of the team (the pairs that are added are the same, so
-  // are the sums), and eight rows cost 5 shuffles instead of the 16 of two passes of eval().  kPairs: such eights whose
-  // loads are issued together.
-  template <int kPairs, bool kLeast>
+  // are the sums), and eight rows cost 5 shuffles instead of the 16 of two passes of eval().
+  template <bool kLeast>
   __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps, unsigned least) {
-    if (t.dist_type == DIST_DOT) eval_pool_t<true, kPairs, kLeast>(pool, n, w, warps, least);
-    else eval_pool_t<false, kPairs, kLeast>(pool, n, w, warps, least);
+    if (t.dist_type == DIST_DOT) eval_pool_t<true, kLeast>(pool, n, w, warps, least);
+    else eval_pool_t<false, kLeast>(pool, n, w, warps, least);
   }
-  template <bool kDot, int kPairs, bool kLeast>
+  template <bool kDot, bool kLeast>
   __device__ __forceinline__ void eval_pool_t(unsigned pool, int n, int w, int warps, unsigned least) {
     const int team = lane_no >> 3, tl = lane_no & 7;
     const bool second = tl & 4;
-    for (int r0 = 8 * w; r0 < n; r0 += 8 * kPairs * warps) {
-      uint2 ea[kPairs], eb[kPairs];
-      float4 va[kPairs][C], vb[kPairs][C];
+    for (int r0 = 8 * w; r0 < n; r0 += 8 * warps) {
+      // rows past n are folded onto the last one: a harmless repeated load whose result nobody writes
+      const uint2 ea = lds64(pool + 8 * min(r0 + team, n - 1)), eb = lds64(pool + 8 * min(r0 + team + 4, n - 1));
+      float4 va[C], vb[C];
+      Row::template load<C, 8, true>(t.vec + (size_t)ea.x * t.row_bytes, tl, 0, t.nchunk, va);
+      Row::template load<C, 8, true>(t.vec + (size_t)eb.x * t.row_bytes, tl, 0, t.nchunk, vb);
+      float4 aa = first4<kDot>(q[0], va[0]), ab = first4<kDot>(q[0], vb[0]);
 #pragma unroll
-      for (int u = 0; u < kPairs; ++u) {
-        // rows past n are folded onto the last one: a harmless repeated load whose result nobody writes
-        const int ra = r0 + 8 * u * warps + team;
-        ea[u] = lds64(pool + 8 * min(ra, n - 1));
-        eb[u] = lds64(pool + 8 * min(ra + 4, n - 1));
+      for (int c = 1; c < C; ++c) {
+        fma4(aa, q[c], va[c], kDot ? DIST_DOT : DIST_L2);
+        fma4(ab, q[c], vb[c], kDot ? DIST_DOT : DIST_L2);
       }
-#pragma unroll
-      for (int u = 0; u < kPairs; ++u) {
-        if (u > 0 && r0 + 8 * u * warps >= n) break;  // warp-uniform
-        Row::template load<C, 8, true>(t.vec + (size_t)ea[u].x * t.row_bytes, tl, 0, t.nchunk, va[u]);
-        Row::template load<C, 8, true>(t.vec + (size_t)eb[u].x * t.row_bytes, tl, 0, t.nchunk, vb[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < kPairs; ++u) {
-        if (u > 0 && r0 + 8 * u * warps >= n) break;
-        float4 aa = first4<kDot>(q[0], va[u][0]), ab = first4<kDot>(q[0], vb[u][0]);
-#pragma unroll
-        for (int c = 1; c < C; ++c) {
-          fma4(aa, q[c], va[u][c], kDot ? DIST_DOT : DIST_L2);
-          fma4(ab, q[c], vb[u][c], kDot ? DIST_DOT : DIST_L2);
-        }
-        float s = fold_two(fold4(aa), fold4(ab));
-        if (kDot) s = -s;
-        const int r = r0 + 8 * u * warps + team + (second ? 4 : 0);
-        if ((tl & 3) == 0 && r < n) put_evaluated<kLeast>(second ? eb[u] : ea[u], s, least);
-      }
+      float s = fold_two(fold4(aa), fold4(ab));
+      if (kDot) s = -s;
+      const int r = r0 + team + (second ? 4 : 0);
+      if ((tl & 3) == 0 && r < n) put_evaluated<kLeast>(second ? eb : ea, s, least);
     }
   }
 };
@@ -301,10 +284,8 @@ struct DistLargeT {
   static constexpr int kChunks = kChunksT;    // chunk columns per row per step
   static constexpr int kSearchMinCtas = kMinCtasT;
   static constexpr int kBuildMinCtas = 8;
-  static constexpr int kWarpsPerSmTarget = 16;
   static constexpr bool kTwoTags = true;
   static constexpr int kTeamMinCtas = 4;
-  static constexpr bool kDeepPool = false;
   static constexpr bool kSharedQuery = true;   // one copy in shared memory
   __host__ __device__ static constexpr size_t smem_bytes(int d) { return (size_t)((d + 127) / 128) * 128 * sizeof(float); }
 
@@ -377,7 +358,7 @@ struct DistLargeT {
   }
   __device__ __forceinline__ float eval_eight(int id, int n) { return eval(id, n); }
   // The same, with rows w, w + warps, ... for warp w.
-  template <int, bool kLeast>
+  template <bool kLeast>
   __device__ __forceinline__ void eval_pool(unsigned pool, int n, int w, int warps, unsigned least) {
     const int lane = lane_id();
     for (int r0 = w; r0 < n; r0 += 32 * warps) {

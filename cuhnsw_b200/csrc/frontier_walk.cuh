@@ -35,7 +35,6 @@ template <class Dist, int W, int P>
 struct FrontierWalk {
   static constexpr int kBuffers = 2 * P;
   static_assert(W > 1 && kBuffers <= 32, "a lane stands for a buffer");
-  static constexpr int kPairs = W >= 8 && P >= 2 * W && Dist::kDeepPool ? 2 : 1;  // few queries: registers to spare
   // Front keys that are prepared.  More than P of them evaluate more for nothing (8 nodes, 1.33 evaluations for each distinct
   // row among the first 16, 1.26 among the first 8, in 6 % more rounds).
   static constexpr int kWindow = P > 8 ? 16 : P;
@@ -153,7 +152,7 @@ struct FrontierWalk {
           filter_posted(w, words);
           __syncthreads();
         }
-        de.template eval_pool<kPairs, true>(pool, posted(Board::kPool), w, W, board + Board::kLeast);
+        de.template eval_pool<true>(pool, posted(Board::kPool), w, W, board + Board::kLeast);
       }
       __syncthreads();
     }
@@ -174,7 +173,7 @@ struct FrontierWalk {
   __device__ __forceinline__ void evaluate_rows(int n) {
     if (lane == 0) sts32(board + Board::kPool, n);
     post(kWalkRows);
-    de.template eval_pool<kPairs, true>(pool, n, 0, W, board + Board::kLeast);
+    de.template eval_pool<true>(pool, n, 0, W, board + Board::kLeast);
     __syncthreads();
     wc.evals += n;
   }
@@ -331,7 +330,7 @@ struct FrontierWalk {
     filter_posted(0, board_words());
     __syncthreads();
     const int total = posted(Board::kPool);
-    de.template eval_pool<kPairs, true>(pool, total, 0, W, board + Board::kLeast);
+    de.template eval_pool<true>(pool, total, 0, W, board + Board::kLeast);
     __syncthreads();
     if (chosen) fr.tag = buffer | ((int)lds32(board + Board::kCount + 4 * rank) << kCountAt);
     wc.evals += total;

@@ -306,7 +306,7 @@ struct Walk {
           filter_posted(w);
           __syncthreads();
         }
-        de.template eval_pool<1, false>(pool, posted(Board::kPool), w, W, 0);
+        de.template eval_pool<false>(pool, posted(Board::kPool), w, W, 0);
       }
       __syncthreads();
     }
@@ -325,7 +325,7 @@ struct Walk {
   __device__ __forceinline__ void evaluate_rows(int n) {
     if (lane == 0) sts32(board + Board::kPool, n);
     post(kWalkRows);
-    de.template eval_pool<1, false>(pool, n, 0, W, 0);
+    de.template eval_pool<false>(pool, n, 0, W, 0);
     __syncthreads();
     wc.evals += n;
   }
@@ -482,7 +482,7 @@ struct Walk {
         filter_posted(0);
         __syncthreads();
         const int total = posted(Board::kPool);
-        de.template eval_pool<1, false>(pool, total, 0, W, 0);
+        de.template eval_pool<false>(pool, total, 0, W, 0);
         __syncthreads();
         if (chosen) mine.count = (int)lds32(board + Board::kCount + 4 * (lane - c));
         wc.evals += total;

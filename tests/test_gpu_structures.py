@@ -144,3 +144,25 @@ def test_visited_table_never_invents_and_keeps_the_recent(entries, n):
   # and it does remember: every id was offered while the table still had room for it
   again = [s for k, (v, s) in enumerate(zip(ids.tolist(), seen.tolist())) if k >= 1 and ids[k - 1] == v]
   assert len(again) > 100 and all(again)
+
+
+@pytest.mark.parametrize("entries,n", [(64, 1000), (64, 524_288), (64, 524_289), (128, 900_000), (1024, 1_183_514),
+                                       (2048, 16_777_216), (2048, 16_777_217), (4096, 2_000_000_000)])
+def test_visited_table_keeps_the_last_four_of_a_bucket(entries, n):
+  """The table against its model, id by id: entries / 4 buckets, whose number is the upper half of a product, each with the
+  last four ids that were new to it.  Tags of 16 and of 32 bits."""
+  lib = cuhnsw_bind.load_library()
+  rng = np.random.default_rng(entries + n)
+  pool = rng.integers(0, n, 3 * entries).astype(np.int64)
+  ids = pool[rng.integers(0, len(pool), 8000)].astype(np.int32)
+  seen = np.zeros(len(ids), np.int32)
+  assert lib.cuhnsw_selftest_visited(entries, n, ids.ctypes.data, len(ids), seen.ctypes.data) == 0
+  bits, buckets = max(1, int(n - 1).bit_length()), entries // 4
+  kept, want = {}, []
+  for v in ids.tolist():
+    bucket = kept.setdefault(((v * 2654435761 << (32 - bits)) % (1 << 32)) * buckets >> 32, [])
+    want.append(int(v in bucket))
+    if not want[-1]:
+      bucket.insert(0, v)
+      del bucket[4:]
+  assert 0 < sum(want) < len(want) and seen.tolist() == want
