@@ -154,8 +154,11 @@ struct DistSmall {
   // (1.18 M x 50: 0.208 s against 0.222 s) and 2.5 % faster for 96 (2 M x 96: 0.310 against 0.318 s);
   // rows of 128 floats are 15 % slower there (1 M x 128: 0.477 against 0.415 s)
   static constexpr int kBuildMinCtas = C <= 3 ? 16 : 12;
-  // visited table of the search with one warp per query: two tags per bucket or four (figures in beam.cuh)
+  // Visited table of the search with one warp per query: two tags per bucket or four (figures in beam.cuh); beside the descent, in
+  // batches that are not scheduled, two also for fp32 rows of 33 values and more (4000 and 4500 queries of 200 000 x 50, ef 100 and 64,
+  // four / two: 0.496 / 0.436 and 0.354 / 0.312 ms; 300 000 x 128 by 1.5 %; rows of up to 32 values and of 16 bits lose 1 to 2 %).
   static constexpr bool kTwoTags = C == 3 && std::is_same<Row, RowF32>::value;
+  static constexpr bool kTwoTagsInside = C >= 2 && std::is_same<Row, RowF32>::value;
   static constexpr int kTeamMinCtas = 5;  // construction with one CTA of four warps per node
   static constexpr bool kSharedQuery = false;  // every warp keeps its own copy of the query
   __host__ __device__ static constexpr size_t smem_bytes(int) { return 0; }
@@ -284,7 +287,7 @@ struct DistLargeT {
   static constexpr int kChunks = kChunksT;    // chunk columns per row per step
   static constexpr int kSearchMinCtas = kMinCtasT;
   static constexpr int kBuildMinCtas = 8;
-  static constexpr bool kTwoTags = true;
+  static constexpr bool kTwoTags = true, kTwoTagsInside = true;
   static constexpr int kTeamMinCtas = 4;
   static constexpr bool kSharedQuery = true;   // one copy in shared memory
   __host__ __device__ static constexpr size_t smem_bytes(int d) { return (size_t)((d + 127) / 128) * 128 * sizeof(float); }

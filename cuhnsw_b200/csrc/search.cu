@@ -210,7 +210,7 @@ static cudaError_t launch_search_tt(const SearchParams& p0, int sm_count, cudaSt
                          : launch_search_tr<Dist, Table, false>(p0, sm_count, stream, sched);
 }
 
-// Which visited table: by row type (Dist::kTwoTags), but two tags per bucket also where four would need 32 bits each and two do
+// Which visited table: by row type (Dist::kTwoTags, kTwoTagsInside), but two tags per bucket also where four would need 32 bits each and two do
 // not: one factor of two of the number of rows, 16.8 to 33.5 M with 2048 entries, whose 4 KB would hold 1024.  17 M x 16, 10 000
 // queries, ef 200 and 300, and 40 000, ef 200: 1.35, 1.94 and 3.81 ms with 1024 entries of 32 bits, 1.31, 1.86 and 3.68 so.
 template <class Dist>
@@ -234,12 +234,12 @@ template <class Dist, class Table, bool kReverse>
 static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaStream_t stream,
                                     const SearchSchedule* sched) {
   SearchParams p = p0;
-  size_t per_warp = Dist::smem_bytes(p.g.d) + WarpList<Table>::smem_bytes(p.ef, p.vsize, p.g.n);
-  per_warp = (per_warp + 15) / 16 * 16;
-  p.smem_per_warp = (int)per_warp;
-  size_t smem = per_warp * kWarpsPerCta;
+  const auto smem_of = [&](size_t list) { return (Dist::smem_bytes(p.g.d) + list + 15) / 16 * 16; };
+  using Inside = std::conditional_t<Dist::kTwoTagsInside, VisitedPairs, Table>;
+  p.smem_per_warp = (int)smem_of(WarpList<Inside>::smem_bytes(p.ef, p.vsize, p.g.n));
+  size_t smem = (size_t)p.smem_per_warp * kWarpsPerCta;
   int per_sm = 0;
-  cudaError_t e = residents(knn_search_kernel<Dist, Table, kReverse, false>, smem, &per_sm);
+  cudaError_t e = residents(knn_search_kernel<Dist, Inside, kReverse, false>, smem, &per_sm);
   if (e != cudaSuccess) return e;
   const long long want = (p.nq + kWarpsPerCta - 1) / kWarpsPerCta;
   long long grid = std::max(1ll, std::min((long long)per_sm * sm_count, want));
@@ -249,12 +249,14 @@ static cudaError_t launch_search_tr(const SearchParams& p0, int sm_count, cudaSt
   if (sched && p.nq > grid * kWarpsPerCta && p.nq <= sched->capacity && p.nq <= 0x7fffffffll) {
     e = schedule_search(p, *sched, stream);
     if (e != cudaSuccess) return e;
+    p.smem_per_warp = (int)smem_of(WarpList<Table>::smem_bytes(p.ef, p.vsize, p.g.n));
+    smem = (size_t)p.smem_per_warp * kWarpsPerCta;
     e = residents(knn_search_kernel<Dist, Table, kReverse, true>, smem, &per_sm);
     if (e != cudaSuccess) return e;
     grid = std::max(1ll, std::min((long long)per_sm * sm_count, want));
     knn_search_kernel<Dist, Table, kReverse, true><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
   } else {
-    knn_search_kernel<Dist, Table, kReverse, false><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
+    knn_search_kernel<Dist, Inside, kReverse, false><<<(unsigned)grid, kWarpsPerCta * 32, smem, stream>>>(p);
   }
   return cudaGetLastError();
 }
