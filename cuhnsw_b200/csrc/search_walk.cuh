@@ -231,19 +231,22 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
 // 300 000 x 64 f16 0.43 / 0.36, 0.49 / 0.42, 0.58 / 0.56, ef 400 0.95 / 0.83; of 1 M x 128 whole numbers 0.84 / 0.83, 0.95 / 0.95, 1.12 / 1.08, 1.92 /
 // 1.94 (4000: 1.95 / 2.20); 1000 of 50 000 x 40, ef 700 1.20 / 0.80; rows of up to 32 values 0.515 / 0.595 at 2000, ef 200.
 constexpr int kShortWalk = 100;      // largest ef of a short walk
-// Smallest ef on a frontier of up to one query per SM, of up to three, and of up to three of fp32 rows above 64 values, whose
+// Smallest ef on a frontier of up to one query per SM, of up to three, and the same of fp32 rows above 64 values, whose
 // evaluations a list's other warps share as well.  Time on the list over that on the frontier at ef 32, 40, 48, 56, 64, 80:
-//   148 queries: 200 000 x 50 with 24 links 1.00 1.06 1.07 1.10 1.15 1.25, with 64 links 0.94 1.04 1.11 1.08 1.10 1.17; 300 000 x 96 f16 0.92
-//   1.05 1.03 1.00 1.05 1.15; 300 000 x 128 whole numbers 1.01 1.02 1.03 1.05 1.05 1.10 (one query of them 0.95 0.97 0.95 0.98 1.01 1.05).
-//   444: 0.96 1.01 1.00 1.01 1.12 1.17, 0.98 1.09 1.09 1.09 1.12 1.16; 0.96 0.99 1.07 1.08 1.08 1.13; 0.88 0.89 0.93 0.93 0.99 1.02.
-constexpr int kFewFrom = 48, kSomeFrom = 56, kSomeFromLong = 80;
+//   one query: 200 000 x 50 with 24 links 1.00 1.05 1.09 1.08 1.09 1.13, with 64 links 1.02 1.06 1.08 1.14 1.19 1.27; 300 000 x 96 f16 0.96 0.99
+//   1.03 1.04 1.06 1.13; 300 000 x 128 whole numbers with 32 links 0.95 0.97 0.95 0.98 1.01 1.05, 200 000 with 48 1.01 1.10 1.11 1.16 1.22 1.25.
+//   148: 1.00 1.06 1.07 1.10 1.15 1.25, 0.94 1.04 1.11 1.08 1.10 1.17; 0.92 1.05 1.03 1.00 1.05 1.15; 1.01 1.02 1.03 1.05 1.05 1.10, 1.01 1.06 1.14 1.16
+//   1.15 1.21.
+//   444: 0.96 1.01 1.00 1.01 1.12 1.17, 0.98 1.09 1.09 1.09 1.12 1.16; 0.96 0.99 1.07 1.08 1.08 1.13; 0.88 0.89 0.93 0.93 0.99 1.02, 0.93 0.96 1.01 1.01 1.06
+//   1.11.
+constexpr int kFewFrom = 40, kSomeFrom = 40, kFewFromLong = 48, kSomeFromLong = 80;
 constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 // The walks that count are those of the searches that take turns with this one on other streams as well (p.beside): a CTA of 16
 // warps fills the registers of an SM, three of eight warps do, and what comes next waits.  32 batches through four streams, ms, by
 // the batch alone / by all: 1.18 M x 50, 148 queries each, ef 64 and 200: 3.25 / 1.97 and 5.00 / 3.52; 444: 3.33 / 2.53 and 5.73 / 4.90; 300 000 x 96
 // f16, 148: 2.95 / 1.54 and 4.50 / 2.66.  Four or more that take turns keep the chip full either way, so three CTAs of eight warps
-// do up to seven per SM (10 batches of 148, 200 and 250 of 1.18 M x 50, ef 100: 1.12, 1.11 and 1.13 times as fast as on the list; of 300 1.05, and
-// 0.9 to 1.0 at ef 60 on other tables); three batches of 200 at once do not fit (0.90).  Known loss: 100 queries of 128 floats each, ef 200 and 350, take 1.09 and 1.21 times what 16 warps took.
+// do up to six per SM (10 batches of 148 and 200 of 1.18 M x 50, ef 100: 1.12 and 1.11 times as fast as on the list, six and ten of 250 1.04 and 1.13, but
+// 0.91 to 0.94 at ef 60 and on 128 floats); three batches of 200 at once do not fit (0.90).  Known loss: 100 queries of 128 floats each, ef 200 and 350, take 1.09 and 1.21 times what 16 warps took.
 // kCtas: how many CTAs of four warps on a list an SM is to hold, said to the compiler, whose own count of registers moves with
 // every change around it: seven of rows up to 64 values, six of up to 96.  ms, so / as it came out: 1000 queries of 200 000 x 32, ef 64
 // and 100, 0.219 / 0.264 and 0.301 / 0.346 (six CTAs); 3000 of 300 000 x 64, ef 128 and 180, 0.588 / 0.625 and 0.714 / 0.764 (72 registers, six in
@@ -251,9 +254,11 @@ constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 template <class Dist, int kCtas, int kFrontierCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   const long long walks = p.nq + p.beside;
-  if (p.ef >= kFewFrom && walks <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
-  const bool some = walks <= (long long)sm_count * 3 || (p.beside >= 3 * p.nq && walks <= (long long)sm_count * 7);
-  if (p.ef >= (p.g.d > 64 && !p.g.rows16 ? kSomeFromLong : kSomeFrom) && walks > sm_count && some)
+  const bool long_rows = p.g.d > 64 && !p.g.rows16;
+  if (p.ef >= (long_rows ? kFewFromLong : kFewFrom) && walks <= sm_count)
+    return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
+  const bool some = walks <= (long long)sm_count * 3 || (p.beside >= 3 * p.nq && walks <= (long long)sm_count * 6);
+  if (p.ef >= (long_rows ? kSomeFromLong : kSomeFrom) && walks > sm_count && some)
     return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
   if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, kCtas>(p, 8192, sm_count, stream, sched);
   if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14 && walks <= (long long)sm_count * 20)
