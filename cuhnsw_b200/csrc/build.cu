@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps, Dist::kTeamMinCtas) build_sea
     walk.fr.sort_done();
     const int nc = min(walk.fr.done, L.ef_construction);
     if (lane == 0) sts32(walk.board + FrontierBoard<kTeamNodes>::kPool, nc);
-    walk.post(kWalkSelect);
+    walk.post(kWalkKeys);
     const int deg = select(nc);
     int* so = p.S.st_ids + (size_t)t * L.stride;
     float* sd = p.S.st_dist + (size_t)t * L.stride;

@@ -402,5 +402,25 @@ __device__ __forceinline__ void write_closest(const SearchParams& p, long long q
   if (fr.lane == 0) p.out_found[qi] = found;
   __syncwarp();
 }
+// The same by all warps of a CTA: each takes 32 of the `done` keys at a time and counts the smaller ones, which is a key's rank, as
+// keys are different.  For more than 32 results of few queries, whose other warps are many and idle.
+// Against the slots sorted in place by warp 0, 16 warps: two queries of 300 000 x 50 for 100 results, ef 128 and 400, 141.9 / 140.0 and 229.4 / 217.8 us.
+// (With four warps it gains nothing, and the code costs rows of 300 floats 3 %.)
+__device__ __forceinline__ void write_ranked(const SearchParams& p, long long qi, const Frontier& fr, int done, int w,
+                                             int warps) {
+  for (int base = 32 * w; base < done; base += 32 * warps) {
+    const int i = base + fr.lane;
+    const unsigned long long k = fr.slot(min(i, done - 1));
+    int rank = 0;
+    for (int j = 0; j < done; j += 2) {
+      const uint4 v = lds128(fr.slots + 8 * j);  // (the number of slots is even)
+      rank += Frontier::word(make_uint2(v.x, v.y)) < k ? 1 : 0;
+      rank += j + 1 < done && Frontier::word(make_uint2(v.z, v.w)) < k ? 1 : 0;
+    }
+    if (i < done && rank < p.topk) write_result(p, qi, rank, true, k);
+  }
+  for (int j = done + 32 * w + fr.lane; j < p.topk; j += 32 * warps) write_result(p, qi, j, false, 0ull);
+  if (w == 0 && fr.lane == 0) p.out_found[qi] = min(done, p.topk);
+}
 
 }  // namespace hnsw

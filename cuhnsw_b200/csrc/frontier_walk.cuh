@@ -142,7 +142,7 @@ struct FrontierWalk {
       __syncthreads();
       const uint2 words = board_words();
       const int op = __shfl_sync(FULL, (int)words.x, 0);
-      if (op == kWalkOver || op == kWalkSelect) return op;
+      if (op == kWalkOver || op == kWalkKeys) return op;
       if (op == kWalkQuery || op == kWalkNode) {
         if (!Dist::kSharedQuery) load(op, queries);
         if (op == kWalkNode) self = posted(Board::kQuery);

@@ -132,8 +132,17 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_frontier_kernel(SearchPa
   walk.bind(smem + Dist::smem_bytes(p.g.d), p.ef, p.slots, p.g.stride0, p.vsize, p.g.n);
   walk.rows = LayerRows(p.g.rows0, p.g.stride0, p.g.upper_base, 0);
   walk.self = -1;
+  using Board = typename FrontierWalk<Dist, W, P>::Board;
+  constexpr bool kShared = W > 4;  // write_ranked
   if (threadIdx.x >= 32) {
-    walk.help(p.queries);
+    if constexpr (kShared) {
+      while (walk.help(p.queries) != kWalkOver) {
+        write_ranked(p, (unsigned)walk.posted(Board::kQuery), walk.fr, walk.posted(Board::kPool), walk.warp(), W);
+        __syncthreads();
+      }
+    } else {
+      walk.help(p.queries);
+    }
     return;
   }
   for (;;) {
@@ -155,7 +164,14 @@ __global__ void __launch_bounds__(32 * W, kMinCtas) knn_frontier_kernel(SearchPa
     }
     walk.seed(cur, dcur);  // layer 0: one key, the entry, which is visited (cuda_search_kernels.cuh:108-112)
     walk.run();
-    write_closest(p, qi, walk.fr);
+    if (!kShared || p.topk <= 32) {
+      write_closest(p, qi, walk.fr);
+    } else {
+      if (lane == 0) sts32(walk.board + Board::kPool, walk.fr.done);
+      walk.post(kWalkKeys);
+      write_ranked(p, qi, walk.fr, walk.fr.done, 0, W);
+      __syncthreads();
+    }
     if (!p.ticket) break;
   }
   walk.finish();

@@ -195,7 +195,7 @@ struct WalkBoard {
   static constexpr int kBytes = (kReq + 8 * (P + 1) + 15) / 16 * 16;
 };
 // (the last two in frontier_walk.cuh only)
-enum { kWalkOver = 0, kWalkQuery = 1, kWalkRound = 2, kWalkRows = 3, kWalkNode = 4, kWalkSelect = 5 };
+enum { kWalkOver = 0, kWalkQuery = 1, kWalkRound = 2, kWalkRows = 3, kWalkNode = 4, kWalkKeys = 5 };
 
 template <class Dist, int W, int P>
 struct Walk {

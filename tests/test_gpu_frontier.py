@@ -108,3 +108,20 @@ def test_searches_in_turn_on_several_streams(d):
         torch.cuda.synchronize()
         for out in got:
           assert all(torch.equal(a, b) for a, b in zip(out, alone[nq, ef])), (ef, count, nq)
+
+
+@pytest.mark.parametrize("d,topk", [(20, 33), (20, 64), (20, 65), (60, 257), (60, 600), (200, 33), (200, 300)])
+def test_many_results_of_few_queries(d, topk):
+  """More than 32 results, ranked by all warps of a CTA: as many as are expanded, fewer, and more than the index holds; alone,
+  and several queries per CTA in turn."""
+  import torch
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  rng = np.random.default_rng(topk)
+  for n in (500, 3000):
+    base = rng.integers(-3, 4, (n, d)).astype(np.float32)
+    opt = dict(dist_type="l2", max_m=12, max_m0=24, ef_construction=64, seed=4, search_team=1)
+    eng, g = _index(base, opt)
+    q = base[rng.integers(0, n, 2 * sms + 3)]
+    for nq, ef in ((1, topk), (3, max(topk, 150)), (sms, max(topk, 150)), (2 * sms + 3, max(topk, 180))):
+      at = np.arange(min(nq, 40))
+      _equal([part[at] for part in eng.search_knn(q[:nq], topk, ef)], oracle.search(g, q[at], topk, ef), (n, nq, ef))
