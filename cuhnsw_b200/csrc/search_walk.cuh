@@ -229,11 +229,6 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
   return cudaGetLastError();
 }
 
-// Which shape.  Measured (ms per launch on a B200, CUDA tensors; one warp per query / the shape chosen here):
-//   1.18 M x 50, ef 200:  1 query 0.264 / 0.142, 148: 0.717 / 0.483, 1000: 1.07 / 0.64, 4000: 1.33 / 1.01,
-//                         6000: 1.36 / 1.29 (10 000: 1.46 / 1.99, so not there)
-//   500 000 x 128, ef 128: 1: 0.269 / 0.133, 1000: 1.28 / 0.70, 3000: 1.52 / 1.07, 6000: 1.59 / 1.47 (10 000: 1.76 / 2.32)
-//   150 000 x 960, ef 300 (the former CTA-per-query kernel / now): 1: 0.338 / 0.251, 300: 1.12 / 0.83, 1000: 1.22 / 1.07
 // Short walks prepare four nodes at a time: their later nodes are less certain and their neighbours overlap more (20 000 x
 // 50, ef 100: 1.6 evaluations for each distinct row with eight, 1.3 with four).
 //
@@ -247,15 +242,17 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
 // 300 000 x 64 f16 0.43 / 0.36, 0.49 / 0.42, 0.58 / 0.56, ef 400 0.95 / 0.83; of 1 M x 128 whole numbers 0.84 / 0.83, 0.95 / 0.95, 1.12 / 1.08, 1.92 /
 // 1.94 (4000: 1.95 / 2.20); 1000 of 50 000 x 40, ef 700 1.20 / 0.80; rows of up to 32 values 0.515 / 0.595 at 2000, ef 200.
 constexpr int kShortWalk = 100;      // largest ef of a short walk
-// Smallest ef on a frontier of up to one query per SM, of up to three, and the same of fp32 rows above 64 values, whose
-// evaluations a list's other warps share as well.  Time on the list over that on the frontier at ef 32, 40, 48, 56, 64, 80:
-//   one query: 200 000 x 50 with 24 links 1.00 1.05 1.09 1.08 1.09 1.13, with 64 links 1.02 1.06 1.08 1.14 1.19 1.27; 300 000 x 96 f16 0.96 0.99
-//   1.03 1.04 1.06 1.13; 300 000 x 128 whole numbers with 32 links 0.95 0.97 0.95 0.98 1.01 1.05, 200 000 with 48 1.01 1.10 1.11 1.16 1.22 1.25.
-//   148: 1.00 1.06 1.07 1.10 1.15 1.25, 0.94 1.04 1.11 1.08 1.10 1.17; 0.92 1.05 1.03 1.00 1.05 1.15; 1.01 1.02 1.03 1.05 1.05 1.10, 1.01 1.06 1.14 1.16
-//   1.15 1.21.
-//   444: 0.96 1.01 1.00 1.01 1.12 1.17, 0.98 1.09 1.09 1.09 1.12 1.16; 0.96 0.99 1.07 1.08 1.08 1.13; 0.88 0.89 0.93 0.93 0.99 1.02, 0.93 0.96 1.01 1.01 1.06
-//   1.11.
-constexpr int kFewFrom = 40, kSomeFrom = 40, kFewFromLong = 48, kSomeFromLong = 80;
+// Smallest ef on a frontier: of a handful of queries, of up to one per SM and more, of more than one per SM of fp32 rows above 64
+// values, whose evaluations a list's other warps share as well, and of up to two per SM of rows above 128 values (of 513 and more: from
+// kShortWalk on).  A frontier saves the merges and costs more per neighbour, so it gains the less the warmer the caches.  Time on the list over
+// that on the frontier, vectors and links in the L2 cache (a program that asks again and again) / not, at ef 48, 58, 80, 100:
+//   one query:  100 000 x 50 0.94 0.97 1.03 1.07; 1.18 M x 50 0.93 0.95 1.03 1.09 / - 1.09 1.14 1.13; 60 000 x 90 f16, 48 links, 0.94 0.98 1.07 1.16;
+//               150 000 x 120 0.91 0.91 0.98 1.05 / 0.95 0.98 1.05 1.09; 50 000 x 24 0.93 0.97 1.04 1.10
+//   37:         0.96 1.00 1.06 1.11; 1.00 1.05 1.14 1.17; 0.94 0.98 1.05 1.15; 0.99 1.03 1.11 1.14; 0.96 0.98 1.04 1.10
+//   148:        0.98 1.00 1.07 1.11; 1.02 1.06 1.13 1.19 / 1.04 1.10 1.11 1.15; 0.97 0.99 1.05 1.13; 0.96 0.98 1.05 1.12 / 1.02 1.05 1.11 1.13; 0.94 0.98 1.03 1.08
+//   444:        0.97 0.98 1.05 1.11; 1.03 1.06 1.13 1.18; 0.99 1.02 1.05 1.10; - - 1.00 1.07 / 0.93 0.93 1.02 1.03; 0.95 0.99 1.03 1.05
+//   wide, one and 148 queries at ef 101, 110, 128, 200:  60 000 x 300 0.92 0.94 0.95 1.07, 0.94 0.94 0.99 1.23;  30 000 x 800 f16 0.98 1.02 1.08 1.24, 0.98 1.00 1.02 1.14
+constexpr int kHandfulFrom = 72, kFewFrom = 56, kSomeFromLong = 80, kWideFrom = 140;
 constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 // The walks that count are those of the searches that take turns with this one on other streams as well (p.beside): a CTA of 16
 // warps fills the registers of an SM, three of eight warps do, and what comes next waits.  32 batches through four streams, ms, by
@@ -271,10 +268,10 @@ template <class Dist, int kCtas, int kFrontierCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   const long long walks = p.nq + p.beside;
   const bool long_rows = p.g.d > 64 && !p.g.rows16;
-  if (p.ef >= (long_rows ? kFewFromLong : kFewFrom) && walks <= sm_count)
+  if (p.ef >= (walks <= 8 ? kHandfulFrom : kFewFrom) && walks <= sm_count)
     return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
   const bool some = walks <= (long long)sm_count * 3 || (p.beside >= 3 * p.nq && walks <= (long long)sm_count * 6);
-  if (p.ef >= (long_rows ? kSomeFromLong : kSomeFrom) && walks > sm_count && some)
+  if (p.ef >= (long_rows ? kSomeFromLong : kFewFrom) && walks > sm_count && some)
     return launch_frontier_t<Dist, 8, 8, 3>(p, 8192, sm_count, stream, sched);
   if (p.ef <= kShortWalk) return launch_walk_t<Dist, 4, 4, kCtas>(p, 8192, sm_count, stream, sched);
   if (p.ef >= kLongNarrow && p.g.d > 32 && p.nq <= (long long)sm_count * 14 && walks <= (long long)sm_count * 20)
@@ -289,13 +286,14 @@ cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t
 template <class Dist>
 cudaError_t launch_walk_wide(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   const bool brief = p.ef <= kShortWalk;
+  const bool frontier = p.ef >= (p.g.d > 512 ? kShortWalk + 1 : kWideFrom);
   const long long walks = p.nq + p.beside;
-  if (!brief && walks <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 16384, sm_count, stream, sched);
+  if (frontier && walks <= sm_count) return launch_frontier_t<Dist, 16, 16, 1>(p, 16384, sm_count, stream, sched);
   // while two CTAs of eight warps per SM hold all queries at once; further on four CTAs of four serve more (60 000 x 960, 2,
   // 3 and 4 queries per SM, four / eight warps: ef 100 1.21 1.06 0.94, ef 200 1.12 0.96 0.78, ef 400 1.12 0.92 0.73)
   if (p.nq <= (long long)sm_count * 2)
-    return brief ? launch_walk_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched)
-                 : launch_frontier_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched);
+    return frontier ? launch_frontier_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched)
+                    : launch_walk_t<Dist, 8, 8, 2>(p, 16384, sm_count, stream, sched);
   if (brief) return launch_walk_t<Dist, 4, 4, 4>(p, 16384, sm_count, stream, sched);
   if (p.ef >= kLongWide) return launch_frontier_t<Dist, 4, 8, 4>(p, 16384, sm_count, stream, sched);
   return launch_walk_t<Dist, 4, 8, 4>(p, 16384, sm_count, stream, sched);
