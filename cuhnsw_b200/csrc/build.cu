@@ -359,8 +359,9 @@ __device__ __forceinline__ int select_team(Dist& de, unsigned keys, int nc, int 
 // walk prepares several nodes at a time (frontier_walk.cuh) and whose warps share the selection.
 constexpr int kTeamWarps = 4, kTeamNodes = 8;
 constexpr int kTeamTable = 4096;          // entries of its visited table
-// largest batch, in nodes per SM (whole builds with 0 / 10 / 20 / 40: 100 000 x 50 24.6 / 23.6 / 24.1 / 25.0 ms,
-// 1 M x 128 364 / 363 / 365 / 370, 30 000 x 960 340 / 332 / 338 / 366, 300 000 x 96 f16 35.0 / 34.4 / 34.8 / 35.9)
+// largest batch, in nodes per SM (graph construction with 0 / 5 / 10 / 20 / 40, ms: 20 000 x 50 7.1 / 6.2 / 6.3 / 6.7 / 7.5, 100 000 x 50 15.3 /
+// 14.1 / 14.2 / 14.6 / 15.8, 60 000 x 80 24.4 / 21.5 / 21.0 / 22.0 / 24.7, 300 000 x 96 f16 32.5 / 31.3 / 31.2 / 31.7 / 33.4, 1 M x 128 303 / 301 / 300 /
+// 302 / 307, 30 000 x 960 45.3 / 40.2 / 41.1 / 46.5 / 64.7)
 constexpr int kTeamPerSm = 10;
 constexpr size_t kTeamSmem = 56u << 10;   // more shared memory than this leaves fewer than four CTAs per SM
 template <class Dist>

@@ -458,8 +458,8 @@ int Engine::ResolveVsize(int cap, long long nq, int* vsize) const {
     // but never below ~4 entries per list slot, where repeats explode.  Wide rows and few queries: few warps
     // are resident whatever the table's size, and a repeated evaluation re-reads kilobytes (1 M x 960, 1000
     // queries, ef 500: 3576 evaluations per query with 2048 entries, 2099 with 16384).
-    // One CTA per query: its launcher sizes the table (walk_table_entries); what is found here only says
-    // that ef fits.
+    // One CTA per query: its launcher sizes the table (walk_table_entries, plan_cta in search_walk.cuh); what is
+    // found here only says that ef fits.
     const int kind = nq < 0 ? kSearchWarp
                             : search_kernel_kind(d_, rows16_, stride0_, cap, nq, opt_.search_team,
                                                  opt_.reverse_cand ? 1 : 0, sm_count_);

@@ -10,8 +10,8 @@
 // Nothing a prepared node brings is seen by the frontier or the visited table before its commit, so keys, visited
 // nodes and results are those of the literal walk, step for step.
 //
-// Bound: the chain of a round, two memory round trips and a commit of about 2500 cycles.  One B200, ms, with the list / so: one
-// query of 100 000 x 50, ef 300: 0.261 / 0.181; 148 of 1.18 M x 50, ef 200: 0.477 / 0.350; 37 of 1 M x 96 bfloat16, ef 128: 0.302 / 0.256;
+// Bound: the chain of a round, two memory round trips and a commit of about 2500 cycles.  One B200, ms of device time with the L2 cache
+// emptied before each launch, with the list / so: one query of 100 000 x 50, ef 300: 0.261 / 0.181; 148 of 1.18 M x 50, ef 200: 0.477 / 0.350; 37 of 1 M x 96 bfloat16, ef 128: 0.302 / 0.256;
 // one of 150 000 x 960, ef 300: 0.326 / 0.253.  It helps the more the longer the list would be (1500 keys: 1.5 to 2.3 times as fast), and the
 // less the more neighbours a node brings, as a commit costs by the neighbour and a merge by the key that is close enough
 // (search_walk.cuh).
@@ -299,7 +299,8 @@ struct FrontierWalk {
     fr.take(k, fresh, seen.full, wc);
     prefetch_row((int)v.y, fresh && k < fr.split && k < fr.limit);  // likely to be prepared in the next round
   }
-  // an adjacency row of the searched layer on its way to the L2 cache
+  // an adjacency row of the searched layer on its way to the L2 cache (37 and 148 queries of 300 000 x 128, ef 200: 0.436 -> 0.421 and 0.481 ->
+  // 0.464 ms, warm caches or not; a table that lies in the cache as a whole, 100 000 x 50, loses 1 to 2 %)
   __device__ __forceinline__ void prefetch_row(int id, bool on) const {
     const int* row = rows.row(on ? id : 0) - lane;
     prefetch_l2_if(on, row);

@@ -31,8 +31,9 @@ struct SearchParams {
   long long beside = 0;  // queries of the searches on other streams that this one runs beside, as far as the engine can tell
   int topk;
   int ef;
-  int vsize;             // visited table entries per warp (power of two); one CTA per query: chosen by its launcher, like
-  int slots = 0;         // its key slots
+  int vsize;             // visited table entries per warp, a power of two; one CTA per query: chosen by its launcher (on a
+                         // frontier a multiple of 64), like
+  int slots = 0;         // the key slots of a frontier
   int table_request = 0; // the option visited_table_size: entries per query the caller wants, 0 = by size
   size_t smem_optin = 0; // shared memory a CTA / an SM can have
   size_t smem_per_sm = 0;

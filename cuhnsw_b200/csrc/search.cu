@@ -269,19 +269,18 @@ size_t search_smem_per_cta(int d, int ef, int vsize, long long n) {
 }
 
 // One CTA per query while that is the faster way: up to so many queries per SM, which no rule on sizes hits for all data.
-// Measured with tables of 200 000 to 500 000 rows of 16 to 48 links, time of one CTA / one warp per query (device buffers,
-// medians of five launches):
+// Measured with tables of 200 000 to 300 000 rows, time of one CTA / one warp per query (device buffers, medians of nine
+// launches, L2 cache emptied before each):
 //   short walks end before rounds and, from a wave on, the entry kernel and the sort pay: 300 000 x 50, 6 and 8 queries per
-//   SM: ef 10 0.87 and 1.38, ef 30 0.81 and 1.07, ef 50 0.73 and 0.90; fp32 rows of 65 values and more, whose evaluations
-//   four warps share, hold out longer: 300 000 x 128, 12 and 20: ef 20 0.77 and 1.04, ef 50 0.61 and 0.86, but with 16
-//   links x 96, 20 per SM, 1.29 at ef 40.
-//   walks of 200 to 400: 0.5 to 0.95 up to 28 per SM, 0.8 to 1.2 at 36, 0.9 to 1.35 at 44.  Rows of up to 32 values leave the
-//   commit's one warp as the longer part if it has many links to merge: 200 000 x 32 with 32 links, ef 250, 8, 12 and 18 per
-//   SM 0.87 1.10 1.32, with 20 links at 20 per SM 1.4 (300 000 with 16 links, ef 300: 0.70 to 0.87 up to 36).
-//   long lists leave an SM 4 to 8 CTAs, each of which merges on one warp: 300 000 x 128, 14 and 26 per SM: ef 600 0.73 and
-//   1.24, ef 800 0.78 and 1.42, ef 1200 1.07 and 1.29; 24 links x 50, ef 1200: 0.86 and 1.04; ef 1000, 14 and 24 per SM: 20
-//   links x 48 1.08 and 1.41, 32 links x 48 1.01 and 1.31.  Once a list is so long that hardly more warps than CTAs fit
-//   either, CTAs win again: ef 4800 0.65 to 1.0.
+//   SM: ef 10 0.86 and 0.88, ef 30 0.83 and 0.81, ef 50 0.81 and 0.80 (the line is at 6 below ef 40, at 14 above: ef 100, 12 and
+//   24 per SM, 0.82 and 0.98); fp32 rows of 65 values and more, whose evaluations four warps share, hold out longer: 300 000 x 128,
+//   12 and 20: ef 20 0.82 and 1.10, ef 50 0.70 and 0.92; 16 links x 96, 20 per SM, 0.96 at ef 40.
+//   walks of 200 to 400: 300 000 x 50, 28 and 36 per SM, 0.91 and 1.06 at ef 200 (44: 1.23), 0.81 and 1.03 at 400; x 128, ef 200, 0.79 and
+//   0.96; 16 links x 96, ef 300, 0.74 and 0.95; rows of up to 32 values: 32 links, ef 250, 8, 12 and 18 per SM 0.68 0.73 0.77, 20 links at 20
+//   0.80, 16 links, ef 300, 28 and 36 0.88 and 1.02.
+//   long lists leave an SM 4 to 8 CTAs: 300 000 x 128, 14 and 26 per SM: ef 600 0.54 and 1.07, ef 800 0.52 and 1.15, ef 1200 0.63 and 1.48;
+//   24 links x 50, ef 1200, 12 and 20: 0.57 and 1.06; ef 1000, 14 and 24 per SM: 20 links x 48 0.57 and 0.93, 32 links x 48 0.62 and 1.07.
+//   Once a list is so long that hardly more warps than CTAs fit either: ef 4800, 20 and 36 per SM, 1.02 and 1.08.
 static int narrow_walks_per_sm(int d, int rows16, int links, int ef) {
   const bool long_rows = d > 64 && !rows16, many_links = links > 24;
   if (ef >= 4000) return 36;
@@ -293,9 +292,9 @@ static int narrow_walks_per_sm(int d, int rows16, int links, int ef) {
   return std::min({d <= 64 && many_links ? 30 : 36, few, many});
 }
 // Wide rows: warps keep 16 float4 in flight each and win once 8 to 16 of them fill an SM; when, depends on the data more than
-// on the sizes.  One CTA / one warp per query at 7, 8 and 10 queries per SM: 100 000 x 200: ef 250 1.06 1.19 1.36, ef 400 1.24
-// 1.37 1.57, ef 700 1.39 1.56 1.72, ef 3000 0.80 0.88 1.03; 200 000 x 150: ef 250 0.75 0.86 0.92, ef 400 0.91 0.98 1.14, ef 700
-// 0.80 0.84 0.99.  60 000 x 960 at 10 and 14: ef 50 0.87 1.01, ef 200 0.99 1.20, ef 400 1.06 1.28, ef 1600 0.72 0.91.
+// on the sizes.  One CTA / one warp per query at 7, 8 and 10 queries per SM: 100 000 x 200: ef 250 0.93 1.03 1.16, ef 400 0.90
+// 1.04 1.17, ef 700 0.97 1.09 1.24, ef 3000 0.56 0.59 0.73; 200 000 x 150: ef 250 0.74 0.78 0.80, ef 400 0.73 0.80 0.80, ef 700
+// 0.67 0.77 0.86.  60 000 x 960 at 10 and 14: ef 50 0.85 0.84, ef 200 1.03 1.16, ef 400 0.85 1.03, ef 1600 0.64 0.75.
 static int wide_walks_per_sm(int d, int ef) {
   if (d > 512) return ef > 200 && ef < 1200 ? 10 : 14;
   return ef > 300 && ef < 2000 ? 7 : 10;

@@ -232,10 +232,10 @@ cudaError_t launch_frontier_t(const SearchParams& p0, int table_top, int sm_coun
 // Short walks prepare four nodes at a time: their later nodes are less certain and their neighbours overlap more (20 000 x
 // 50, ef 100: 1.6 evaluations for each distinct row with eight, 1.3 with four).
 //
-// List or frontier, ms.  Up to one query per SM 16 warps x 16 nodes: one of 100 000 x 50, ef 300 0.261 / 0.181; 148 of 1.18 M x 50,
+// List or frontier, ms of device time with the L2 cache emptied before each launch.  Up to one query per SM 16 warps x 16 nodes: one of 100 000 x 50, ef 300 0.261 / 0.181; 148 of 1.18 M x 50,
 // ef 60 0.251 / 0.225, ef 200 0.477 / 0.350; 37 of 1 M x 128 whole numbers, ef 64 0.274 / 0.244; one and 148 of 600 000 x 50, ef 1500 1.27 /
 // 0.72 and 3.01 / 1.60; but ef 10 0.049 / 0.055 and 0.080 / 0.092, ef 25 the same.  Up to three 8 x 8 in three CTAs per SM: 300 of 300 000 x
-// 96 whole numbers, ef 128 0.443 / 0.369; 300 of 300 000 x 64 f16 0.357 / 0.291; 444 of 200 000 x 128 whole numbers, ef 40 0.240 / 0.236.
+// 96 whole numbers, ef 128 0.443 / 0.369; 300 of 300 000 x 64 f16 0.357 / 0.291.
 // Beyond, short and middling walks are faster on the one or on the other by the data (1000 of 500 000 x 64 whole numbers, ef 64
 // 0.339 / 0.408, ef 128 0.485 / 0.529; of 300 000 x 96 0.400 / 0.394, 0.540 / 0.499) and get the list, long ones are not slower on the
 // frontier on any of nine tables: 600, 1000 and 2000 of 1.18 M x 50, ef 200 0.67 / 0.55, 0.67 / 0.61, 0.76 / 0.66, ef 400 1.19 / 0.89; of

@@ -1,6 +1,7 @@
-"""Searches and construction of one warp per query or node with visited tables of all sizes, from 64 entries that forget nearly
-every id to one that is sized by the engine: what is expanded and found must not depend on it.  Lists around the sizes where
-the ranking changes, rows of one and two chunks, data full of exact ties, against the oracle."""
+"""Searches of one warp per query and construction with visited tables of all sizes, from 64 entries that forget nearly every id
+to one that is sized by the engine: what is expanded and found must not depend on it.  Lists around the sizes where the
+ranking changes, rows of one and two chunks, data full of exact ties, against the oracle.  (Batches of up to ten nodes per SM,
+as in the first test, are built by one CTA per node, larger ones by one warp.)"""
 import numpy as np
 import pytest
 
