@@ -259,7 +259,10 @@ constexpr int kLongNarrow = 200, kLongWide = 250;  // smallest ef of a long walk
 // the batch alone / by all: 1.18 M x 50, 148 queries each, ef 64 and 200: 3.25 / 1.97 and 5.00 / 3.52; 444: 3.33 / 2.53 and 5.73 / 4.90; 300 000 x 96
 // f16, 148: 2.95 / 1.54 and 4.50 / 2.66.  Four or more that take turns keep the chip full either way, so three CTAs of eight warps
 // do up to six per SM (10 batches of 148 and 200 of 1.18 M x 50, ef 100: 1.12 and 1.11 times as fast as on the list, six and ten of 250 1.04 and 1.13, but
-// 0.91 to 0.94 at ef 60 and on 128 floats); three batches of 200 at once do not fit (0.90).  Known loss: 100 queries of 128 floats each, ef 200 and 350, take 1.09 and 1.21 times what 16 warps took.
+// 0.91 to 0.94 at ef 60 and on 128 floats); three batches of 200 at once do not fit (0.90).  fp32 rows above 64 values gain by 16
+// warps up to 1.4 per SM in turn (32 batches of 50 of 300 000 x 128, 300 000 x 80 and 600 000 x 110, ef 200: 1.09, 1.19 and 1.15 times as fast as on the list
+// with 8, 1.25, 1.25 and 1.34 with 16); three batches of 74 at once would not (0.83 to 0.91 at ef 100).  What 100 of them gain steadily with 16 (ef 350:
+// 1.38 against 1.15 on 128 floats) they lose in a burst of three (ef 100: 0.80 against 1.08).
 // kCtas: how many CTAs of four warps on a list an SM is to hold, said to the compiler, whose own count of registers moves with
 // every change around it: seven of rows up to 64 values, six of up to 96.  ms, so / as it came out: 1000 queries of 200 000 x 32, ef 64
 // and 100, 0.219 / 0.264 and 0.301 / 0.346 (six CTAs); 3000 of 300 000 x 64, ef 128 and 180, 0.588 / 0.625 and 0.714 / 0.764 (72 registers, six in
@@ -268,7 +271,8 @@ template <class Dist, int kCtas, int kFrontierCtas>
 cudaError_t launch_walk_narrow(const SearchParams& p, int sm_count, cudaStream_t stream, const SearchSchedule* sched) {
   const long long walks = p.nq + p.beside;
   const bool long_rows = p.g.d > 64 && !p.g.rows16;
-  if (p.ef >= (walks <= 8 ? kHandfulFrom : kFewFrom) && walks <= sm_count)
+  const bool few = long_rows && p.beside > 0 ? 5 * walks <= 7ll * sm_count : walks <= sm_count;
+  if (p.ef >= (walks <= 8 ? kHandfulFrom : kFewFrom) && few)
     return launch_frontier_t<Dist, 16, 16, 1>(p, 8192, sm_count, stream, sched);
   const bool some = walks <= (long long)sm_count * 3 || (p.beside >= 3 * p.nq && walks <= (long long)sm_count * 6);
   if (p.ef >= (long_rows ? kSomeFromLong : kFewFrom) && walks > sm_count && some)
